@@ -230,7 +230,7 @@ static cy_status product_chunk(const Basis& B, const KernelSet& ks, bool centere
     const BasisDev* Bd = B.d;
     void* args[] = {(void*)&Bd, (void*)&aj, (void*)&a_stride, (void*)&bj, (void*)&b_stride, (void*)&resid};
     CY_TRY(launch(ks.mul_for(B.h.l64, centered), centered ? "mul_centered" : "mul", B.h.logn,
-                  dim3(k * ks.blocks_per_prime, nj), dim3(ks.threads), ks.smem_mul, st, args));
+                  dim3(nj * ks.blocks_per_prime, k), dim3(ks.threads), ks.smem_mul, st, args));
     return launch_epi(B, resid, oj, nj, st, epi_name(B.h.mode), lm);
 }
 
@@ -242,7 +242,7 @@ static cy_status keyswitch_chunk(const Basis& B, const KernelSet& ks, int sel, c
     const BasisDev* Bd = B.d;
     int cs = lm ? 1 : B.h.l64, ls = lm ? B.h.n : 1;  // limb w of coefficient i at [i * cs + w * ls]
     void* args[] = {(void*)&Bd, (void*)&cj, (void*)&evk, (void*)&ell, (void*)&resid, (void*)&cs, (void*)&ls};
-    CY_TRY(launch(ks.ks_for(B.h.l64, sel), "keyswitch", B.h.logn, dim3(k * ks.blocks_per_prime, nj),
+    CY_TRY(launch(ks.ks_for(B.h.l64, sel), "keyswitch", B.h.logn, dim3(nj * ks.blocks_per_prime, k),
                   dim3(ks.threads), ks.smem_ks[sel], st, args));
     return launch_epi(B, resid, oj, nj, st, epi_name(B.h.mode));
 }

@@ -79,8 +79,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     __shared__ uint32_t s_qhalf[L32MAX];
     const int tau = threadIdx.x;
     const uint32_t h = cluster_rank();
-    const int prime = blockIdx.x >> 1;
-    const int job = blockIdx.y;
+    const int prime = blockIdx.y;
+    const int job = blockIdx.x >> 1;
     const int k = B->k, l64 = B->l64;
     for (int i = tau; i < L32MAX; i += PL::G) {
         s_crt[i] = B->crt[prime][i];
@@ -157,8 +157,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     extern __shared__ uint32_t smem[];
     const int tau = threadIdx.x;
     const uint32_t h = cluster_rank();
-    const int prime = blockIdx.x >> 1;
-    const int job = blockIdx.y;
+    const int prime = blockIdx.y;
+    const int job = blockIdx.x >> 1;
     const int k = B->k, l64 = L64 > 0 ? L64 : B->l64;
     const Mod m = load_mod(B, prime);
     const uint32_t p = m.p;
