@@ -1,7 +1,7 @@
 // api.cpp -- the extern "C" boundary (include/cuyashe.h).
 //
 // Launch sequence of one product batch, per chunk of jobs:
-//   k_mul / k_keyswitch  grid (k primes, jobs)  -> residues in the workspace
+//   k_mul / k_keyswitch  grid (jobs, k primes)  -> residues in the workspace
 //   k_epi                grid (jobs * N / 256)  -> limbs (or plaintext words)
 // all on the caller's stream, no host synchronisation, no allocation once the
 // workspace has grown to the chunk size. The reference allocates 4 residue

@@ -24,14 +24,6 @@ __device__ __forceinline__ uint32_t shoup(uint32_t x, uint32_t w, uint32_t ws, u
     return x * w - q * p;
 }
 
-// a * b * 2^-32 mod p in [0, 2p) for a, b in [0, 2p), p < 2^30; pinv = -p^-1 mod 2^32.
-__device__ __forceinline__ uint32_t mont(uint32_t a, uint32_t b, uint32_t p, uint32_t pinv) {
-    const uint64_t T = (uint64_t)a * b;
-    const uint32_t m = (uint32_t)T * pinv;
-    const uint64_t u = T + (uint64_t)m * p;  // low word is zero
-    return (uint32_t)(u >> 32);
-}
-
 // The modulus with the constants derived from it. Each field is loaded from
 // memory on its own (BasisDev::p, p2, np, np2), so that the compiler cannot
 // relate them: it then emits the lazy reduction min(x, x - 2p) as one
@@ -50,6 +42,17 @@ __device__ __forceinline__ Mod mod_of(uint32_t p) { return Mod{p, 2 * p, 0u - p,
 // x * w mod p in [0, 2p), any 32-bit x (Shoup, with -p from m)
 __device__ __forceinline__ uint32_t shoup_m(uint32_t x, uint32_t w, uint32_t ws, const Mod& m) {
     return __umulhi(x, ws) * m.np + x * w;
+}
+
+// x in [0, 4p) -> [0, 2p)
+__device__ __forceinline__ uint32_t red_2p(uint32_t x, const Mod& m) { return __viaddmin_u32(x, m.np2, x); }
+
+// a * b * 2^-32 mod p in (0, 2p) for a, b in [0, 2p), p < 2^30; pinv = p^-1 mod 2^32:
+// a b and m p (m = a b p^-1 mod 2^32) have equal low words, so the difference of
+// their high words (in (-p, p)) is exact.
+__device__ __forceinline__ uint32_t mont(uint32_t a, uint32_t b, uint32_t pinv, const Mod& m) {
+    const uint64_t T = (uint64_t)a * b;
+    return (uint32_t)(T >> 32) - __umulhi((uint32_t)T * pinv, m.p) + m.p;
 }
 
 // Cooley-Tukey butterfly (Harvey's lazy form): X, Y in [0, 4p) -> X + wY, X - wY in [0, 4p).

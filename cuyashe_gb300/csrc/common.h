@@ -53,13 +53,13 @@ struct BasisDev {
     uint32_t B1[L32MAX];       //                                YASHE: (q - R_M) << s
     uint32_t p[KMAX];
     uint32_t p2[KMAX], np[KMAX], np2[KMAX];  // 2p, -p, -2p (mod 2^32), read apart from p (arith.cuh, Mod)
-    uint32_t pinv[KMAX];       // -p^-1 mod 2^32
-    uint32_t ycon[KMAX];       // residue -> [X * Mhat_i^-1]_{p_i} factor (N^-1, Montgomery folded)
+    uint32_t pinv[KMAX];       // p^-1 mod 2^32
+    uint32_t ycon[KMAX];       // residue -> [X * Mhat_i^-1]_{p_i} factor (N^-1, Montgomery factors folded)
     uint32_t ycon_sh[KMAX];    // Shoup companion of ycon
     uint32_t flo[KMAX], fhi[KMAX];  // floor(2^64/p_i) split in words (estimate of X'/M)
-    uint32_t qmodp[KMAX];      // q mod p_i (centering)
+    uint32_t qmont[KMAX];      // q 2^-32 mod p_i (centering)
     uint32_t r32[KMAX], r32_sh[KMAX];  // 2^32 mod p_i with Shoup companion
-    uint32_t crt[KMAX][L32MAX];        // 2^(32 j) mod p_i
+    uint32_t crt[KMAX][L32MAX + 1];    // 2^(32 j) mod p_i
     uint32_t A0[KMAX][L32MAX];  // MODQ: (Mhat_i mod q) << s     YASHE: (I_i mod q) << s, t*Mhat_i = I_i q + R_i
     uint32_t A1[KMAX][L32MAX];  //                                YASHE: R_i << s
     uint32_t frac[KMAX][2];     // YASHE: floor(R_i 2^64 / q) (lo, hi words)

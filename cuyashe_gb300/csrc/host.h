@@ -71,8 +71,9 @@ struct Basis {
 
 // Host constants only (no device memory): smallest prefix of the table primes
 // whose product exceeds `bound`.
-// `scale_n` folds N^-1 (inverse NTT without scaling) and `mont` folds 2^32
-// (Montgomery pointwise product) into the residue factors of the epilogue.
+// `scale_n` folds N^-1 (inverse NTT without scaling) and `mont` folds 2^96 (2^-32
+// from the CRT split of each operand and from the Montgomery pointwise product)
+// into the residue factors of the epilogue.
 cy_status basis_constants(BasisDev& h, int* crt_bits, int n, const BigUInt& q, int mode, const BigUInt& bound,
                           uint32_t t, bool mont, bool scale_n, bool centered);
 cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, const BigUInt& bound, uint32_t t,

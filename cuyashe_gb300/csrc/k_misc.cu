@@ -105,9 +105,10 @@ void* epi_kernel(int l32, int mode) {
 // multiplied by scale[i] (value, Shoup companion) when `scale` is not null.
 __global__ void k_crt(const BasisDev* __restrict__ B, const uint64_t* __restrict__ X, uint32_t* __restrict__ res,
                       const uint32_t* __restrict__ scale, int njobs) {
+    // word j times 2^(32 (j + 1)): the factor cancels the 2^-32 of the reduction
     __shared__ uint32_t s_crt[KMAX * L32MAX];
     const int k = B->k, logn = B->logn, l64 = B->l64;
-    for (int i = threadIdx.x; i < k * L32MAX; i += blockDim.x) s_crt[i] = B->crt[i / L32MAX][i % L32MAX];
+    for (int i = threadIdx.x; i < k * L32MAX; i += blockDim.x) s_crt[i] = B->crt[i / L32MAX][i % L32MAX + 1];
     __syncthreads();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int n = 1 << logn;

@@ -47,7 +47,10 @@ __device__ __forceinline__ void mixed_ntt_unit(const MixedJob& J, const MixedUni
     const GroupSync bar{1 + sub, G};
     uint32_t* sm = smem + sub * SUBW;
     const BasisDev* __restrict__ B = J.B;
-    const PrimeCtx c = load_prime_ctx(B, prime);
+    PrimeCtx c = load_prime_ctx(B, prime);
+    // 1024-thread schedule: 64 registers per thread, constants folded from p
+    if (LOGE == 3) c.m = mod_of(c.p);
+    const Mod& m = c.m;
     uint32_t x[2][E];
     constexpr int W = 2 * L64;
     uint32_t cc[W], qh[W];
@@ -65,12 +68,10 @@ __device__ __forceinline__ void mixed_ntt_unit(const MixedJob& J, const MixedUni
         x[0][e] = crt_words<W, CENTER>(wa, cc, qh, c);
         x[1][e] = crt_words<W, CENTER>(wb, cc, qh, c);
     }
-    // 1024-thread schedule: 64 registers per thread, constants folded from p
-    const Mod m = LOGE == 3 ? mod_of(c.p) : c.m;
     int buf = ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, STRIDE, 0, bar);
     uint32_t z[1][E];
 #pragma unroll
-    for (int e = 0; e < E; e++) z[0][e] = mont(red(x[0][e], 2 * c.p), red(x[1][e], 2 * c.p), c.p, c.pinv);
+    for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
     ntt_inverse<PL, 1, GroupSync>(z, B->ipsi[prime], m, tau, sm, STRIDE, buf, bar);
     uint32_t* out = J.resid + (size_t)prime * PL::N;
 #pragma unroll

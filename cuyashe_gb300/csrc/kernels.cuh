@@ -53,7 +53,7 @@ __device__ __forceinline__ uint32_t mac_red(uint32_t a, uint32_t b, const Mod& m
 
 // Per-prime constants a product kernel keeps in registers.
 struct PrimeCtx {
-    uint32_t p, pinv, r32, r32_sh, one_sh, qmodp;
+    uint32_t p, pinv, cadd;  // p, p^-1 mod 2^32, 2p - (q 2^-32 mod p)
     Mod m;
 };
 
@@ -62,46 +62,48 @@ __device__ __forceinline__ PrimeCtx load_prime_ctx(const BasisDev* __restrict__ 
     c.m = load_mod(B, i);
     c.p = c.m.p;
     c.pinv = B->pinv[i];
-    c.r32 = B->r32[i];
-    c.r32_sh = B->r32_sh[i];
-    c.one_sh = (uint32_t)(0x100000000ULL / c.p);  // Shoup companion of 1
-    c.qmodp = B->qmodp[i];
+    c.cadd = c.m.p2 - B->qmont[i];
     return c;
 }
 
-// 64-bit partial sum T (< 2^64) -> value in [0, 2p)
-__device__ __forceinline__ uint32_t fold64(uint64_t T, const PrimeCtx& c) {
-    const uint32_t hi = (uint32_t)(T >> 32), lo = (uint32_t)T;
-    const uint32_t a = shoup(hi, c.r32, c.r32_sh, c.p) + shoup(lo, 1u, c.one_sh, c.p);
-    return red(a, 2 * c.p);
+// x 2^-32 mod p in (0, 4p) (valid forward-NTT input) from T = x + a multiple of p,
+// T < 4p 2^32: T and m p (m = T p^-1 mod 2^32) have equal low words, so the
+// difference of the high words is exact. REDUCE: T's high word may reach 2p and is
+// brought below it first. neg: all ones where q is to be subtracted from x, else 0.
+template <bool REDUCE>
+__device__ __forceinline__ uint32_t crt_finish(uint64_t T, uint32_t neg, const PrimeCtx& c) {
+    uint32_t hi = (uint32_t)(T >> 32);
+    if (REDUCE) hi = __viaddmin_u32(hi, c.m.np2, hi);
+    const uint32_t h = __umulhi((uint32_t)T * c.pinv, c.p);
+    return hi - h + (c.p ^ (neg & (c.p ^ c.cadd)));  // (-p, 2p) + p, or + 2p - (q 2^-32 mod p)
 }
 
-// Residue of coefficient `pos` of a polynomial stored as [N][l64] limbs, in
-// [0, 4p) (valid forward-NTT input). `crt` (shared memory) holds 2^(32 j) mod p
-// for j < 2*l64 <= L32MAX. With CENTER, values above (q-1)/2 stand for x - q.
+// T with its high word (below 4p) brought below 2p: the same residue, and two more
+// products of a word and a residue fit.
+__device__ __forceinline__ uint64_t crt_lazy(uint64_t T, const PrimeCtx& c) {
+    const uint32_t hi = (uint32_t)(T >> 32);
+    return (uint64_t)__viaddmin_u32(hi, c.m.np2, hi) << 32 | (uint32_t)T;
+}
+
+// Residue (times 2^-32) in (0, 4p) of coefficient `pos` of a polynomial stored as
+// [N][l64] limbs. `crt` (shared memory) holds 2^(32 j) mod p for j < 2*l64 <= L32MAX.
+// With CENTER, values above (q-1)/2 stand for x - q.
 template <bool CENTER>
 __device__ __forceinline__ uint32_t crt_coef(const uint64_t* __restrict__ src, int pos, int l64,
                                              const uint32_t* crt, const uint32_t* qhalf, const PrimeCtx& c) {
     const uint64_t* s = src + (size_t)pos * l64;
     uint64_t T = 0;
-    uint32_t acc = 0;
     bool gt = false;
     for (int j = 0; j < l64; j++) {
         const uint64_t limb = __ldg(s + j);
         const uint32_t lo = (uint32_t)limb, hi = (uint32_t)(limb >> 32);
-        T += (uint64_t)lo * crt[2 * j] + (uint64_t)hi * crt[2 * j + 1];
+        T = crt_lazy(T, c) + (uint64_t)lo * crt[2 * j] + (uint64_t)hi * crt[2 * j + 1];
         if (CENTER) {
-            const uint32_t h0 = qhalf[2 * j], h1 = qhalf[2 * j + 1];
-            gt = (lo > h0) || (lo == h0 && gt);
-            gt = (hi > h1) || (hi == h1 && gt);
-        }
-        if ((j & 1) || j == l64 - 1) {  // at most 4 products of < 2^62 per partial sum
-            acc = red(acc + fold64(T, c), 2 * c.p);
-            T = 0;
+            const uint64_t h = (uint64_t)qhalf[2 * j + 1] << 32 | qhalf[2 * j];
+            gt = limb > h || (limb == h && gt);
         }
     }
-    if (CENTER && gt) acc = acc + 2 * c.p - c.qmodp;  // [0, 4p)
-    return acc;
+    return crt_finish<true>(T, gt ? ~0u : 0u, c);
 }
 
 // The limbs of one coefficient as 32-bit words (16-byte loads when L64 is even).
@@ -126,53 +128,68 @@ __device__ __forceinline__ void load_words(const uint64_t* __restrict__ p, uint3
     }
 }
 
-// Residue in [0, 4p) of the coefficient whose 32-bit words are w (compile-time
-// count W); cc[j] = 2^(32 j) mod p. With CENTER, values above (q-1)/2 (words
-// qh) stand for x - q.
+// All ones when x (words w) is above (q-1)/2 (words qh), else 0: (q-1)/2 - x borrows
+// exactly then, so one subtract-with-borrow chain and its final borrow spread to a
+// mask (no compares, no selects, no branches).
+template <int W>
+__device__ __forceinline__ uint32_t above_half(const uint32_t (&w)[W], const uint32_t (&qh)[W]) {
+    static_assert(W % 2 == 0 && W >= 2 && W <= 12, "an even number of words");
+    // 64-bit words: each asm statement must hold the whole chain (the carry flag does
+    // not outlive it), so one statement per width
+    auto v = [&](int i) { return (uint64_t)w[2 * i + 1] << 32 | w[2 * i]; };
+    auto h = [&](int i) { return (uint64_t)qh[2 * i + 1] << 32 | qh[2 * i]; };
+    uint32_t mask;
+    if constexpr (W == 2) {
+        asm("{\n\t.reg .u64 d;\n\tsub.cc.u64 d, %1, %2;\n\tsubc.u32 %0, 0, 0;\n\t}"
+            : "=r"(mask) : "l"(h(0)), "l"(v(0)));
+    } else if constexpr (W == 4) {
+        asm("{\n\t.reg .u64 d;\n\tsub.cc.u64 d, %1, %2;\n\tsubc.cc.u64 d, %3, %4;\n\tsubc.u32 %0, 0, 0;\n\t}"
+            : "=r"(mask) : "l"(h(0)), "l"(v(0)), "l"(h(1)), "l"(v(1)));
+    } else if constexpr (W == 6) {
+        asm("{\n\t.reg .u64 d;\n\tsub.cc.u64 d, %1, %2;\n\tsubc.cc.u64 d, %3, %4;\n\tsubc.cc.u64 d, %5, %6;\n\t"
+            "subc.u32 %0, 0, 0;\n\t}"
+            : "=r"(mask) : "l"(h(0)), "l"(v(0)), "l"(h(1)), "l"(v(1)), "l"(h(2)), "l"(v(2)));
+    } else if constexpr (W == 8) {
+        asm("{\n\t.reg .u64 d;\n\tsub.cc.u64 d, %1, %2;\n\tsubc.cc.u64 d, %3, %4;\n\tsubc.cc.u64 d, %5, %6;\n\t"
+            "subc.cc.u64 d, %7, %8;\n\tsubc.u32 %0, 0, 0;\n\t}"
+            : "=r"(mask)
+            : "l"(h(0)), "l"(v(0)), "l"(h(1)), "l"(v(1)), "l"(h(2)), "l"(v(2)), "l"(h(3)), "l"(v(3)));
+    } else if constexpr (W == 10) {
+        asm("{\n\t.reg .u64 d;\n\tsub.cc.u64 d, %1, %2;\n\tsubc.cc.u64 d, %3, %4;\n\tsubc.cc.u64 d, %5, %6;\n\t"
+            "subc.cc.u64 d, %7, %8;\n\tsubc.cc.u64 d, %9, %10;\n\tsubc.u32 %0, 0, 0;\n\t}"
+            : "=r"(mask)
+            : "l"(h(0)), "l"(v(0)), "l"(h(1)), "l"(v(1)), "l"(h(2)), "l"(v(2)), "l"(h(3)), "l"(v(3)), "l"(h(4)),
+              "l"(v(4)));
+    } else {
+        asm("{\n\t.reg .u64 d;\n\tsub.cc.u64 d, %1, %2;\n\tsubc.cc.u64 d, %3, %4;\n\tsubc.cc.u64 d, %5, %6;\n\t"
+            "subc.cc.u64 d, %7, %8;\n\tsubc.cc.u64 d, %9, %10;\n\tsubc.cc.u64 d, %11, %12;\n\t"
+            "subc.u32 %0, 0, 0;\n\t}"
+            : "=r"(mask)
+            : "l"(h(0)), "l"(v(0)), "l"(h(1)), "l"(v(1)), "l"(h(2)), "l"(v(2)), "l"(h(3)), "l"(v(3)), "l"(h(4)),
+              "l"(v(4)), "l"(h(5)), "l"(v(5)));
+    }
+    return mask;
+}
+
+// Residue (times 2^-32) in (0, 4p) of the coefficient whose 32-bit words are w
+// (compile-time count W); cc[j] = 2^(32 j) mod p. With CENTER, values above (q-1)/2
+// (words qh) stand for x - q. The factor 2^-32 is folded into the ICRT constants,
+// so that word 0 needs no product and one Montgomery step (a multiply, a mul.hi)
+// ends the sum. The fma-heavy pipe bounds these kernels (mul.hi and wide products take
+// four of its cycles per warp, other multiplies two): the sum of W products and two
+// Shoup reductions per four words that this replaces took 32 of them at W = 4 against
+// 48 for the coefficient's forward transform, this takes 18. 512 tensor products at
+// N = 4096, 127-bit q: 224 -> 194 us; at N = 8192, 190-bit q: 1044 -> 791 us.
 template <int W, bool CENTER>
 __device__ __forceinline__ uint32_t crt_words(const uint32_t (&w)[W], const uint32_t (&cc)[W],
                                               const uint32_t (&qh)[W], const PrimeCtx& c) {
-    uint32_t acc = 0;
+    uint64_t T = w[0];
 #pragma unroll
-    for (int j0 = 0; j0 < W; j0 += 4) {
-        uint64_t T = 0;
-#pragma unroll
-        for (int j = j0; j < j0 + 4 && j < W; j++) T += (uint64_t)w[j] * cc[j];  // < 4 * 2^62
-        const uint32_t f = fold64(T, c);
-        acc = (j0 == 0) ? f : red(acc + f, 2 * c.p);
+    for (int j = 1; j < W; j++) {
+        if (j >= 4 && j % 2 == 0) T = crt_lazy(T, c);  // below 2p 2^32, two products more
+        T += (uint64_t)w[j] * cc[j];
     }
-    if (CENTER) {
-        // x > (q-1)/2: one 64- or 128-bit compare (no branch) for two or four
-        // words; for more, the top words decide unless they are equal (rare),
-        // then the lower words do
-        bool gt;
-        if constexpr (W == 2) {
-            gt = ((uint64_t)w[1] << 32 | w[0]) > ((uint64_t)qh[1] << 32 | qh[0]);
-        } else if constexpr (W == 4) {
-            // (q-1)/2 - x borrows exactly when x > (q-1)/2: one subtract-with-borrow
-            // chain, its final borrow spread to a mask (no compares, no selects)
-            uint32_t mask;
-            asm("{\n\t.reg .u32 d;\n\t"
-                "sub.cc.u32 d, %1, %5;\n\t"
-                "subc.cc.u32 d, %2, %6;\n\t"
-                "subc.cc.u32 d, %3, %7;\n\t"
-                "subc.cc.u32 d, %4, %8;\n\t"
-                "subc.u32 %0, 0, 0;\n\t}"
-                : "=r"(mask)
-                : "r"(qh[0]), "r"(qh[1]), "r"(qh[2]), "r"(qh[3]), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]));
-            return acc + (mask & (2 * c.p - c.qmodp));  // [0, 4p)
-        } else {
-            gt = w[W - 1] > qh[W - 1];
-            if (w[W - 1] == qh[W - 1]) {
-                bool g = false;
-#pragma unroll
-                for (int j = 0; j < W - 1; j++) g = (w[j] > qh[j]) || (w[j] == qh[j] && g);
-                gt = g;
-            }
-        }
-        acc += gt ? 2 * c.p - c.qmodp : 0u;  // [0, 4p)
-    }
-    return acc;
+    return crt_finish<(W > 3)>(T, CENTER ? above_half<W>(w, qh) : 0u, c);
 }
 
 // --------------------------------------------------------------------------
@@ -261,7 +278,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
     else buf = ntt_forward<PL, 2>(x, psi, c.m, tau, smem, STRIDE, 0, CtaSync(), 1, B->psi_r[prime]);
     uint32_t z[1][E];
 #pragma unroll
-    for (int e = 0; e < E; e++) z[0][e] = mont(red(x[0][e], 2 * c.p), red(x[1][e], 2 * c.p), c.p, c.pinv);
+    for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
     if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, B->ipsi_r[prime], c.m, tau, smem + STRIDE, STRIDE == 0, nullptr);
     else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, STRIDE, buf, CtaSync(), 1, B->ipsi_r[prime]);
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;

@@ -219,26 +219,27 @@ cy_status basis_constants(BasisDev& h, int* crt_bits, int n, const BigUInt& q, i
         h.p2[i] = 2 * p;
         h.np[i] = 0u - p;
         h.np2[i] = 0u - 2 * p;
-        // -p^-1 mod 2^32 by Newton iteration
+        // p^-1 mod 2^32 by Newton iteration
         uint32_t inv = p;
         for (int it = 0; it < 5; it++) inv *= 2u - p * inv;
-        h.pinv[i] = (uint32_t)(0u - inv);
+        h.pinv[i] = inv;
         const BigUInt Mhat = M / BigUInt(p);
         const uint32_t mh = Mhat.mod_u32(p);
         uint32_t f = invmod32(mh, p);
         if (scale_n) f = mulmod32(f, invmod32((uint32_t)(n % p), p), p);
-        if (mont) f = mulmod32(f, (uint32_t)((1ull << 32) % p), p);
+        if (mont)  // 2^-32 from the CRT split of each operand and from the pointwise product
+            for (int it = 0; it < 3; it++) f = mulmod32(f, (uint32_t)((1ull << 32) % p), p);
         h.ycon[i] = f;
         h.ycon_sh[i] = shoup_of(f, p);
         const uint64_t F = (uint64_t)(((unsigned __int128)1 << 64) / p);
         h.fhi[i] = (uint32_t)(F >> 32);
         h.flo[i] = (uint32_t)F;
-        h.qmodp[i] = q.mod_u32(p);
         const uint32_t r32 = (uint32_t)((1ull << 32) % p);
+        h.qmont[i] = mulmod32(q.mod_u32(p), invmod32(r32, p), p);
         h.r32[i] = r32;
         h.r32_sh[i] = shoup_of(r32, p);
         uint32_t c = 1;
-        for (int j = 0; j < L32MAX; j++) {
+        for (int j = 0; j <= L32MAX; j++) {
             h.crt[i][j] = c;
             c = mulmod32(c, r32, p);
         }
