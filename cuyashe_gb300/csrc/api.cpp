@@ -27,7 +27,7 @@ namespace cy {
 const char* last_error_message();
 void* addsub_kernel(int l64, bool sub);
 void* crt_kernel();
-void* shoup_pairs_kernel();
+void* evk_mont_kernel();
 void* evk_rows_kernel();
 
 static constexpr int kEpiThreads = 256;
@@ -236,7 +236,7 @@ static cy_status product_chunk(const Basis& B, const KernelSet& ks, bool centere
 
 // One chunk of keyswitches c_j -> out_j (out may alias c), residues in `resid`;
 // lm: c is limb-major ([job][limb][N]).
-static cy_status keyswitch_chunk(const Basis& B, const KernelSet& ks, int sel, const uint64_t* cj, const uint2* evk,
+static cy_status keyswitch_chunk(const Basis& B, const KernelSet& ks, int sel, const uint64_t* cj, const uint32_t* evk,
                                  int ell, uint64_t* oj, int nj, uint32_t* resid, cudaStream_t st, int lm = 0) {
     const int k = B.h.k;
     const BasisDev* Bd = B.d;
@@ -287,7 +287,7 @@ static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, l
 // chunk_k > 0 sizes the chunks as for a basis of that many primes (the tuner
 // uses the HE multiply's chunks, which are sized by its larger basis).
 // lm: c is limb-major (the tuner times the layout of the HE multiply's keyswitch)
-static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint2* evk, int ell, uint64_t* out,
+static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint32_t* evk, int ell, uint64_t* out,
                                int batch, Workspace& ws, cudaStream_t st, int variant = -1, int chunk_k = 0,
                                int lm = 0) {
     if (batch == 0) return CY_OK;
@@ -314,7 +314,7 @@ static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint2* e
 // YASHE rounding into out, then (relin) its keyswitch in place; chunks alternate
 // between two lanes.
 // ks_variant >= 0 forces the keyswitch schedule (the autotuner's timing runs).
-cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint2* evk, int ell, const uint64_t* c1,
+cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
                         const uint64_t* c2, uint64_t* out, int batch, bool do_relin, Workspace& ws, cudaStream_t st,
                         int ks_variant) {
     if (batch == 0) return CY_OK;
@@ -444,25 +444,25 @@ int yashe_chunk_jobs(const Basis& tensor, const Basis& relin, int ell, bool do_r
     return chunk;
 }
 
-cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint2* evk, int ell, uint64_t* out, int batch,
+cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* evk, int ell, uint64_t* out, int batch,
                             Workspace& ws, cudaStream_t st, int variant, int chunk_k, int lm) {
     return run_keyswitch(B, c, evk, ell, out, batch, ws, st, variant, chunk_k, lm);
 }
 
-// Evaluation key in the keyswitch basis, NTT domain, with Shoup companions:
-// d_evk [ell][k][N] of (value, floor(value 2^32 / p)); at N = ROWS_N a second
-// copy laid out by lane follows it (the 64-coefficient keyswitch reads that
-// one). Synchronous.
-cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint2** d_evk) {
+// Evaluation key in the keyswitch basis, NTT domain, in Montgomery form: d_evk
+// [ell][k][N] of value 2^32 mod p (the keyswitch sums products with the digits in 64
+// bits and reduces once); at N = ROWS_N a second copy laid out by lane follows it
+// (the 64-coefficient keyswitch reads that one). Synchronous.
+cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint32_t** d_evk) {
     const int k = relin.h.k;
     const size_t words = (size_t)ell * k * n;
     const bool rows = relin.h.logn == ROWS_LOGN;
     uint64_t* d_limbs = nullptr;
     uint32_t* d_res = nullptr;
-    uint2* out = nullptr;
+    uint32_t* out = nullptr;
     cudaError_t e = cudaMalloc(&d_limbs, sizeof(uint64_t) * (size_t)ell * n * l64);
     if (e == cudaSuccess) e = cudaMalloc(&d_res, sizeof(uint32_t) * words);
-    if (e == cudaSuccess) e = cudaMalloc(&out, sizeof(uint2) * words * (rows ? 2 : 1));
+    if (e == cudaSuccess) e = cudaMalloc(&out, sizeof(uint32_t) * words * (rows ? 2 : 1));
     if (e == cudaSuccess)
         e = cudaMemcpy(d_limbs, h_evk, sizeof(uint64_t) * (size_t)ell * n * l64, cudaMemcpyHostToDevice);
     cy_status st = (e == cudaSuccess) ? CY_OK : cuda_error(e, "evaluation key upload");
@@ -472,10 +472,10 @@ cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n,
         const BasisDev* Bd = relin.d;
         long long total = (long long)words;
         void* args[] = {(void*)&Bd, (void*)&d_res, (void*)&out, (void*)&total};
-        st = launch(shoup_pairs_kernel(), "shoup_pairs", relin.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256),
+        st = launch(evk_mont_kernel(), "evk_mont", relin.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256),
                     0, 0, args);
         if (st == CY_OK && rows) {
-            uint2* out_rows = out + words;
+            uint32_t* out_rows = out + words;
             void* rargs[] = {(void*)&out, (void*)&out_rows, (void*)&total};
             st = launch(evk_rows_kernel(), "evk_rows", relin.h.logn, dim3((unsigned)((total + 255) / 256)),
                         dim3(256), 0, 0, rargs);

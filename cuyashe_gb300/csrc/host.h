@@ -161,7 +161,7 @@ struct cy_yashe {
     uint64_t* d_f = nullptr;
     uint64_t* d_f2 = nullptr;
     uint64_t* d_h = nullptr;    // public key (GPU encryption)
-    uint2* d_evk = nullptr;     // [ell][k'][N] NTT-domain evaluation key
+    uint32_t* d_evk = nullptr;  // [ell][k'][N] NTT-domain evaluation key times 2^32
     uint64_t* d_cdt = nullptr;  // discrete Gaussian thresholds (GPU sampling)
     int n_cdt = 0;
     ~cy_yashe();

@@ -125,28 +125,26 @@ __global__ void k_crt(const BasisDev* __restrict__ B, const uint64_t* __restrict
     }
 }
 
-// Shoup companions of NTT-domain values: out[j] = (v, floor(v 2^32 / p_i)) for
-// the residue vectors of a [ell][k][N] array.
-__global__ void k_shoup_pairs(const BasisDev* __restrict__ B, const uint32_t* __restrict__ v, uint2* __restrict__ out,
-                              long long total) {
+// Montgomery form of NTT-domain values: out[j] = v 2^32 mod p_i for the residue
+// vectors of a [ell][k][N] array.
+__global__ void k_evk_mont(const BasisDev* __restrict__ B, const uint32_t* __restrict__ v, uint32_t* __restrict__ out,
+                           long long total) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int prime = (int)((idx >> B->logn) % B->k);
-    const uint32_t p = B->p[prime];
-    const uint32_t x = v[idx];
-    out[idx] = make_uint2(x, (uint32_t)(((uint64_t)x << 32) / p));
+    out[idx] = (uint32_t)(((uint64_t)v[idx] << 32) % B->p[prime]);
 }
 
-// The copy of an NTT-domain evaluation key [ell][k][ROWS_N] of (value, Shoup)
-// pairs laid out by lane for the row pass of the 64-coefficient schedule: the
-// entry at position 64 tau + u goes to record [u/2][tau], word u mod 2.
-__global__ void k_evk_rows(const uint2* __restrict__ in, uint2* __restrict__ out, long long total) {
+// The copy of an NTT-domain evaluation key [ell][k][ROWS_N] laid out by lane for
+// the row pass of the 64-coefficient schedule: the entry at position 64 tau + u
+// goes to the 16-byte record [u/4][tau], word u mod 4.
+__global__ void k_evk_rows(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, long long total) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const long long row = idx / ROWS_N;
     const int pos = (int)(idx % ROWS_N);
     const int tau = pos >> 6, u = pos & 63;
-    out[row * ROWS_N + (u >> 1) * 2 * ROWS_G + 2 * tau + (u & 1)] = in[idx];
+    out[row * ROWS_N + (u >> 2) * 4 * ROWS_G + 4 * tau + (u & 3)] = in[idx];
 }
 
 // Elementwise c = a +/- b mod q over [count][l64] limbs (inputs in [0, q)).
@@ -278,7 +276,7 @@ cy_status move_polys(uint64_t* const* d_ptrs, uint64_t* flat, int count, size_t 
 }
 
 void* crt_kernel() { return (void*)k_crt; }
-void* shoup_pairs_kernel() { return (void*)k_shoup_pairs; }
+void* evk_mont_kernel() { return (void*)k_evk_mont; }
 void* evk_rows_kernel() { return (void*)k_evk_rows; }
 
 }  // namespace cy

@@ -89,7 +89,6 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
                                               uint32_t* __restrict__ done) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E, G = PL::G;
-    constexpr int LAST = PL::NPASS - 1;
     constexpr int SUBW = 4 * PL::SMW;
     constexpr int STRIDE = 2 * PL::SMW;
     const int sub = threadIdx.x / G, tau = threadIdx.x % G;
@@ -100,9 +99,9 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
     const BasisDev* __restrict__ B = J.B2;
     const Mod m = LOGE == 3 ? mod_of(B->p[prime]) : load_mod(B, prime);
     const int k2 = J.k2, ell = J.ell;
-    uint32_t acc[1][E];
+    uint64_t T[E];  // sums of products with the key (see k_keyswitch)
 #pragma unroll
-    for (int e = 0; e < E; e++) acc[0][e] = 0;
+    for (int e = 0; e < E; e++) T[e] = 0;
     int buf = 0;
     for (int d0 = 0; d0 < ell; d0 += 2) {
         uint32_t x[2][E];
@@ -123,18 +122,22 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
         }
         buf = ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, STRIDE, buf, bar);
 #pragma unroll
+        for (int e = 0; e < E; e++) T[e] = lazy_high(T[e], m);
+#pragma unroll
         for (int o = 0; o < 2; o++) {
             const int d = d0 + o;
             if (d < ell) {
-                const uint2* __restrict__ g = J.evk + ((size_t)d * k2 + prime) * PL::N;
+                uint32_t v[E];
+                load_evk<PL>(J.evk + ((size_t)d * k2 + prime) * PL::N, tau, v);
 #pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const uint2 W = __ldg(g + slot_pos<PL, LAST>(tau, e));
-                    acc[0][e] = mac_red(acc[0][e], shoup_m(x[o][e], W.x, W.y, m), m);
-                }
+                for (int e = 0; e < E; e++) T[e] += (uint64_t)x[o][e] * v[e];
             }
         }
     }
+    uint32_t acc[1][E];
+    const uint32_t pinv = B->pinv[prime];
+#pragma unroll
+    for (int e = 0; e < E; e++) acc[0][e] = mac_finish<true>(T[e], pinv, m);
     ntt_inverse<PL, 1, GroupSync>(acc, B->ipsi[prime], m, tau, sm, STRIDE, buf, bar);
     uint32_t* out = J.resid + (size_t)prime * PL::N;
 #pragma unroll

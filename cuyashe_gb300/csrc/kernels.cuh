@@ -80,9 +80,9 @@ __device__ __forceinline__ uint32_t crt_finish(uint64_t T, uint32_t neg, const P
 
 // T with its high word (below 4p) brought below 2p: the same residue, and two more
 // products of a word and a residue fit.
-__device__ __forceinline__ uint64_t crt_lazy(uint64_t T, const PrimeCtx& c) {
+__device__ __forceinline__ uint64_t lazy_high(uint64_t T, const Mod& m) {
     const uint32_t hi = (uint32_t)(T >> 32);
-    return (uint64_t)__viaddmin_u32(hi, c.m.np2, hi) << 32 | (uint32_t)T;
+    return (uint64_t)__viaddmin_u32(hi, m.np2, hi) << 32 | (uint32_t)T;
 }
 
 // Residue (times 2^-32) in (0, 4p) of coefficient `pos` of a polynomial stored as
@@ -97,7 +97,7 @@ __device__ __forceinline__ uint32_t crt_coef(const uint64_t* __restrict__ src, i
     for (int j = 0; j < l64; j++) {
         const uint64_t limb = __ldg(s + j);
         const uint32_t lo = (uint32_t)limb, hi = (uint32_t)(limb >> 32);
-        T = crt_lazy(T, c) + (uint64_t)lo * crt[2 * j] + (uint64_t)hi * crt[2 * j + 1];
+        T = lazy_high(T, c.m) + (uint64_t)lo * crt[2 * j] + (uint64_t)hi * crt[2 * j + 1];
         if (CENTER) {
             const uint64_t h = (uint64_t)qhalf[2 * j + 1] << 32 | qhalf[2 * j];
             gt = limb > h || (limb == h && gt);
@@ -186,7 +186,7 @@ __device__ __forceinline__ uint32_t crt_words(const uint32_t (&w)[W], const uint
     uint64_t T = w[0];
 #pragma unroll
     for (int j = 1; j < W; j++) {
-        if (j >= 4 && j % 2 == 0) T = crt_lazy(T, c);  // below 2p 2^32, two products more
+        if (j >= 4 && j % 2 == 0) T = lazy_high(T, c.m);  // below 2p 2^32, two products more
         T += (uint64_t)w[j] * cc[j];
     }
     return crt_finish<(W > 3)>(T, CENTER ? above_half<W>(w, qh) : 0u, c);
@@ -287,26 +287,69 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
 }
 
 // --------------------------------------------------------------------------
-// k_keyswitch: one block per (prime, job). Digits are the 32-bit words of the
+// k_keyswitch: one block per (job, prime). Digits are the 32-bit words of the
 // coefficients of c in [0, q) (w = 2^32), processed ND at a time.
-// evk: [ell][k][N] (value, Shoup companion) in the forward-NTT output order.
+// evk: [ell][k][N] values times 2^32 mod p in the forward-NTT output order.
 // --------------------------------------------------------------------------
+// The E key values of thread tau after the last forward pass (contiguous positions).
+template <class PL>
+__device__ __forceinline__ void load_evk(const uint32_t* __restrict__ g, int tau, uint32_t (&v)[PL::E]) {
+    constexpr int LAST = PL::NPASS - 1, E = PL::E;
+    static_assert(PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE, "contiguous last-pass positions");
+    const uint32_t* s = g + group_base<PL, LAST>(tau, 0);
+    if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int h = 0; h < E / 4; h++) {
+            const uint4 W = __ldg(reinterpret_cast<const uint4*>(s) + h);
+            v[4 * h] = W.x;
+            v[4 * h + 1] = W.y;
+            v[4 * h + 2] = W.z;
+            v[4 * h + 3] = W.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; e++) v[e] = __ldg(s + e);
+    }
+}
+
+// Sum of up to four products of a digit in [0, 4p) and a key value below p (T < 4p 2^32)
+// -> T 2^-32 mod p in [0, 2p). MANY: more than two products since T was below 2^32.
+template <bool MANY>
+__device__ __forceinline__ uint32_t mac_finish(uint64_t T, uint32_t pinv, const Mod& m) {
+    uint32_t hi = (uint32_t)(T >> 32);
+    if (MANY) hi = __viaddmin_u32(hi, m.np2, hi);
+    return red_2p(hi - __umulhi((uint32_t)T * pinv, m.p) + m.p, m);  // (0, 3p) -> [0, 2p)
+}
+
+// The products with the key are summed in 64 bits (one wide multiply-add each) and
+// reduced once per coefficient by a Montgomery step; a Shoup product per digit and
+// coefficient took three multiplies and twice the key bytes.
+// ONE: all digits in one pass (kernels of one or two limbs), no sums kept across
+// transforms. Otherwise the 64-bit sums stay in registers with 8 or 16 coefficients
+// per thread; with more (ACC32) each pass's sums are reduced and added to 32-bit ones.
+template <int L64, int ND>
+__host__ __device__ constexpr bool ks_one_pass() {
+    return (L64 == 1 && ND >= 2) || (L64 == 2 && ND >= 4);
+}
+
 // SINGLE: one exchange region (two barriers per exchange) instead of two, so
 // that more blocks fit in shared memory.
 template <int LOGN, int LOGE, int L64, int ND, int MINB = 0, bool SINGLE = false>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_min_blocks<LOGN, LOGE>()))
-    k_keyswitch(const BasisDev* __restrict__ B, const uint64_t* __restrict__ C, const uint2* __restrict__ evk,
+    k_keyswitch(const BasisDev* __restrict__ B, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
                 int ell, uint32_t* __restrict__ resid, int cs, int ls) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
     constexpr int LAST = PL::NPASS - 1;
+    constexpr bool ONE = ks_one_pass<L64, ND>();
+    constexpr bool ACC32 = !ONE && LOGE > 4;
     extern __shared__ uint32_t smem[];  // exchange regions, ND operands x SMW each
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
     const int k = B->k, l64 = L64 > 0 ? L64 : B->l64;
     const Mod m = load_mod(B, prime);
-    const uint32_t p = m.p;
+    const uint32_t p = m.p, pinv = B->pinv[prime];
     const uint2* __restrict__ psi = B->psi[prime];
     const uint2* __restrict__ ipsi = B->ipsi[prime];
     const uint64_t* cj = C + (size_t)job * PL::N * l64;
@@ -316,11 +359,15 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     // in the constant bank.
     constexpr int STRIDE = SINGLE ? 0 : region_stride<PL, ND>();
 
-    uint32_t acc[1][E];
+    uint64_t T[E];           // sums of products
+    uint32_t acc[1][E];      // reduced sums: the inverse transform's input
 #pragma unroll
-    for (int e = 0; e < E; e++) acc[0][e] = 0;
+    for (int e = 0; e < E; e++) {
+        T[e] = 0;
+        acc[0][e] = 0;
+    }
     int buf = 0;
-    for (int d0 = 0; d0 < ell; d0 += ND) {
+    for (int d0 = 0; d0 < (ONE ? 1 : ell); d0 += ND) {
         uint32_t x[ND][E];
 #pragma unroll
         for (int e = 0; e < E; e++) {
@@ -370,39 +417,50 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
         } else {
             buf = ntt_forward<PL, ND>(x, psi, m, tau, smem, STRIDE, buf, CtaSync(), 1, B->psi_r[prime]);
         }
+        if constexpr (rows_pass<PL, LAST>()) {
+            // the key's copy laid out by lane (after the [ell][k][N] table): values u .. u+3
+            // of lane tau are the 16-byte record [u/4][tau]
+            static_assert(ND == 1, "one digit per pass with 64 coefficients per thread");
+            const uint4* g4 = reinterpret_cast<const uint4*>(evk + ((size_t)(ell + d0) * k + prime) * PL::N) + tau;
 #pragma unroll
-        for (int o = 0; o < ND; o++) {
-            const int d = d0 + o;
-            if (d < ell) {
-                const uint2* __restrict__ g = evk + ((size_t)d * k + prime) * PL::N;
-                if constexpr (rows_pass<PL, LAST>()) {
-                    // the key's copy laid out by lane (after the [ell][k][N] table): the
-                    // pair (u, u+1) of lane tau is the 16-byte record [u/2][tau]
-                    const uint4* g4 = reinterpret_cast<const uint4*>(g + (size_t)ell * k * PL::N) + tau;
+            for (int h = 0; h < E / 4; h++) {
+                const uint4 W = __ldg(g4 + h * PL::G);
+                const uint32_t v[4] = {W.x, W.y, W.z, W.w};
 #pragma unroll
-                    for (int h = 0; h < E / 2; h++) {
-                        const uint4 W = __ldg(g4 + h * PL::G);
-                        acc[0][2 * h] = mac_red(acc[0][2 * h], shoup_m(x[o][2 * h], W.x, W.y, m), m);
-                        acc[0][2 * h + 1] = mac_red(acc[0][2 * h + 1], shoup_m(x[o][2 * h + 1], W.z, W.w, m), m);
-                    }
-                } else if constexpr (PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE) {
-                    // after the last pass a thread's E positions are contiguous: 16-byte loads
-                    const uint4* g4 = reinterpret_cast<const uint4*>(g + group_base<PL, LAST>(tau, 0));
-#pragma unroll
-                    for (int h = 0; h < E / 2; h++) {
-                        const uint4 W = __ldg(g4 + h);
-                        acc[0][2 * h] = mac_red(acc[0][2 * h], shoup_m(x[o][2 * h], W.x, W.y, m), m);
-                        acc[0][2 * h + 1] = mac_red(acc[0][2 * h + 1], shoup_m(x[o][2 * h + 1], W.z, W.w, m), m);
-                    }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < E; e++) {
-                        const uint2 W = __ldg(g + slot_pos<PL, LAST>(tau, e));
-                        acc[0][e] = mac_red(acc[0][e], shoup_m(x[o][e], W.x, W.y, m), m);
-                    }
+                for (int j = 0; j < 4; j++) {  // one product: (x v 2^-32) in (0, 2p)
+                    const uint64_t t = (uint64_t)x[0][4 * h + j] * v[j];
+                    const uint32_t r = (uint32_t)(t >> 32) - __umulhi((uint32_t)t * pinv, p) + p;
+                    acc[0][4 * h + j] = mac_red(acc[0][4 * h + j], r, m);
                 }
             }
+        } else {
+            if constexpr (ACC32) {
+#pragma unroll
+                for (int e = 0; e < E; e++) T[e] = 0;
+            }
+#pragma unroll
+            for (int o = 0; o < ND; o++) {
+                const int d = d0 + o;
+                if (!ONE && !ACC32 && o % 2 == 0) {  // two products fit on top of a high word below 2p
+#pragma unroll
+                    for (int e = 0; e < E; e++) T[e] = lazy_high(T[e], m);
+                }
+                if (d < ell) {
+                    uint32_t v[E];
+                    load_evk<PL>(evk + ((size_t)d * k + prime) * PL::N, tau, v);
+#pragma unroll
+                    for (int e = 0; e < E; e++) T[e] += (uint64_t)x[o][e] * v[e];
+                }
+            }
+            if constexpr (ACC32) {
+#pragma unroll
+                for (int e = 0; e < E; e++) acc[0][e] = mac_red(acc[0][e], mac_finish<(ND > 2)>(T[e], pinv, m), m);
+            }
         }
+    }
+    if constexpr (!ACC32 && !rows_pass<PL, LAST>()) {
+#pragma unroll
+        for (int e = 0; e < E; e++) acc[0][e] = mac_finish<!(ONE && ND <= 2)>(T[e], pinv, m);
     }
     if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, B->ipsi_r[prime], m, tau, smem, true, nullptr);
     else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), 1, B->ipsi_r[prime]);

@@ -148,12 +148,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
 // k_keyswitch for N = 16384 on a block pair, ND digits per pass (see k_keyswitch).
 template <int L64, int ND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
-    k_keyswitch_pair(const BasisDev* __restrict__ B, const uint64_t* __restrict__ C, const uint2* __restrict__ evk,
+    k_keyswitch_pair(const BasisDev* __restrict__ B, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
                      int ell, uint32_t* __restrict__ resid, int cs, int ls) {
     using PL = PairPlan;
     constexpr int E = PL::E;
-    constexpr int LAST = PL::NPASS - 1;
-    static_assert(PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE, "contiguous last-pass positions");
     extern __shared__ uint32_t smem[];
     const int tau = threadIdx.x;
     const uint32_t h = cluster_rank();
@@ -173,9 +171,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const uint2 w0 = __ldg(psi + 1);
     cluster_barrier();  // both blocks have started before any remote store
 
-    uint32_t acc[1][E];
+    uint64_t T[E];  // sums of products with the key (see k_keyswitch)
 #pragma unroll
-    for (int e = 0; e < E; e++) acc[0][e] = 0;
+    for (int e = 0; e < E; e++) T[e] = 0;
     int buf = 0;
     for (int d0 = 0; d0 < ell; d0 += ND) {
         uint32_t x[ND][E];
@@ -203,18 +201,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
 #pragma unroll
         for (int o = 0; o < ND; o++) {
             const int d = d0 + o;
-            if (d < ell) {
-                const uint2* __restrict__ g = evk + ((size_t)d * k + prime) * (2 * kPairHalf) + h * kPairHalf;
-                const uint4* g4 = reinterpret_cast<const uint4*>(g + group_base<PL, LAST>(tau, 0));
+            if (o % 2 == 0) {
 #pragma unroll
-                for (int q = 0; q < E / 2; q++) {
-                    const uint4 W = __ldg(g4 + q);
-                    acc[0][2 * q] = mac_red(acc[0][2 * q], shoup_m(x[o][2 * q], W.x, W.y, m), m);
-                    acc[0][2 * q + 1] = mac_red(acc[0][2 * q + 1], shoup_m(x[o][2 * q + 1], W.z, W.w, m), m);
-                }
+                for (int e = 0; e < E; e++) T[e] = lazy_high(T[e], m);
+            }
+            if (d < ell) {
+                uint32_t v[E];
+                load_evk<PL>(evk + ((size_t)d * k + prime) * (2 * kPairHalf) + h * kPairHalf, tau, v);
+#pragma unroll
+                for (int e = 0; e < E; e++) T[e] += (uint64_t)x[o][e] * v[e];
             }
         }
     }
+    uint32_t acc[1][E];
+    const uint32_t pinv = B->pinv[prime];
+#pragma unroll
+    for (int e = 0; e < E; e++) acc[0][e] = mac_finish<true>(T[e], pinv, m);
     ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), tm);
     pair_finish(acc, recv, h, tau, p, __ldg(ipsi + 1), resid + ((size_t)job * k + prime) * (2 * kPairHalf));
 }

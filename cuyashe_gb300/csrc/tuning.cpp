@@ -29,12 +29,12 @@ namespace cy {
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
                           cudaStream_t st, int variant);
-cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint2* evk, int ell, uint64_t* out, int batch,
+cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* evk, int ell, uint64_t* out, int batch,
                             Workspace& ws, cudaStream_t st, int variant, int chunk_k, int lm);
-cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint2** d_evk);
+cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint32_t** d_evk);
 
 cy_status run_ntt_api(const Basis& B, uint32_t* res, int batch, bool inverse, cudaStream_t st, int variant);
-cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint2* evk, int ell, const uint64_t* c1,
+cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
                         const uint64_t* c2, uint64_t* out, int batch, bool do_relin, Workspace& ws, cudaStream_t st,
                         int ks_variant);
 
@@ -175,7 +175,7 @@ static cy_status tune_product(const Basis& B, bool centered, int batch, cudaStre
 // waves of that schedule, its keyswitch overlapping the tensor products of the
 // neighbouring chunks), with the tensor schedule already chosen. Timing the
 // keyswitch alone kept a schedule 3% slower in the multiply.
-static cy_status tune_keyswitch(const cy_yashe* y, const uint2* evk, int batch, cudaStream_t st) {
+static cy_status tune_keyswitch(const cy_yashe* y, const uint32_t* evk, int batch, cudaStream_t st) {
     const int n = y->ring->n, l64 = y->ring->l64;
     const size_t bytes = sizeof(uint64_t) * (size_t)batch * n * l64;
     std::vector<uint64_t> h1 = random_polys(batch, n, l64, y->ring->qbits, 3);
@@ -242,8 +242,8 @@ cy_status cy_yashe_autotune(cy_yashe* y, int batch, cy_stream_t stream) {
     cudaStream_t st = (cudaStream_t)stream;
     CY_TRY(tune_product(r->mul, false, batch, st));
     CY_TRY(tune_product(y->tensor, true, batch, st));
-    const uint2* evk = y->d_evk;
-    uint2* tmp = nullptr;
+    const uint32_t* evk = y->d_evk;
+    uint32_t* tmp = nullptr;
     if (!evk) {  // no keys yet: an evaluation key of random values has the same cost
         std::vector<uint64_t> h = random_polys(y->ell, r->n, r->l64, r->qbits, 4);
         CY_TRY(prepare_evk(y->relin, h.data(), y->ell, r->n, r->l64, &tmp));
