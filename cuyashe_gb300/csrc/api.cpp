@@ -130,25 +130,24 @@ static const char* epi_name(int mode) {
     return mode == EPI_YASHE ? "epi_yashe" : mode == EPI_DECRYPT ? "epi_decrypt" : "epi_modq";
 }
 
-// Epilogues specialised for the basis's prime count are used unless this is set.
+// The epilogues with constants as a parameter are used unless this is set.
 static std::atomic<int> g_epi_generic{0};
 
-// ICRT epilogue of basis B over `nj` jobs of residues [job][k][N] into `out`: the
-// kernel specialised for B's prime count (constants passed by value) when there
-// is one, else the generic kernel.
+// ICRT epilogue of basis B over `nj` jobs of residues [job][k][N] into `out`.
 // lm: outputs limb-major ([job][limb][N]), for the keyswitch that follows in an
-// HE multiply (its digit loads then cover consecutive words)
+// HE multiply (its digit loads then cover consecutive words).
+// any_x: residues of any X (cy_icrt), not only of |X| < M/4: k_epi's 64-bit estimate
+// of v decides up to the ends of (-M/2, M/2)
 static cy_status launch_epi(const Basis& B, const uint32_t* resid, void* out, int nj, cudaStream_t st,
-                            const char* name, int lm = 0) {
+                            const char* name, int lm = 0, bool any_x = false) {
     const BasisDev* Bd = B.d;
     unsigned long long fl = epi_frac_limit();
     const long long coefs = (long long)nj * B.h.n;
-    if (B.epi && !g_epi_generic.load()) {
-        const long long per = (long long)kEpiThreads * B.epi->coefs_per_thread;
+    if (!any_x && !g_epi_generic.load()) {
         void* args[] = {(void*)B.epi_param.data(), (void*)&Bd, (void*)&resid, (void*)&out, (void*)&nj, (void*)&fl,
                         (void*)&lm};
-        return launch(B.epi->func, name, B.h.logn, dim3((unsigned)((coefs + per - 1) / per)), dim3(kEpiThreads), 0,
-                      st, args);
+        return launch(B.epi->func, name, B.h.logn, dim3((unsigned)((coefs + kEpiThreads - 1) / kEpiThreads)),
+                      dim3(kEpiThreads), 0, st, args);
     }
     void* args[] = {(void*)&Bd, (void*)&resid, (void*)&out, (void*)&nj, (void*)&fl, (void*)&lm};
     return launch(epi_kernel(B.h.l32, B.h.mode), name, B.h.logn, dim3(epi_blocks(coefs, B.h.l32)), dim3(kEpiThreads),
@@ -723,7 +722,7 @@ cy_status cy_icrt(cy_ring* r, const uint32_t* d_res, uint64_t* d_x, int batch, c
     for (int j0 = 0; j0 < batch; j0 += 65536) {
         int nj = std::min(65536, batch - j0);
         const uint32_t* rj = d_res + (size_t)j0 * B.h.k * r->n;
-        CY_TRY(launch_epi(B, rj, d_x + (size_t)j0 * r->n * r->l64, nj, (cudaStream_t)stream, "epi_modq"));
+        CY_TRY(launch_epi(B, rj, d_x + (size_t)j0 * r->n * r->l64, nj, (cudaStream_t)stream, "epi_modq", 0, true));
     }
     return CY_OK;
 }

@@ -45,6 +45,7 @@ struct BasisDev {
     uint32_t t;        // plaintext modulus (YASHE / DECRYPT)
     uint32_t centered; // inputs are taken as symmetric representatives (YASHE)
     uint64_t mu;       // floor(2^(32*l32+37) / q')
+    uint64_t mu45;     // floor(2^(32*l32+44) / q')
     uint32_t qn[L32MAX];       // q'
     uint32_t q[L32MAX];        // q
     uint32_t qhalf[L32MAX];    // (q-1)/2

@@ -33,19 +33,19 @@ const KernelSet& kernel_variant(int logn, int v);
 // Tuned operations (keys of the autotuner's table).
 enum TuneOp { TUNE_MUL = 0, TUNE_MULC = 1, TUNE_KS = 2, TUNE_NTT = 3, TUNE_OPS = 4 };
 
-// ICRT epilogue for `l32` words of q and epilogue mode (EpiMode).
+// ICRT epilogue for `l32` words of q and epilogue mode (EpiMode) with its constants
+// in shared memory (residues of any X: cy_icrt; comparison).
 void* epi_kernel(int l32, int mode);
 
-// Epilogue specialised for a prime count (k_epi_k): the kernel, the size of its
-// first parameter (the basis constants by value) and the function that writes
-// that parameter from a basis. Null when (l32, k, mode) has no specialisation.
-struct EpiSpecial {
+// Epilogue with the constants of its basis as the first parameter, by value
+// (k_epi_c): the kernel, that parameter's size and the function that writes it. The
+// common parameter sets have one compiled for their prime count.
+struct EpiConstKernel {
     void* func;
     size_t param_bytes;
     void (*fill)(const BasisDev& h, void* param);
-    int coefs_per_thread;
 };
-const EpiSpecial* epi_special(int l32, int k, int mode);
+const EpiConstKernel* epi_const(int l32, int k, int mode);
 
 // Bytes of shared memory an exchange region set needs, and whether the kernel
 // alternates two regions (one barrier per exchange) or reuses one (two).

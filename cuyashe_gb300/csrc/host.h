@@ -61,7 +61,7 @@ struct Basis {
     BasisDev* d = nullptr;
     uint32_t* d_ninv = nullptr;  // [k][4]: N^-1 mod p_i, N^-1 psi_i^-(NMAX/2), each with its Shoup companion
     int crt_bits = 0;
-    const EpiSpecial* epi = nullptr;     // specialised epilogue of this basis, if any
+    const EpiConstKernel* epi = nullptr;   // epilogue of this basis
     std::vector<unsigned char> epi_param;  // its parameter block (constants by value)
     Basis() = default;
     Basis(const Basis&) = delete;

@@ -1,0 +1,14 @@
+// Epilogues for any prime count, q of 1 to 5 words (k_epi_c with K = 0).
+#include "kernels.cuh"
+
+namespace cy {
+
+#define CY_EPI_ANY(L, MODE) {(void*)k_epi_c<L, MODE, 0>, sizeof(EpiConst<L, KMAX>), fill_epi_const<L, KMAX>}
+#define CY_EPI_ROW(L) {CY_EPI_ANY(L, EPI_MODQ), CY_EPI_ANY(L, EPI_YASHE), CY_EPI_ANY(L, EPI_DECRYPT)}
+
+const EpiConstKernel* epi_any1(int l32, int mode) {
+    static const EpiConstKernel table[][3] = {CY_EPI_ROW(1), CY_EPI_ROW(2), CY_EPI_ROW(3), CY_EPI_ROW(4), CY_EPI_ROW(5)};
+    return &table[l32 - 1][mode];
+}
+
+}  // namespace cy

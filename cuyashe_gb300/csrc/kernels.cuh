@@ -1019,25 +1019,38 @@ __global__ void __launch_bounds__(256) k_epi(const BasisDev* __restrict__ B, con
 }
 
 // --------------------------------------------------------------------------
-// k_epi_k: the MODQ / YASHE epilogue for a compile-time prime count K. The
-// basis constants travel by value as a kernel parameter (constant bank), so each
-// constant is a uniform operand of the instruction that uses it: no shared-memory
-// staging, no address arithmetic, no guards. The prime loop is straight-line
-// code with a carry pass every four primes (four products of < 2^62 plus a
-// normalised word stay below 2^64).
+// k_epi_c: the epilogue with its constants in the constant bank. The constants of a
+// basis travel by value as a kernel parameter, so each is a uniform operand of the
+// instruction that uses it: no shared-memory staging, no barrier, no address
+// arithmetic per thread. K > 0: the prime count at compile time (straight-line code);
+// K = 0: any count, in groups of four (a carry pass each: four products of a residue
+// and a word plus a normalised word stay below 2^64) with the next group's residues in
+// flight, and a rest of up to three.
+//
+// The kernel is bound by the fma-heavy pipe (a wide or high product takes four of its
+// cycles, a low one two), so what a prime costs there was cut: v = round(sum y_i / p_i)
+// is summed in 26-bit fixed point from 13-bit factors (one shift and one low product
+// instead of a wide and a high one): each term is low by at most 2^-13 + 2^-13, the sum
+// of 40 by less than 0.01, and |X| < M/4 leaves 0.25. (cy_icrt takes residues of any X
+// and keeps k_epi's 64-bit sum.) Barrett's quotient is formed from 32-bit pieces
+// of 45-bit operands and is at most one low, so one conditional subtraction ends it.
+// Measured with those of k_epi_k, the kernel this replaces, at N = 4096, 127-bit q.
 // --------------------------------------------------------------------------
-template <int L, int K>
+template <int L>
+struct __align__(16) EpiPrimeC {
+    uint32_t p, np, ycon, ycon_sh;
+    uint32_t g, F0, F1, pad;  // floor(2^43 / p); R_i / q in units of 2^-64 (YASHE)
+    uint32_t A0[L];
+};
+template <int L, int KS>
 struct EpiConst {
-    uint32_t p[K], np[K], ycon[K], ycon_sh[K], fhi[K], flo[K], F0[K], F1[K];
-    uint32_t A0[K][L];
+    EpiPrimeC<L> pr[KS];
     uint32_t B0[L], qn[L], qhalf_n[L];
     uint32_t FM[2];
-    uint64_t mu;
-    int shift, l64, logn;
+    uint32_t mu_lo, mu_hi;  // floor(2^(32 L + 44) / q')
+    uint32_t t;
+    int shift, logn, k;
 };
-
-// x in [0, 2m) -> [0, m) with nm = -m
-__device__ __forceinline__ uint32_t red_neg(uint32_t x, uint32_t nm) { return __viaddmin_u32(x, nm, x); }
 
 // The exact YASHE rounding of yashe_round_exact with the constants read from
 // the basis in global memory (the rare path of k_epi_k).
@@ -1061,111 +1074,211 @@ __device__ __noinline__ uint64_t yashe_round_exact_g(const BasisDev* __restrict_
     return barrett<L>(c1, B->qn, B->mu, rdummy);
 }
 
-template <int L, int MODE, int K, int C>
-__global__ void __launch_bounds__(256) k_epi_k(const __grid_constant__ EpiConst<L, K> P,
+// Carry chains over 32-bit words (consecutive volatile statements: the compiler emits
+// no other instruction that touches the carry flag in between).
+__device__ __forceinline__ uint32_t sub_cc(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm volatile("sub.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t subc_cc(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm volatile("subc.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t sub_borrow() {  // all ones if the chain borrowed
+    uint32_t r;
+    asm volatile("subc.u32 %0, 0, 0;" : "=r"(r));
+    return r;
+}
+
+// x (normalised columns, below 2^(32 L + 37)) modulo q' (top bit of word L-1 set):
+// returns the quotient, writes the remainder to r. With x1 = floor(x / 2^(32 L - 8))
+// and mu = floor(2^(32 L + 44) / q') below 2^46, Q = floor(x1 mu / 2^52) is the
+// quotient or one less (the two roundings cost less than 2^-6 together).
+template <int L>
+__device__ __forceinline__ uint64_t barrett_c(const Cols<L>& x, const uint32_t (&qn)[L], uint32_t mu_lo,
+                                              uint32_t mu_hi, uint32_t (&r)[L]) {
+    const uint32_t t1 = (uint32_t)x.c[L], t0 = (uint32_t)x.c[L - 1];
+    const uint32_t xl = __funnelshift_l(t0, t1, 8);
+    const uint32_t xh = __funnelshift_l(t1, (uint32_t)x.c[L + 1], 8);
+    const uint64_t S = (uint64_t)xh * mu_lo + (uint64_t)xl * mu_hi + __umulhi(xl, mu_lo);
+    uint64_t Q = (S >> 20) + ((uint64_t)(xh * mu_hi) << 12);
+    const uint32_t Ql = (uint32_t)Q, Qh = (uint32_t)(Q >> 32);
+    uint32_t P[L + 1];
+    uint64_t carry = 0;
+#pragma unroll
+    for (int w = 0; w < L; w++) {
+        const uint64_t lo = (uint64_t)Ql * qn[w] + (uint32_t)carry;
+        P[w] = (uint32_t)lo;
+        carry = (uint64_t)Qh * qn[w] + ((lo >> 32) + (carry >> 32));
+    }
+    P[L] = (uint32_t)carry;
+    uint32_t rr[L + 1], t[L + 1];
+    rr[0] = sub_cc((uint32_t)x.c[0], P[0]);
+#pragma unroll
+    for (int w = 1; w <= L; w++) rr[w] = subc_cc((uint32_t)x.c[w], P[w]);
+    t[0] = sub_cc(rr[0], qn[0]);
+#pragma unroll
+    for (int w = 1; w < L; w++) t[w] = subc_cc(rr[w], qn[w]);
+    t[L] = subc_cc(rr[L], 0u);
+    const bool keep = sub_borrow() != 0;
+#pragma unroll
+    for (int w = 0; w < L; w++) r[w] = keep ? rr[w] : t[w];
+    return keep ? Q : Q + 1;
+}
+
+// x in [0, 2m) -> [0, m) with nm = -m
+__device__ __forceinline__ uint32_t red_neg(uint32_t x, uint32_t nm) { return __viaddmin_u32(x, nm, x); }
+
+template <int L, int MODE, int K>
+__global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<L, (K ? K : KMAX)> P,
                                                const BasisDev* __restrict__ B, const uint32_t* __restrict__ resid,
                                                void* __restrict__ out, int njobs, unsigned long long frac_limit,
                                                int lm) {
-    static_assert(MODE == EPI_MODQ || MODE == EPI_YASHE, "mod-q and YASHE epilogues only");
-    const int logn = P.logn;
+    constexpr int L64 = (L + 1) / 2;
+    const int logn = P.logn, shift = P.shift;
     const int n = 1 << logn;
-    const long long total = (long long)njobs << logn;
-    const long long base = (long long)blockIdx.x * blockDim.x * C + threadIdx.x;
-    if (base >= total) return;
-    const uint32_t* r0[C];
-    uint64_t* dst[C];
-    bool store[C];
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-        long long idx = base + (long long)c * blockDim.x;  // coalesced across the warp for every c
-        store[c] = idx < total;
-        if (!store[c]) idx = base;  // computed and not written
-        const long long job = idx >> logn;
-        const int coef = (int)(idx & (n - 1));
-        r0[c] = resid + (size_t)job * K * n + coef;
-        dst[c] = reinterpret_cast<uint64_t*>(out) + (size_t)job * n * P.l64 +
-                 (lm ? (size_t)coef : (size_t)coef * P.l64);
-    }
-    const size_t lstride = lm ? (size_t)n : 1;
-    uint32_t r[K][C];
-#pragma unroll
-    for (int i = 0; i < K; i++)
-#pragma unroll
-        for (int c = 0; c < C; c++) r[i][c] = __ldcg(r0[c] + (size_t)i * n);
+    const int k = K ? K : P.k;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)njobs << logn) return;
+    const long long job = idx >> logn;
+    const int coef = (int)(idx & (n - 1));
+    const uint32_t* r0 = resid + (size_t)job * k * n + coef;
 
-    Cols<L> c0[C];
-    Cols<2> fz[C];
-    uint64_t vacc[C];
+    Cols<L> x;   // sum y_i A0_i
+    Cols<2> z;   // YASHE: Z = sum y_i F_i in 32-bit columns
+    uint32_t vs = 0x2000000u;  // sum y_i / p_i + 1/2 in units of 2^-26
+    x.zero();
+    z.zero();
+    auto absorb = [&](const EpiPrimeC<L>& E, uint32_t res) {
+        const uint32_t y = red_neg(__umulhi(res, E.ycon_sh) * E.np + res * E.ycon, E.np);
+        vs += (y >> 17) * E.g;
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-        c0[c].zero();
-        fz[c].zero();
-        vacc[c] = 0;
-    }
-#pragma unroll
-    for (int i = 0; i < K; i++) {
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-            const uint32_t y = red_neg(shoup(r[i][c], P.ycon[i], P.ycon_sh[i], P.p[i]), P.np[i]);
-            vacc[c] += (uint64_t)y * P.fhi[i] + __umulhi(y, P.flo[i]);  // sum y_i/p_i in 2^-32 units
-#pragma unroll
-            for (int w = 0; w < L; w++) c0[c].c[w] += (uint64_t)y * P.A0[i][w];
-            if (MODE == EPI_YASHE) {
-                fz[c].c[0] += (uint64_t)y * P.F0[i];
-                fz[c].c[1] += (uint64_t)y * P.F1[i];
-            }
-        }
-        if (i % 4 == 3 && i + 1 < K) {
-#pragma unroll
-            for (int c = 0; c < C; c++) {
-                c0[c].norm();
-                if (MODE == EPI_YASHE) fz[c].norm();
-            }
-        }
-    }
-    // products since the last carry pass; v adds one more
-    constexpr bool NORM_BEFORE_V = (K % 4 == 0);
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-        const uint32_t v = (uint32_t)((vacc[c] + 0x80000000ULL) >> 32);  // X = sum y_i Mhat_i - v M
-        Cols<L>& x = c0[c];
-        if (NORM_BEFORE_V) x.norm();
-#pragma unroll
-        for (int w = 0; w < L; w++) x.c[w] += (uint64_t)v * P.B0[w];
+        for (int w = 0; w < L; w++) x.c[w] += (uint64_t)y * E.A0[w];
         if (MODE == EPI_YASHE) {
-            Cols<2>& z = fz[c];
-            if (NORM_BEFORE_V) z.norm();
-            z.c[0] += (uint64_t)v * P.FM[0];
-            z.c[1] += (uint64_t)v * P.FM[1];
-            z.c[1] += 0x80000000u;  // + 1/2
-            z.norm();
-            const uint64_t frac = z.c[0] | (z.c[1] << 32);
-            uint64_t Q2 = z.c[2] | (z.c[3] << 32);  // round(S/q) + v, S = sum y_i R_i - v R_M
-            if (frac >= frac_limit) Q2 = yashe_round_exact_g<L>(B, r0[c], (size_t)n, v);
-            // x += Q2 << shift (each added word < 2^32: the columns stay below 2^64)
-            const uint64_t lo = Q2 << P.shift;
-            const uint64_t hi = P.shift ? (Q2 >> (64 - P.shift)) : 0;
-            x.c[0] += (uint32_t)lo;
-            x.c[1] += (uint32_t)(lo >> 32);
-            x.c[2] += hi;
+            z.c[0] += (uint64_t)y * E.F0;
+            z.c[1] += (uint64_t)y * E.F1;
         }
-        x.norm();
-        uint32_t rm[L];
-        barrett<L>(x, P.qn, P.mu, rm);  // rm = (result mod q) << shift
-        if (!store[c]) continue;
-        uint32_t o[L];
+    };
+    if constexpr (K > 0) {
+        uint32_t r[K];
 #pragma unroll
-        for (int w = 0; w < L; w++) {
-            const uint32_t nx = (w + 1 < L) ? rm[w + 1] : 0u;
-            o[w] = __funnelshift_r(rm[w], nx, P.shift);
+        for (int i = 0; i < K; i++) r[i] = __ldcg(r0 + (size_t)i * n);
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            absorb(P.pr[i], r[i]);
+            if (i % 4 == 3 && i + 1 < K) {
+                x.norm();
+                if (MODE == EPI_YASHE) z.norm();
+            }
+        }
+    } else {
+        const int rest = k & 3, whole = k - rest;
+        uint32_t cur[4], nxt[4];
+        auto load = [&](int i, uint32_t(&d)[4]) {  // past the last prime: its residue again, not used
+#pragma unroll
+            for (int j = 0; j < 4; j++) d[j] = __ldcg(r0 + (size_t)min(i + j, k - 1) * n);
+        };
+        load(0, cur);
+#pragma unroll 1
+        for (int i = 0; i < whole; i += 4) {
+            load(i + 4, nxt);
+#pragma unroll
+            for (int j = 0; j < 4; j++) absorb(P.pr[i + j], cur[j]);
+            x.norm();
+            if (MODE == EPI_YASHE) z.norm();
+#pragma unroll
+            for (int j = 0; j < 4; j++) cur[j] = nxt[j];
         }
 #pragma unroll
-        for (int j = 0; j < (L + 1) / 2; j++) {
-            const uint64_t lo32 = o[2 * j];
-            const uint64_t hi32 = (2 * j + 1 < L) ? o[2 * j + 1] : 0u;
-            if (j < P.l64) dst[c][j * lstride] = lo32 | (hi32 << 32);
+        for (int j = 0; j < 3; j++)
+            if (j < rest) absorb(P.pr[whole + j], cur[j]);
+    }
+    // every table prime is at least 2^18 below 2^30: four products leave 2^50 for what follows
+    const uint32_t v = vs >> 26;  // X = sum y_i Mhat_i - v M
+#pragma unroll
+    for (int w = 0; w < L; w++) x.c[w] += (uint64_t)v * P.B0[w];
+    if (MODE == EPI_YASHE) {
+        z.c[0] += (uint64_t)v * P.FM[0];
+        z.c[1] += (uint64_t)v * P.FM[1] + 0x80000000u;  // + 1/2
+        z.norm();
+        const uint64_t frac = z.c[0] | (z.c[1] << 32);
+        uint64_t Q2 = z.c[2] | (z.c[3] << 32);  // round(S/q) + v, S = sum y_i R_i - v R_M
+        if (frac >= frac_limit) Q2 = yashe_round_exact_g<L>(B, r0, (size_t)n, v);
+        // x += Q2 << shift
+        const uint64_t lo = Q2 << shift;
+        const uint64_t hi = shift ? (Q2 >> (64 - shift)) : 0;
+        x.c[0] += (uint32_t)lo;
+        x.c[1] += (uint32_t)(lo >> 32);
+        x.c[2] += hi;
+    }
+    x.norm();
+    uint32_t qn[L], rm[L];
+#pragma unroll
+    for (int w = 0; w < L; w++) qn[w] = P.qn[w];
+    barrett_c<L>(x, qn, P.mu_lo, P.mu_hi, rm);  // rm = (result mod q) << shift
+    if constexpr (MODE == EPI_DECRYPT) {
+        Cols<L> c2;
+#pragma unroll
+        for (int w = 0; w < L; w++) c2.c[w] = (uint64_t)P.t * rm[w] + P.qhalf_n[w];
+        c2.c[L] = c2.c[L + 1] = 0;
+        c2.norm();
+        uint32_t rd[L];
+        uint64_t Q = barrett_c<L>(c2, qn, P.mu_lo, P.mu_hi, rd);  // round(t x / q) in [0, t]
+        if (Q >= P.t) Q -= P.t;
+        reinterpret_cast<uint64_t*>(out)[idx] = Q;
+    } else {
+        uint64_t o[L64];
+#pragma unroll
+        for (int j = 0; j < L64; j++) {
+            auto word = [&](int w) { return w < L ? __funnelshift_r(rm[w], w + 1 < L ? rm[w + 1] : 0u, shift) : 0u; };
+            o[j] = (uint64_t)word(2 * j + 1) << 32 | word(2 * j);
+        }
+        uint64_t* dst = reinterpret_cast<uint64_t*>(out) + (size_t)job * n * L64;
+        if (lm) {
+#pragma unroll
+            for (int j = 0; j < L64; j++) dst[(size_t)j * n + coef] = o[j];
+        } else if constexpr (L64 % 2 == 0) {
+            ulonglong2* d2 = reinterpret_cast<ulonglong2*>(dst + (size_t)coef * L64);
+#pragma unroll
+            for (int j = 0; j < L64 / 2; j++) d2[j] = make_ulonglong2(o[2 * j], o[2 * j + 1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < L64; j++) dst[(size_t)coef * L64 + j] = o[j];
         }
     }
+}
+
+// Constants of a basis for k_epi_c (K = 0 or KS = K primes).
+template <int L, int KS>
+void fill_epi_const(const BasisDev& h, void* param) {
+    static_assert(sizeof(EpiConst<L, KS>) <= 4096, "fits a kernel parameter");
+    EpiConst<L, KS>& c = *static_cast<EpiConst<L, KS>*>(param);
+    for (int i = 0; i < h.k; i++) {
+        EpiPrimeC<L>& e = c.pr[i];
+        e.p = h.p[i];
+        e.np = 0u - h.p[i];
+        e.ycon = h.ycon[i];
+        e.ycon_sh = h.ycon_sh[i];
+        e.g = (uint32_t)((1ull << 43) / h.p[i]);
+        e.F0 = h.frac[i][0];
+        e.F1 = h.frac[i][1];
+        for (int w = 0; w < L; w++) e.A0[w] = h.A0[i][w];
+    }
+    for (int w = 0; w < L; w++) {
+        c.B0[w] = h.B0[w];
+        c.qn[w] = h.qn[w];
+        c.qhalf_n[w] = h.qhalf_n[w];
+    }
+    c.FM[0] = h.frac_m[0];
+    c.FM[1] = h.frac_m[1];
+    c.mu_lo = (uint32_t)h.mu45;
+    c.mu_hi = (uint32_t)(h.mu45 >> 32);
+    c.t = h.t;
+    c.shift = h.shift;
+    c.logn = h.logn;
+    c.k = h.k;
 }
 
 }  // namespace cy

@@ -98,12 +98,11 @@ extern "C" cy_status cy_polymul_noalloc(cy_ring* r, const uint64_t* d_a, const u
     // blocks_per_prime > 1 for schedules that run one product on a pair of blocks
     CY_TRY(launch_noalloc(ks.mul_for(B.h.l64, false), "mul_noalloc", B.h.logn, dim3(batch * ks.blocks_per_prime, k),
                           dim3(ks.threads), ks.smem_mul, st, args));
-    void* epi = epi_kernel(B.h.l32, EPI_MODQ);
     unsigned long long fl = 0;  // mod-q epilogue: no rounding estimate
     int lm = 0;                 // outputs in the [job][N][limb] layout
-    void* eargs[] = {(void*)&Bd, (void*)&scratch, (void*)&d_c, (void*)&batch, (void*)&fl, (void*)&lm};
+    void* eargs[] = {(void*)B.epi_param.data(), (void*)&Bd, (void*)&scratch, (void*)&d_c, (void*)&batch, (void*)&fl,
+                     (void*)&lm};
     const long long threads = (long long)batch * n;
-    const long long per = 256ll * epi_coefs_per_thread(B.h.l32);
-    return launch_noalloc(epi, "epi_modq_noalloc", B.h.logn, dim3((unsigned)((threads + per - 1) / per)), dim3(256),
+    return launch_noalloc(B.epi->func, "epi_modq_noalloc", B.h.logn, dim3((unsigned)((threads + 255) / 256)), dim3(256),
                           0, st, eargs);
 }

@@ -193,6 +193,7 @@ cy_status basis_constants(BasisDev& h, int* crt_bits, int n, const BigUInt& q, i
     const BigUInt qn = q.shl(h.shift);
     const BigUInt mu = BigUInt::pow2(32 * h.l32 + 37) / qn;
     h.mu = mu.low64();
+    h.mu45 = (BigUInt::pow2(32 * h.l32 + 44) / qn).low64();
     qn.to_words32(h.qn, L32MAX);
     q.to_words32(h.q, L32MAX);
     const BigUInt qhalf = (q - BigUInt(1)).shr(1);
@@ -288,11 +289,10 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
         ninv[4 * i + 2] = vw;
         ninv[4 * i + 3] = shoup_of(vw, p);
     }
-    b.epi = epi_special(b.h.l32, b.h.k, b.h.mode);
-    if (b.epi) {
-        b.epi_param.assign(b.epi->param_bytes, 0);
-        b.epi->fill(b.h, b.epi_param.data());
-    }
+    b.epi = epi_const(b.h.l32, b.h.k, b.h.mode);
+    if (!b.epi) return set_error(CY_ERR_INTERNAL, "missing epilogue");
+    b.epi_param.assign(b.epi->param_bytes, 0);
+    b.epi->fill(b.h, b.epi_param.data());
     CY_CUDA(cudaMalloc(&b.d, sizeof(BasisDev)));
     CY_CUDA(cudaMemcpy(b.d, &b.h, sizeof(BasisDev), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMalloc(&b.d_ninv, sizeof(uint32_t) * ninv.size()));

@@ -63,3 +63,20 @@ def test_residues_of_edge_coefficients(bits):
     torch.cuda.synchronize()
     for i, p in enumerate(R.primes):
         assert [int(v) for v in res[0, i]] == [x % p for x in a]
+
+
+@pytest.mark.parametrize("bits", [31, 62, 95, 127, 160, 190, 224, 250, 288, 320, 352, 380])
+def test_largest_products(bits):
+    """All coefficients q - 1: the product's coefficients run from -(n - 2)(q - 1)^2 to
+    n (q - 1)^2, the ends of the range the ICRT's estimate of the multiple of M must
+    resolve; every number of 32-bit words of q."""
+    import torch
+
+    import cuyashe_gb300 as cy
+
+    n, q = 256, (1 << bits) - 1
+    R = cy.Ring(n, q)
+    a = [q - 1] * n
+    out = R.download(R.polymul(R.upload([a]), R.upload([a])))
+    torch.cuda.synchronize()
+    assert list(out[0]) == ring.polymul_mod(a, a, q)
