@@ -226,8 +226,7 @@ static cy_status product_chunk(const Basis& B, const KernelSet& ks, bool centere
                                long long a_stride, const uint64_t* bj, long long b_stride, void* oj, int nj,
                                uint32_t* resid, cudaStream_t st, int lm = 0) {
     const int k = B.h.k;
-    const BasisDev* Bd = B.d;
-    void* args[] = {(void*)&Bd, (void*)&aj, (void*)&a_stride, (void*)&bj, (void*)&b_stride, (void*)&resid};
+    void* args[] = {(void*)&B.prod, (void*)&aj, (void*)&a_stride, (void*)&bj, (void*)&b_stride, (void*)&resid};
     CY_TRY(launch(ks.mul_for(B.h.l64, centered), centered ? "mul_centered" : "mul", B.h.logn,
                   dim3(nj * ks.blocks_per_prime, k), dim3(ks.threads), ks.smem_mul, st, args));
     return launch_epi(B, resid, oj, nj, st, epi_name(B.h.mode), lm);
@@ -238,9 +237,8 @@ static cy_status product_chunk(const Basis& B, const KernelSet& ks, bool centere
 static cy_status keyswitch_chunk(const Basis& B, const KernelSet& ks, int sel, const uint64_t* cj, const uint32_t* evk,
                                  int ell, uint64_t* oj, int nj, uint32_t* resid, cudaStream_t st, int lm = 0) {
     const int k = B.h.k;
-    const BasisDev* Bd = B.d;
     int cs = lm ? 1 : B.h.l64, ls = lm ? B.h.n : 1;  // limb w of coefficient i at [i * cs + w * ls]
-    void* args[] = {(void*)&Bd, (void*)&cj, (void*)&evk, (void*)&ell, (void*)&resid, (void*)&cs, (void*)&ls};
+    void* args[] = {(void*)&B.prod, (void*)&cj, (void*)&evk, (void*)&ell, (void*)&resid, (void*)&cs, (void*)&ls};
     CY_TRY(launch(ks.ks_for(B.h.l64, sel), "keyswitch", B.h.logn, dim3(nj * ks.blocks_per_prime, k),
                   dim3(ks.threads), ks.smem_ks[sel], st, args));
     return launch_epi(B, resid, oj, nj, st, epi_name(B.h.mode));
@@ -360,7 +358,6 @@ static cy_status run_ntt(const Basis& B, uint32_t* res, int batch, bool inverse,
     if (batch == 0) return CY_OK;
     const KernelSet& ks =
         kernel_variant(B.h.logn, variant >= 0 ? variant : tuned_variant(B.h.logn, B.h.l64, TUNE_NTT));
-    const BasisDev* Bd = B.d;
     const uint32_t* ninv = B.d_ninv;
     const long long rows = (long long)batch * B.h.k * (B.h.n / 64);
     if (inverse && ks.intt_tma && B.h.logn == 12 && ntt_tma_usable(res, rows)) {  // input tiles by TMA
@@ -369,19 +366,19 @@ static cy_status run_ntt(const Basis& B, uint32_t* res, int batch, bool inverse,
         int* err = nullptr;
         CY_TRY(intt_tma_prepare(res, rows, B.h.k, batch, &map, &grid, &err));
         uint32_t spin = ntt_tma_spin_limit(), extra = ntt_tma_extra_tx();
-        void* args[] = {(void*)&Bd, (void*)&map, (void*)&res, (void*)&ninv, (void*)&batch, (void*)&err, (void*)&spin,
+        void* args[] = {(void*)&B.prod, (void*)&map, (void*)&res, (void*)&ninv, (void*)&batch, (void*)&err, (void*)&spin,
                         (void*)&extra};
         return launch(intt_tma_kernel(), "ntt_inv", B.h.logn, grid, dim3(64), intt_tma_smem(), st, args);
     }
     if (ks.ntt_jobs_per_block == 1) {  // k_ntt1: grid (jobs, primes)
-        void* args[] = {(void*)&Bd, (void*)&res, (void*)&ninv, (void*)&batch};
+        void* args[] = {(void*)&B.prod, (void*)&res, (void*)&ninv, (void*)&batch};
         return launch(ks.ntt[inverse ? 1 : 0], inverse ? "ntt_inv" : "ntt_fwd", B.h.logn, dim3(batch, B.h.k),
                       dim3(ks.threads), ks.smem_ntt, st, args);
     }
     for (int j0 = 0; j0 < batch; j0 += 2 * 65535) {  // two jobs per block
         int nj = std::min(2 * 65535, batch - j0);
         uint32_t* rj = res + (size_t)j0 * B.h.k * B.h.n;
-        void* args[] = {(void*)&Bd, (void*)&rj, (void*)&ninv, (void*)&nj};
+        void* args[] = {(void*)&B.prod, (void*)&rj, (void*)&ninv, (void*)&nj};
         CY_TRY(launch(ks.ntt[inverse ? 1 : 0], inverse ? "ntt_inv" : "ntt_fwd", B.h.logn, dim3(B.h.k, (nj + 1) / 2),
                       dim3(ks.threads), ks.smem_ntt, st, args));
     }

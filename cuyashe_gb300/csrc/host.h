@@ -59,6 +59,7 @@ const std::vector<uint32_t>& table_primes();  // host-only, no CUDA
 struct Basis {
     BasisDev h{};
     BasisDev* d = nullptr;
+    ProdParams prod{};  // first parameter of the product, keyswitch and transform kernels
     uint32_t* d_ninv = nullptr;  // [k][4]: N^-1 mod p_i, N^-1 psi_i^-(NMAX/2), each with its Shoup companion
     int crt_bits = 0;
     const EpiConstKernel* epi = nullptr;   // epilogue of this basis

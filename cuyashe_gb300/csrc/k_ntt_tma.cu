@@ -130,7 +130,7 @@ __device__ __forceinline__ void write_row(uint8_t* t, int r, const uint32_t (&x)
 // up waiting for a tile (spin_limit polls). `extra_tx` > 0 only in the test of
 // that path (the tile's barrier then waits for bytes that never come).
 __global__ void __launch_bounds__(64, 10)
-    k_intt_tma(const BasisDev* __restrict__ B, const __grid_constant__ CUtensorMap map, uint32_t* __restrict__ res,
+    k_intt_tma(const __grid_constant__ ProdParams M, const __grid_constant__ CUtensorMap map, uint32_t* __restrict__ res,
                const uint32_t* __restrict__ ninv, int njobs, int* __restrict__ err, uint32_t spin_limit,
                uint32_t extra_tx) {
     extern __shared__ uint8_t smem_raw[];
@@ -138,10 +138,10 @@ __global__ void __launch_bounds__(64, 10)
     uint8_t* tile = smem_raw + ((1024u - (tma::saddr(smem_raw) & 1023u)) & 1023u);  // the swizzle's 1024-byte period
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
-    const int k = B->k;
-    const Mod m = load_mod(B, prime);
-    const uint2* __restrict__ tw = B->ipsi[prime];
-    const uint2* __restrict__ twr = B->ipsi_r[prime];
+    const int k = M.k;
+    const Mod m = load_mod(M.pr[prime]);
+    const uint2* __restrict__ tw = table_of(M.ipsi, prime);
+    const uint2* __restrict__ twr = rows_of(M.ipsi_r, prime);
     const int step = gridDim.x;
     int job = blockIdx.x;
     if (tau == 0) {

@@ -46,6 +46,11 @@ __device__ __forceinline__ Mod load_mod(const BasisDev* __restrict__ B, int i) {
     return m;
 }
 
+// The tables of prime i (ProdParams).
+__device__ __forceinline__ const uint2* table_of(const uint2* base, int i) { return base + (size_t)i * NMAX; }
+__device__ __forceinline__ const uint2* rows_of(const uint2* base, int i) { return base + (size_t)i * ROWS_WORDS; }
+__device__ __forceinline__ Mod load_mod(const PrimeParam& q) { return Mod{q.p, q.p2, q.np, q.np2}; }
+
 // a + b reduced from [0, 4p) to [0, 2p) (a, b in [0, 2p)): one add, one add-then-min
 __device__ __forceinline__ uint32_t mac_red(uint32_t a, uint32_t b, const Mod& m) {
     return __viaddmin_u32(a, b, a + b + m.np2);
@@ -64,6 +69,10 @@ __device__ __forceinline__ PrimeCtx load_prime_ctx(const BasisDev* __restrict__ 
     c.pinv = B->pinv[i];
     c.cadd = c.m.p2 - B->qmont[i];
     return c;
+}
+
+__device__ __forceinline__ PrimeCtx load_prime_ctx(const PrimeParam& q) {
+    return PrimeCtx{q.p, q.pinv, q.cadd, load_mod(q)};
 }
 
 // x 2^-32 mod p in (0, 4p) (valid forward-NTT input) from T = x + a multiple of p,
@@ -86,7 +95,7 @@ __device__ __forceinline__ uint64_t lazy_high(uint64_t T, const Mod& m) {
 }
 
 // Residue (times 2^-32) in (0, 4p) of coefficient `pos` of a polynomial stored as
-// [N][l64] limbs. `crt` (shared memory) holds 2^(32 j) mod p for j < 2*l64 <= L32MAX.
+// [N][l64] limbs. `crt` holds 2^(32 j) mod p for j < 2*l64 <= L32MAX.
 // With CENTER, values above (q-1)/2 stand for x - q.
 template <bool CENTER>
 __device__ __forceinline__ uint32_t crt_coef(const uint64_t* __restrict__ src, int pos, int l64,
@@ -221,25 +230,19 @@ constexpr int ks_min_blocks() {
 // fit in shared memory.
 template <int LOGN, int LOGE, int L64, bool CENTER, int MINB = 0, bool SINGLE = false>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul_min_blocks<LOGN, LOGE>()))
-    k_mul(const BasisDev* __restrict__ B, const uint64_t* __restrict__ A, long long a_stride,
+    k_mul(const __grid_constant__ ProdParams M, const uint64_t* __restrict__ A, long long a_stride,
           const uint64_t* __restrict__ Bv, long long b_stride, uint32_t* __restrict__ resid) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
     extern __shared__ uint32_t smem[];  // exchange regions, 2 operands x SMW each
-    __shared__ uint32_t s_crt[L32MAX];
-    __shared__ uint32_t s_qhalf[L32MAX];
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
-    const int k = B->k, l64 = B->l64;
-    for (int i = tau; i < L32MAX; i += PL::G) {  // blocks of small N have fewer than L32MAX threads
-        s_crt[i] = B->crt[prime][i];
-        s_qhalf[i] = B->qhalf[i];
-    }
-    const PrimeCtx c = load_prime_ctx(B, prime);
-    const uint2* __restrict__ psi = B->psi[prime];
-    const uint2* __restrict__ ipsi = B->ipsi[prime];
-    __syncthreads();
+    const int k = M.k;
+    const PrimeParam& Q = M.pr[prime];
+    const PrimeCtx c = load_prime_ctx(Q);
+    const uint2* __restrict__ psi = table_of(M.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
 
     const uint64_t* a = A + (size_t)job * a_stride;
     const uint64_t* b = Bv + (size_t)job * b_stride;
@@ -249,8 +252,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
         uint32_t cc[W], qh[W];
 #pragma unroll
         for (int j = 0; j < W; j++) {
-            cc[j] = s_crt[j];
-            qh[j] = s_qhalf[j];
+            cc[j] = Q.crt[j];
+            qh[j] = M.qhalf[j];
         }
 #pragma unroll
         for (int e = 0; e < E; e++) {
@@ -265,8 +268,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int pos = slot_pos<PL, 0>(tau, e);
-            x[0][e] = crt_coef<CENTER>(a, pos, l64, s_crt, s_qhalf, c);
-            x[1][e] = crt_coef<CENTER>(b, pos, l64, s_crt, s_qhalf, c);
+            x[0][e] = crt_coef<CENTER>(a, pos, M.l64, Q.crt, M.qhalf, c);
+            x[1][e] = crt_coef<CENTER>(b, pos, M.l64, Q.crt, M.qhalf, c);
         }
     }
     constexpr int STRIDE = SINGLE ? 0 : region_stride<PL, 2>();
@@ -274,13 +277,13 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
     // the pass code (the unrolled three transforms overflow the instruction cache)
     constexpr bool LOOP64 = LOGN == 12 && LOGE == 6;
     int buf = 0;
-    if constexpr (LOOP64) ntt64_forward<PL, 2>(x, psi, B->psi_r[prime], c.m, tau, smem);
-    else buf = ntt_forward<PL, 2>(x, psi, c.m, tau, smem, STRIDE, 0, CtaSync(), 1, B->psi_r[prime]);
+    if constexpr (LOOP64) ntt64_forward<PL, 2>(x, psi, rows_of(M.psi_r, prime), c.m, tau, smem);
+    else buf = ntt_forward<PL, 2>(x, psi, c.m, tau, smem, STRIDE, 0, CtaSync(), 1, rows_of(M.psi_r, prime));
     uint32_t z[1][E];
 #pragma unroll
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
-    if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, B->ipsi_r[prime], c.m, tau, smem + STRIDE, STRIDE == 0, nullptr);
-    else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, STRIDE, buf, CtaSync(), 1, B->ipsi_r[prime]);
+    if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, rows_of(M.ipsi_r, prime), c.m, tau, smem + STRIDE, STRIDE == 0, nullptr);
+    else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, STRIDE, buf, CtaSync(), 1, rows_of(M.ipsi_r, prime));
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = z[0][e];
@@ -336,7 +339,7 @@ __host__ __device__ constexpr bool ks_one_pass() {
 // that more blocks fit in shared memory.
 template <int LOGN, int LOGE, int L64, int ND, int MINB = 0, bool SINGLE = false>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_min_blocks<LOGN, LOGE>()))
-    k_keyswitch(const BasisDev* __restrict__ B, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
+    k_keyswitch(const __grid_constant__ ProdParams M, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
                 int ell, uint32_t* __restrict__ resid, int cs, int ls) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
@@ -347,11 +350,12 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
-    const int k = B->k, l64 = L64 > 0 ? L64 : B->l64;
-    const Mod m = load_mod(B, prime);
-    const uint32_t p = m.p, pinv = B->pinv[prime];
-    const uint2* __restrict__ psi = B->psi[prime];
-    const uint2* __restrict__ ipsi = B->ipsi[prime];
+    const PrimeParam& Q = M.pr[prime];
+    const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
+    const Mod m = load_mod(Q);
+    const uint32_t p = m.p, pinv = Q.pinv;
+    const uint2* __restrict__ psi = table_of(M.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
     const uint64_t* cj = C + (size_t)job * PL::N * l64;
     // limb w of coefficient pos at cj[pos * cs + w * ls]: (cs, ls) = (limbs, 1) for
     // [N][limb], (1, N) for limb-major (the HE multiply's intermediate: a warp's
@@ -397,7 +401,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
                     }
                 }
 #pragma unroll
-                for (int o = 0; o < ND; o++) x[o][e] = red(w[o], 2 * p);  // digit < 2^32 < 6p -> [0, 4p)
+                for (int o = 0; o < ND; o++) x[o][e] = red_2p(w[o], m);  // digit < 2^32 < 6p -> [0, 4p)
             } else {
 #pragma unroll
                 for (int o = 0; o < ND; o++) {
@@ -407,15 +411,15 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
                         const uint64_t limb = __ldg(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
                         w = (uint32_t)(limb >> (32 * (d & 1)));
                     }
-                    x[o][e] = red(w, 2 * p);  // digit < 2^32 < 6p -> [0, 4p)
+                    x[o][e] = red_2p(w, m);  // digit < 2^32 < 6p -> [0, 4p)
                 }
             }
         }
         if constexpr (LOGN == 12 && LOGE == 6) {  // one copy of the pass code (see k_mul)
-            ntt64_forward<PL, ND>(x, psi, B->psi_r[prime], m, tau, smem, true);
+            ntt64_forward<PL, ND>(x, psi, rows_of(M.psi_r, prime), m, tau, smem, true);
             buf++;
         } else {
-            buf = ntt_forward<PL, ND>(x, psi, m, tau, smem, STRIDE, buf, CtaSync(), 1, B->psi_r[prime]);
+            buf = ntt_forward<PL, ND>(x, psi, m, tau, smem, STRIDE, buf, CtaSync(), 1, rows_of(M.psi_r, prime));
         }
         if constexpr (rows_pass<PL, LAST>()) {
             // the key's copy laid out by lane (after the [ell][k][N] table): values u .. u+3
@@ -462,8 +466,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
 #pragma unroll
         for (int e = 0; e < E; e++) acc[0][e] = mac_finish<!(ONE && ND <= 2)>(T[e], pinv, m);
     }
-    if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, B->ipsi_r[prime], m, tau, smem, true, nullptr);
-    else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), 1, B->ipsi_r[prime]);
+    if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, rows_of(M.ipsi_r, prime), m, tau, smem, true, nullptr);
+    else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), 1, rows_of(M.ipsi_r, prime));
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = acc[0][e];
@@ -478,7 +482,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
 // --------------------------------------------------------------------------
 template <int LOGN, int LOGE, bool INV>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
-    k_ntt(const BasisDev* __restrict__ B, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
+    k_ntt(const __grid_constant__ ProdParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
           int njobs) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
@@ -488,8 +492,9 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
     const int prime = blockIdx.x;
     const int job0 = 2 * blockIdx.y;
     const bool two = job0 + 1 < njobs;
-    const int k = B->k;
-    const Mod m = load_mod(B, prime);
+    const int k = M.k;
+    const PrimeParam& Q = M.pr[prime];
+    const Mod m = load_mod(Q);
     const uint32_t p = m.p;
     uint32_t* v[2] = {res + ((size_t)job0 * k + prime) * PL::N, res + ((size_t)(two ? job0 + 1 : job0) * k + prime) * PL::N};
     uint32_t x[2][E];
@@ -501,7 +506,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
         for (int o = 0; o < 2; o++)
 #pragma unroll
             for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, 0>(tau, e)];
-        ntt_forward<PL, 2>(x, B->psi[prime], m, tau, smem, STRIDE, 0);
+        ntt_forward<PL, 2>(x, table_of(M.psi, prime), m, tau, smem, STRIDE, 0);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
             if (o == 1 && !two) break;
@@ -535,7 +540,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
                 for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, LAST>(tau, e)];
             }
         }
-        ntt_inverse<PL, 2>(x, B->ipsi[prime], m, tau, smem, STRIDE, 0);
+        ntt_inverse<PL, 2>(x, table_of(M.ipsi, prime), m, tau, smem, STRIDE, 0);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
             if (o == 1 && !two) break;
@@ -565,7 +570,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
 // code (ntt_core.cuh, ntt64_forward / ntt64_inverse).
 template <int LOGN, int LOGE, bool INV, int MINB = 0, bool COAL = false, int TPB = 1, bool LOOP = false>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB : 1))
-    k_ntt1(const BasisDev* __restrict__ B, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
+    k_ntt1(const __grid_constant__ ProdParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
            int njobs) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
@@ -579,8 +584,9 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
     const bool store = job_raw < njobs;
     const int job = store ? job_raw : njobs - 1;
     const int prime = blockIdx.y;
-    const int k = B->k;
-    const Mod m = load_mod(B, prime);
+    const int k = M.k;
+    const PrimeParam& Q = M.pr[prime];
+    const Mod m = load_mod(Q);
     const uint32_t p = m.p;
     uint32_t* v = res + ((size_t)job * k + prime) * PL::N;
     uint32_t x[1][E];
@@ -592,8 +598,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
     if (!INV) {
 #pragma unroll
         for (int e = 0; e < E; e++) x[0][e] = COAL ? __ldcs(v + slot_pos<PL, 0>(tau, e)) : v[slot_pos<PL, 0>(tau, e)];
-        if constexpr (LOOP) ntt64_forward<PL, 1>(x, B->psi[prime], B->psi_r[prime], m, tau, smem);
-        else ntt_forward<PL, 1>(x, B->psi[prime], m, tau, smem, STRIDE, 0, CtaSync(), 1, B->psi_r[prime]);
+        if constexpr (LOOP) ntt64_forward<PL, 1>(x, table_of(M.psi, prime), rows_of(M.psi_r, prime), m, tau, smem);
+        else ntt_forward<PL, 1>(x, table_of(M.psi, prime), m, tau, smem, STRIDE, 0, CtaSync(), 1, rows_of(M.psi_r, prime));
         if constexpr (COAL) {
             // row tau (positions 64 tau + u) into the padded region (word 65 tau + u),
             // then column tau (positions tau + 64 m, word 65 m + tau) to global memory
@@ -644,9 +650,9 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
         }
         // N^-1 is applied inside the last stage (outputs in [0, p))
         if constexpr (LOOP)
-            ntt64_inverse<PL, 1>(x, B->ipsi[prime], B->ipsi_r[prime], m, tau, smem, stride == 0, ninv + 4 * prime);
+            ntt64_inverse<PL, 1>(x, table_of(M.ipsi, prime), rows_of(M.ipsi_r, prime), m, tau, smem, stride == 0, ninv + 4 * prime);
         else
-            ntt_inverse<PL, 1>(x, B->ipsi[prime], m, tau, smem, stride, 0, CtaSync(), 1, B->ipsi_r[prime],
+            ntt_inverse<PL, 1>(x, table_of(M.ipsi, prime), m, tau, smem, stride, 0, CtaSync(), 1, rows_of(M.ipsi_r, prime),
                                ninv + 4 * prime);
         if (store) {
 #pragma unroll

@@ -70,27 +70,22 @@ __device__ __forceinline__ void pair_finish(uint32_t (&x)[1][PairPlan::E], uint3
 // k_mul for N = 16384 on a block pair (see k_mul for the arguments).
 template <int L64, bool CENTER>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
-    k_mul_pair(const BasisDev* __restrict__ B, const uint64_t* __restrict__ A, long long a_stride,
+    k_mul_pair(const __grid_constant__ ProdParams M, const uint64_t* __restrict__ A, long long a_stride,
                const uint64_t* __restrict__ Bv, long long b_stride, uint32_t* __restrict__ resid) {
     using PL = PairPlan;
     constexpr int E = PL::E;
     extern __shared__ uint32_t smem[];
-    __shared__ uint32_t s_crt[L32MAX];
-    __shared__ uint32_t s_qhalf[L32MAX];
     const int tau = threadIdx.x;
     const uint32_t h = cluster_rank();
     const int prime = blockIdx.y;
     const int job = blockIdx.x >> 1;
-    const int k = B->k, l64 = B->l64;
-    for (int i = tau; i < L32MAX; i += PL::G) {
-        s_crt[i] = B->crt[prime][i];
-        s_qhalf[i] = B->qhalf[i];
-    }
-    const PrimeCtx c = load_prime_ctx(B, prime);
-    const uint2* __restrict__ psi = B->psi[prime];
-    const uint2* __restrict__ ipsi = B->ipsi[prime];
+    const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
+    const PrimeParam& Q = M.pr[prime];
+    const PrimeCtx c = load_prime_ctx(Q);
+    const uint2* __restrict__ psi = table_of(M.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
     uint32_t* recv = smem + region_bytes<PL, 2>() / 4;
-    cluster_barrier();  // both blocks have started before any remote store; s_crt is ready
+    cluster_barrier();  // both blocks have started before any remote store
 
     // CRT split of this block's half of a and b only; the peer's half arrives in
     // the first words of this block's exchange region (unused until the first
@@ -106,8 +101,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
             uint32_t cc[W], qh[W];
 #pragma unroll
             for (int j = 0; j < W; j++) {
-                cc[j] = s_crt[j];
-                qh[j] = s_qhalf[j];
+                cc[j] = Q.crt[j];
+                qh[j] = M.qhalf[j];
             }
             uint32_t w[W];
             load_words<L64>(a + (size_t)pos * L64, w);
@@ -115,8 +110,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
             load_words<L64>(b + (size_t)pos * L64, w);
             x[1][e] = crt_words<W, CENTER>(w, cc, qh, c);
         } else {
-            x[0][e] = crt_coef<CENTER>(a, pos, l64, s_crt, s_qhalf, c);
-            x[1][e] = crt_coef<CENTER>(b, pos, l64, s_crt, s_qhalf, c);
+            x[0][e] = crt_coef<CENTER>(a, pos, l64, Q.crt, M.qhalf, c);
+            x[1][e] = crt_coef<CENTER>(b, pos, l64, Q.crt, M.qhalf, c);
         }
 #pragma unroll
         for (int o = 0; o < 2; o++) store_peer(&smem[o * kPairHalf + pos], h ^ 1u, x[o][e]);
@@ -148,7 +143,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
 // k_keyswitch for N = 16384 on a block pair, ND digits per pass (see k_keyswitch).
 template <int L64, int ND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
-    k_keyswitch_pair(const BasisDev* __restrict__ B, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
+    k_keyswitch_pair(const __grid_constant__ ProdParams M, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
                      int ell, uint32_t* __restrict__ resid, int cs, int ls) {
     using PL = PairPlan;
     constexpr int E = PL::E;
@@ -157,11 +152,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const uint32_t h = cluster_rank();
     const int prime = blockIdx.y;
     const int job = blockIdx.x >> 1;
-    const int k = B->k, l64 = L64 > 0 ? L64 : B->l64;
-    const Mod m = load_mod(B, prime);
+    const PrimeParam& Q = M.pr[prime];
+    const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
+    const Mod m = load_mod(Q);
     const uint32_t p = m.p;
-    const uint2* __restrict__ psi = B->psi[prime];
-    const uint2* __restrict__ ipsi = B->ipsi[prime];
+    const uint2* __restrict__ psi = table_of(M.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
     const uint64_t* cj = C + (size_t)job * (2 * kPairHalf) * l64;
     // limb w of coefficient pos at cj[pos * cs + w * ls]: (limbs, 1) for [N][limb],
     // (1, N) for limb-major
@@ -191,8 +187,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
                     wl = (uint32_t)(ll >> (32 * (d & 1)));
                     wh = (uint32_t)(lh >> (32 * (d & 1)));
                 }
-                lo[o] = red(wl, 2 * p);  // digit < 2^32 < 6p -> [0, 4p)
-                hi[o] = red(wh, 2 * p);
+                lo[o] = red_2p(wl, m);  // digit < 2^32 < 6p -> [0, 4p)
+                hi[o] = red_2p(wh, m);
                 ct_bfly(lo[o], hi[o], w0.x, w0.y, m);  // first stage of the whole transform
                 x[o][e] = h ? hi[o] : lo[o];
             }
@@ -214,7 +210,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
         }
     }
     uint32_t acc[1][E];
-    const uint32_t pinv = B->pinv[prime];
+    const uint32_t pinv = Q.pinv;
 #pragma unroll
     for (int e = 0; e < E; e++) acc[0][e] = mac_finish<true>(T[e], pinv, m);
     ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), tm);

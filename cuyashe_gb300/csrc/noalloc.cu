@@ -94,7 +94,7 @@ extern "C" cy_status cy_polymul_noalloc(cy_ring* r, const uint64_t* d_a, const u
     const KernelSet& ks = kernel_set(B.h.logn);
     const BasisDev* Bd = B.d;
     long long stride = (long long)n * r->l64;
-    void* args[] = {(void*)&Bd, (void*)&d_a, (void*)&stride, (void*)&d_b, (void*)&stride, (void*)&scratch};
+    void* args[] = {(void*)&B.prod, (void*)&d_a, (void*)&stride, (void*)&d_b, (void*)&stride, (void*)&scratch};
     // blocks_per_prime > 1 for schedules that run one product on a pair of blocks
     CY_TRY(launch_noalloc(ks.mul_for(B.h.l64, false), "mul_noalloc", B.h.logn, dim3(batch * ks.blocks_per_prime, k),
                           dim3(ks.threads), ks.smem_mul, st, args));

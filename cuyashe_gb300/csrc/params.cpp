@@ -10,6 +10,8 @@
 #include <map>
 #include <mutex>
 
+#include <algorithm>
+
 #include "host.h"
 
 namespace cy {
@@ -289,6 +291,23 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
         ninv[4 * i + 2] = vw;
         ninv[4 * i + 3] = shoup_of(vw, p);
     }
+    for (int i = 0; i < b.h.k; i++) {
+        PrimeParam& q = b.prod.pr[i];
+        q.p = b.h.p[i];
+        q.p2 = b.h.p2[i];
+        q.np = b.h.np[i];
+        q.np2 = b.h.np2[i];
+        q.pinv = b.h.pinv[i];
+        q.cadd = b.h.p2[i] - b.h.qmont[i];
+        std::copy(b.h.crt[i], b.h.crt[i] + L32MAX, q.crt);
+    }
+    std::copy(b.h.qhalf, b.h.qhalf + L32MAX, b.prod.qhalf);
+    b.prod.k = b.h.k;
+    b.prod.l64 = b.h.l64;
+    b.prod.psi = b.h.psi[0];
+    b.prod.ipsi = b.h.ipsi[0];
+    b.prod.psi_r = b.h.psi_r[0];
+    b.prod.ipsi_r = b.h.ipsi_r[0];
     b.epi = epi_const(b.h.l32, b.h.k, b.h.mode);
     if (!b.epi) return set_error(CY_ERR_INTERNAL, "missing epilogue");
     b.epi_param.assign(b.epi->param_bytes, 0);
