@@ -47,8 +47,4 @@ struct EpiConstKernel {
 };
 const EpiConstKernel* epi_const(int l32, int k, int mode);
 
-// Bytes of shared memory an exchange region set needs, and whether the kernel
-// alternates two regions (one barrier per exchange) or reuses one (two).
-constexpr size_t kSmemDoubleLimit = 200 * 1024;
-
 }  // namespace cy

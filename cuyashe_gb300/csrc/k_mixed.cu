@@ -38,9 +38,7 @@ __device__ __forceinline__ void mixed_ntt_unit(const MixedJob& J, const MixedUni
                                                uint32_t* __restrict__ done) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E, G = PL::G;
-    // two exchange regions of two operands per sub-group (the same size at every N)
-    constexpr int SUBW = 4 * PL::SMW;
-    constexpr int STRIDE = 2 * PL::SMW;
+    constexpr int SUBW = 2 * PL::SMW;  // exchange buffer of two operands per sub-group
     const int sub = threadIdx.x / G, tau = threadIdx.x % G;
     if (sub >= U.count) return;  // fewer primes than sub-groups in this unit
     const int prime = U.first + sub;
@@ -68,11 +66,11 @@ __device__ __forceinline__ void mixed_ntt_unit(const MixedJob& J, const MixedUni
         x[0][e] = crt_words<W, CENTER>(wa, cc, qh, c);
         x[1][e] = crt_words<W, CENTER>(wb, cc, qh, c);
     }
-    int buf = ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, STRIDE, 0, bar);
+    ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, false, bar);
     uint32_t z[1][E];
 #pragma unroll
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
-    ntt_inverse<PL, 1, GroupSync>(z, B->ipsi[prime], m, tau, sm, STRIDE, buf, bar);
+    ntt_inverse<PL, 1, GroupSync>(z, B->ipsi[prime], m, tau, sm, bar);
     uint32_t* out = J.resid + (size_t)prime * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = z[0][e];
@@ -89,8 +87,7 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
                                               uint32_t* __restrict__ done) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E, G = PL::G;
-    constexpr int SUBW = 4 * PL::SMW;
-    constexpr int STRIDE = 2 * PL::SMW;
+    constexpr int SUBW = 2 * PL::SMW;
     const int sub = threadIdx.x / G, tau = threadIdx.x % G;
     if (sub >= U.count) return;
     const int prime = U.first + sub;
@@ -102,7 +99,6 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
     uint64_t T[E];  // sums of products with the key (see k_keyswitch)
 #pragma unroll
     for (int e = 0; e < E; e++) T[e] = 0;
-    int buf = 0;
     for (int d0 = 0; d0 < ell; d0 += 2) {
         uint32_t x[2][E];
 #pragma unroll
@@ -120,7 +116,7 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
                 x[o][e] = __viaddmin_u32(w, m.np2, w);  // digit < 2^32 < 6p -> [0, 4p)
             }
         }
-        buf = ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, STRIDE, buf, bar);
+        ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, d0 > 0, bar);
 #pragma unroll
         for (int e = 0; e < E; e++) T[e] = lazy_high(T[e], m);
 #pragma unroll
@@ -138,7 +134,7 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
     const uint32_t pinv = B->pinv[prime];
 #pragma unroll
     for (int e = 0; e < E; e++) acc[0][e] = mac_finish<true>(T[e], pinv, m);
-    ntt_inverse<PL, 1, GroupSync>(acc, B->ipsi[prime], m, tau, sm, STRIDE, buf, bar);
+    ntt_inverse<PL, 1, GroupSync>(acc, B->ipsi[prime], m, tau, sm, bar);
     uint32_t* out = J.resid + (size_t)prime * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = acc[0][e];
@@ -271,15 +267,15 @@ __global__ void __launch_bounds__(MixedSched<LOGE>::THREADS, MixedSched<LOGE>::M
 }
 
 // Dynamic shared memory: the same at every N for one schedule
-// ((threads / (N/E)) sub-groups x 4 operand buffers of N + N/E words).
+// ((threads / (N/E)) sub-groups x 2 operand buffers of N words).
 template <int LOGE>
 constexpr size_t mixed_smem() {
-    return (size_t)(MixedSched<LOGE>::THREADS / NttPlan<13, LOGE>::G) * 4 * NttPlan<13, LOGE>::SMW * sizeof(uint32_t);
+    return (size_t)(MixedSched<LOGE>::THREADS / NttPlan<13, LOGE>::G) * 2 * NttPlan<13, LOGE>::SMW * sizeof(uint32_t);
 }
-static_assert(mixed_smem<3>() == (size_t)2 * 4 * NttPlan<12, 3>::SMW * 4 &&
-                  mixed_smem<3>() == (size_t)8 * 4 * NttPlan<10, 3>::SMW * 4 &&
-                  mixed_smem<4>() == (size_t)2 * 4 * NttPlan<12, 4>::SMW * 4 &&
-                  mixed_smem<4>() == (size_t)8 * 4 * NttPlan<10, 4>::SMW * 4,
+static_assert(mixed_smem<3>() == (size_t)2 * 2 * NttPlan<12, 3>::SMW * 4 &&
+                  mixed_smem<3>() == (size_t)8 * 2 * NttPlan<10, 3>::SMW * 4 &&
+                  mixed_smem<4>() == (size_t)2 * 2 * NttPlan<12, 4>::SMW * 4 &&
+                  mixed_smem<4>() == (size_t)8 * 2 * NttPlan<10, 4>::SMW * 4,
               "one shared-memory size serves every transform length");
 
 // schedule 0: 8 coefficients per thread, 1024 threads; 1: 16 per thread, 512 threads

@@ -1,8 +1,5 @@
-// Kernel instantiations for N = 4096 with 2^4 coefficients per thread and two
-// exchange regions, compiled for the three product blocks per SM that their 69.6 KB
-// of shared memory allows (85 registers per thread instead of 64). The
-// keyswitch, whose two four-operand regions admit one block per SM, gets the
-// whole register file.
+// Kernel instantiations for N = 4096 with 2^4 coefficients per thread: three product
+// blocks per SM (80 registers), the keyswitch with the whole register file.
 #include "kernels.cuh"
 
 namespace cy {

@@ -4,5 +4,5 @@
 #include "kernels.cuh"
 
 namespace cy {
-void fill_n14_e4d1(KernelSet& ks) { fill_kernel_set<14, 4, true, 0, 0, false, false, 1>(ks); }
+void fill_n14_e4d1(KernelSet& ks) { fill_kernel_set<14, 4, true, 0, 0, 1>(ks); }
 }  // namespace cy

@@ -25,15 +25,10 @@
 
 namespace cy {
 
-// Exchange-region stride (words) for a kernel whose widest exchange carries
-// NOPS operands: two alternating regions when they fit, else one (stride 0).
-template <class PL, int NOPS>
-__host__ __device__ constexpr int region_stride() {
-    return (size_t)2 * NOPS * PL::SMW * 4 <= kSmemDoubleLimit ? NOPS * PL::SMW : 0;
-}
+// Bytes of the exchange buffer of NOPS operands.
 template <class PL, int NOPS>
 __host__ __device__ constexpr size_t region_bytes() {
-    return (size_t)(region_stride<PL, NOPS>() ? 2 : 1) * NOPS * PL::SMW * 4;
+    return (size_t)NOPS * PL::SMW * 4;
 }
 
 // The modulus of prime i with its derived constants, each read on its own.
@@ -226,15 +221,13 @@ constexpr int ks_min_blocks() {
 
 // MINB > 0 overrides the blocks per SM the kernel is compiled for (a schedule
 // with a larger register budget per thread).
-// SINGLE: one exchange region (two barriers per exchange), so that more blocks
-// fit in shared memory.
-template <int LOGN, int LOGE, int L64, bool CENTER, int MINB = 0, bool SINGLE = false>
+template <int LOGN, int LOGE, int L64, bool CENTER, int MINB = 0>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul_min_blocks<LOGN, LOGE>()))
     k_mul(const __grid_constant__ ProdParams M, const uint64_t* __restrict__ A, long long a_stride,
           const uint64_t* __restrict__ Bv, long long b_stride, uint32_t* __restrict__ resid) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
-    extern __shared__ uint32_t smem[];  // exchange regions, 2 operands x SMW each
+    extern __shared__ uint32_t smem[];  // exchange buffer, 2 operands x SMW
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
@@ -272,18 +265,16 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
             x[1][e] = crt_coef<CENTER>(b, pos, M.l64, Q.crt, M.qhalf, c);
         }
     }
-    constexpr int STRIDE = SINGLE ? 0 : region_stride<PL, 2>();
     // 64 coefficients per thread at N = 4096: both transforms loop over one copy of
     // the pass code (the unrolled three transforms overflow the instruction cache)
     constexpr bool LOOP64 = LOGN == 12 && LOGE == 6;
-    int buf = 0;
     if constexpr (LOOP64) ntt64_forward<PL, 2>(x, psi, rows_of(M.psi_r, prime), c.m, tau, smem);
-    else buf = ntt_forward<PL, 2>(x, psi, c.m, tau, smem, STRIDE, 0, CtaSync(), 1, rows_of(M.psi_r, prime));
+    else ntt_forward<PL, 2>(x, psi, c.m, tau, smem, false, CtaSync(), 1, rows_of(M.psi_r, prime));
     uint32_t z[1][E];
 #pragma unroll
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
-    if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, rows_of(M.ipsi_r, prime), c.m, tau, smem + STRIDE, STRIDE == 0, nullptr);
-    else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, STRIDE, buf, CtaSync(), 1, rows_of(M.ipsi_r, prime));
+    if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, rows_of(M.ipsi_r, prime), c.m, tau, smem, nullptr);
+    else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime));
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = z[0][e];
@@ -335,9 +326,7 @@ __host__ __device__ constexpr bool ks_one_pass() {
     return (L64 == 1 && ND >= 2) || (L64 == 2 && ND >= 4);
 }
 
-// SINGLE: one exchange region (two barriers per exchange) instead of two, so
-// that more blocks fit in shared memory.
-template <int LOGN, int LOGE, int L64, int ND, int MINB = 0, bool SINGLE = false>
+template <int LOGN, int LOGE, int L64, int ND, int MINB = 0>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_min_blocks<LOGN, LOGE>()))
     k_keyswitch(const __grid_constant__ ProdParams M, const uint64_t* __restrict__ C, const uint32_t* __restrict__ evk,
                 int ell, uint32_t* __restrict__ resid, int cs, int ls) {
@@ -346,7 +335,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     constexpr int LAST = PL::NPASS - 1;
     constexpr bool ONE = ks_one_pass<L64, ND>();
     constexpr bool ACC32 = !ONE && LOGE > 4;
-    extern __shared__ uint32_t smem[];  // exchange regions, ND operands x SMW each
+    extern __shared__ uint32_t smem[];  // exchange buffer, ND operands x SMW
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
@@ -361,7 +350,6 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     // [N][limb], (1, N) for limb-major (the HE multiply's intermediate: a warp's
     // loads of one limb are then contiguous). Kernel parameters, so that they stay
     // in the constant bank.
-    constexpr int STRIDE = SINGLE ? 0 : region_stride<PL, ND>();
 
     uint64_t T[E];           // sums of products
     uint32_t acc[1][E];      // reduced sums: the inverse transform's input
@@ -370,7 +358,6 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
         T[e] = 0;
         acc[0][e] = 0;
     }
-    int buf = 0;
     for (int d0 = 0; d0 < (ONE ? 1 : ell); d0 += ND) {
         uint32_t x[ND][E];
 #pragma unroll
@@ -416,10 +403,9 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
             }
         }
         if constexpr (LOGN == 12 && LOGE == 6) {  // one copy of the pass code (see k_mul)
-            ntt64_forward<PL, ND>(x, psi, rows_of(M.psi_r, prime), m, tau, smem, true);
-            buf++;
+            ntt64_forward<PL, ND>(x, psi, rows_of(M.psi_r, prime), m, tau, smem, d0 > 0);
         } else {
-            buf = ntt_forward<PL, ND>(x, psi, m, tau, smem, STRIDE, buf, CtaSync(), 1, rows_of(M.psi_r, prime));
+            ntt_forward<PL, ND>(x, psi, m, tau, smem, d0 > 0, CtaSync(), 1, rows_of(M.psi_r, prime));
         }
         if constexpr (rows_pass<PL, LAST>()) {
             // the key's copy laid out by lane (after the [ell][k][N] table): values u .. u+3
@@ -466,8 +452,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
 #pragma unroll
         for (int e = 0; e < E; e++) acc[0][e] = mac_finish<!(ONE && ND <= 2)>(T[e], pinv, m);
     }
-    if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, rows_of(M.ipsi_r, prime), m, tau, smem, true, nullptr);
-    else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), 1, rows_of(M.ipsi_r, prime));
+    if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, rows_of(M.ipsi_r, prime), m, tau, smem, nullptr);
+    else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime));
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = acc[0][e];
@@ -498,7 +484,6 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
     const uint32_t p = m.p;
     uint32_t* v[2] = {res + ((size_t)job0 * k + prime) * PL::N, res + ((size_t)(two ? job0 + 1 : job0) * k + prime) * PL::N};
     uint32_t x[2][E];
-    constexpr int STRIDE = region_stride<PL, 2>();
     // after the last pass a thread's E positions are contiguous (16-byte accesses)
     constexpr bool VEC = PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE && E % 4 == 0;
     if (!INV) {
@@ -506,7 +491,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
         for (int o = 0; o < 2; o++)
 #pragma unroll
             for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, 0>(tau, e)];
-        ntt_forward<PL, 2>(x, table_of(M.psi, prime), m, tau, smem, STRIDE, 0);
+        ntt_forward<PL, 2>(x, table_of(M.psi, prime), m, tau, smem);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
             if (o == 1 && !two) break;
@@ -540,7 +525,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
                 for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, LAST>(tau, e)];
             }
         }
-        ntt_inverse<PL, 2>(x, table_of(M.ipsi, prime), m, tau, smem, STRIDE, 0);
+        ntt_inverse<PL, 2>(x, table_of(M.ipsi, prime), m, tau, smem);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
             if (o == 1 && !two) break;
@@ -590,20 +575,16 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
     const uint32_t p = m.p;
     uint32_t* v = res + ((size_t)job * k + prime) * PL::N;
     uint32_t x[1][E];
-    // one exchange (two passes) needs no barrier ahead of its writes: a second,
-    // never used region offset stands in for the alternation; more passes share
-    // one region with a barrier before each exchange
-    constexpr int STRIDE = PL::NPASS <= 2 ? PL::SMW : 0;
     constexpr bool VEC = PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE && E % 4 == 0;
     if (!INV) {
 #pragma unroll
         for (int e = 0; e < E; e++) x[0][e] = COAL ? __ldcs(v + slot_pos<PL, 0>(tau, e)) : v[slot_pos<PL, 0>(tau, e)];
         if constexpr (LOOP) ntt64_forward<PL, 1>(x, table_of(M.psi, prime), rows_of(M.psi_r, prime), m, tau, smem);
-        else ntt_forward<PL, 1>(x, table_of(M.psi, prime), m, tau, smem, STRIDE, 0, CtaSync(), 1, rows_of(M.psi_r, prime));
+        else ntt_forward<PL, 1>(x, table_of(M.psi, prime), m, tau, smem, false, CtaSync(), 1, rows_of(M.psi_r, prime));
         if constexpr (COAL) {
-            // row tau (positions 64 tau + u) into the padded region (word 65 tau + u),
-            // then column tau (positions tau + 64 m, word 65 m + tau) to global memory
-            __syncthreads();
+            // row tau (positions 64 tau + u) into the padded buffer (word 65 tau + u: the words
+            // this thread read last), then column tau (positions tau + 64 m, word 65 m + tau)
+            // to global memory
 #pragma unroll
             for (int u = 0; u < E; u++) smem[65 * tau + u] = red(red(x[0][u], 2 * p), p);
             __syncthreads();
@@ -624,16 +605,14 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
             for (int e = 0; e < E; e++) v[slot_pos<PL, LAST>(tau, e)] = red(red(x[0][e], 2 * p), p);
         }
     } else {
-        int stride = STRIDE;
         if constexpr (COAL) {
-            // columns in (coalesced), rows out of the padded region; the exchange
-            // of the inverse then reuses the region after a barrier (stride 0)
+            // columns in (coalesced), rows out of the padded buffer; the inverse's exchange then
+            // writes back the words each thread read
 #pragma unroll
             for (int m = 0; m < E; m++) smem[tau + 65 * m] = __ldcs(v + tau + 64 * m);
             __syncthreads();
 #pragma unroll
             for (int u = 0; u < E; u++) x[0][u] = smem[65 * tau + u];
-            stride = 0;
         } else if constexpr (VEC) {
             const uint4* s4 = reinterpret_cast<const uint4*>(v + group_base<PL, LAST>(tau, 0));
 #pragma unroll
@@ -650,9 +629,9 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
         }
         // N^-1 is applied inside the last stage (outputs in [0, p))
         if constexpr (LOOP)
-            ntt64_inverse<PL, 1>(x, table_of(M.ipsi, prime), rows_of(M.ipsi_r, prime), m, tau, smem, stride == 0, ninv + 4 * prime);
+            ntt64_inverse<PL, 1>(x, table_of(M.ipsi, prime), rows_of(M.ipsi_r, prime), m, tau, smem, ninv + 4 * prime);
         else
-            ntt_inverse<PL, 1>(x, table_of(M.ipsi, prime), m, tau, smem, stride, 0, CtaSync(), 1, rows_of(M.ipsi_r, prime),
+            ntt_inverse<PL, 1>(x, table_of(M.ipsi, prime), m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime),
                                ninv + 4 * prime);
         if (store) {
 #pragma unroll
@@ -1291,40 +1270,39 @@ void fill_epi_const(const BasisDev& h, void* param) {
 
 namespace cy {
 
-template <int LOGN, int LOGE, int L64, int MB_MUL, int MB_KS, bool SINGLE_KS, bool SINGLE_MUL, int ND_LO, int ND_HI>
+template <int LOGN, int LOGE, int L64, int MB_MUL, int MB_KS, int ND_LO, int ND_HI>
 void fill_l64(KernelSet& ks) {
-    ks.mul[L64][0] = (void*)k_mul<LOGN, LOGE, L64, false, MB_MUL, SINGLE_MUL>;
-    ks.mul[L64][1] = (void*)k_mul<LOGN, LOGE, L64, true, MB_MUL, SINGLE_MUL>;
-    ks.ks[L64][0] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_LO, MB_KS, SINGLE_KS>;
-    ks.ks[L64][1] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_HI, MB_KS, SINGLE_KS>;
+    ks.mul[L64][0] = (void*)k_mul<LOGN, LOGE, L64, false, MB_MUL>;
+    ks.mul[L64][1] = (void*)k_mul<LOGN, LOGE, L64, true, MB_MUL>;
+    ks.ks[L64][0] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_LO, MB_KS>;
+    ks.ks[L64][1] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_HI, MB_KS>;
 }
 
 // SPECIALISE: also instantiate the kernels for 1, 2, 3 and 6 limbs (q of up to
 // 64, 128, 192 and 384 bits); other limb counts use the generic kernels.
 // MB_MUL / MB_KS > 0: blocks per SM the product / keyswitch kernels are
 // compiled for (0: the defaults above).
-// SINGLE_KS / SINGLE_MUL: the keyswitch / product kernels use one exchange region.
 // ND_LO: digits per pass of the keyswitch kernel used when four do not fit (2, or 1
 // for fewer registers); ND_HI: digits per pass of the one used when the digit
 // count is a multiple of four and it fits (4, or 2 for fewer registers).
 // SPEC_MASK: the limb counts (bit L64) that get specialised kernels when
 // SPECIALISE is set.
-template <int LOGN, int LOGE, bool SPECIALISE, int MB_MUL = 0, int MB_KS = 0, bool SINGLE_KS = false,
-          bool SINGLE_MUL = false, int ND_LO = 2, int ND_HI = 4, unsigned SPEC_MASK = 0x4Eu>
+template <int LOGN, int LOGE, bool SPECIALISE, int MB_MUL = 0, int MB_KS = 0, int ND_LO = 2, int ND_HI = 4,
+          unsigned SPEC_MASK = 0x4Eu>
 void fill_kernel_set(KernelSet& ks) {
     using PL = NttPlan<LOGN, LOGE>;
     ks.logn = LOGN;
     ks.loge = LOGE;
     ks.threads = PL::G;
-    fill_l64<LOGN, LOGE, 0, MB_MUL, MB_KS, SINGLE_KS, SINGLE_MUL, ND_LO, ND_HI>(ks);
+    fill_l64<LOGN, LOGE, 0, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (SPECIALISE && (SPEC_MASK & 2u))
-        fill_l64<LOGN, LOGE, 1, MB_MUL, MB_KS, SINGLE_KS, SINGLE_MUL, ND_LO, ND_HI>(ks);
+        fill_l64<LOGN, LOGE, 1, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (SPECIALISE && (SPEC_MASK & 4u))
-        fill_l64<LOGN, LOGE, 2, MB_MUL, MB_KS, SINGLE_KS, SINGLE_MUL, ND_LO, ND_HI>(ks);
+        fill_l64<LOGN, LOGE, 2, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (SPECIALISE && (SPEC_MASK & 8u))
-        fill_l64<LOGN, LOGE, 3, MB_MUL, MB_KS, SINGLE_KS, SINGLE_MUL, ND_LO, ND_HI>(ks);
+        fill_l64<LOGN, LOGE, 3, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (SPECIALISE && (SPEC_MASK & 64u))
-        fill_l64<LOGN, LOGE, 6, MB_MUL, MB_KS, SINGLE_KS, SINGLE_MUL, ND_LO, ND_HI>(ks);
+        fill_l64<LOGN, LOGE, 6, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (LOGE >= 6) {  // one transform per block (k_ntt1), coalesced row side at N = 4096
         // N = 4096: coalesced row side, the two passes as a loop over one copy of the
         // pass code, 96 registers (10 blocks per SM), measured best in both directions
@@ -1336,10 +1314,10 @@ void fill_kernel_set(KernelSet& ks) {
         ks.ntt[0] = (void*)k_ntt<LOGN, LOGE, false>;
         ks.ntt[1] = (void*)k_ntt<LOGN, LOGE, true>;
     }
-    ks.smem_mul = SINGLE_MUL ? (size_t)2 * PL::SMW * 4 : region_bytes<PL, 2>();
-    ks.smem_ks[0] = SINGLE_KS ? (size_t)ND_LO * PL::SMW * 4 : region_bytes<PL, ND_LO>();
-    ks.smem_ks[1] = SINGLE_KS ? (size_t)ND_HI * PL::SMW * 4 : region_bytes<PL, ND_HI>();
-    ks.smem_ntt = LOGE >= 6 ? (size_t)PL::SMW * 4 : region_bytes<PL, 2>();
+    ks.smem_mul = region_bytes<PL, 2>();
+    ks.smem_ks[0] = region_bytes<PL, ND_LO>();
+    ks.smem_ks[1] = region_bytes<PL, ND_HI>();
+    ks.smem_ntt = LOGE >= 6 ? region_bytes<PL, 1>() : region_bytes<PL, 2>();
 }
 
 }  // namespace cy

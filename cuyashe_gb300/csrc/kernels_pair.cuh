@@ -44,7 +44,7 @@ __device__ __forceinline__ void store_peer(const uint32_t* local, uint32_t peer,
 using PairPlan = NttPlan<13, 3>;  // one half of N = 16384, 8 coefficients per thread, 1024 threads
 constexpr int kPairHalf = PairPlan::N;
 
-// Exchange words (two regions when they fit) plus the half received from the peer.
+// Exchange buffer plus the half received from the peer.
 template <int NOPS>
 __host__ __device__ constexpr size_t pair_smem_bytes() {
     return region_bytes<PairPlan, NOPS>() + (size_t)kPairHalf * 4;
@@ -129,14 +129,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
             x[o][e] = h ? hi : lo;
         }
     }
-    __syncthreads();  // every thread has read region 0 before the first exchange writes it
-    constexpr int STRIDE = region_stride<PL, 2>();
+    __syncthreads();  // every thread has read the buffer before the first exchange writes it
     const int tm = 2 + (int)h;
-    int buf = ntt_forward<PL, 2>(x, psi, c.m, tau, smem, STRIDE, 0, CtaSync(), tm);
+    ntt_forward<PL, 2>(x, psi, c.m, tau, smem, false, CtaSync(), tm);
     uint32_t z[1][E];
 #pragma unroll
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
-    ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, STRIDE, buf, CtaSync(), tm);
+    ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, CtaSync(), tm);
     pair_finish(z, recv, h, tau, c.p, __ldg(ipsi + 1), resid + ((size_t)job * k + prime) * (2 * kPairHalf));
 }
 
@@ -162,7 +161,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     // limb w of coefficient pos at cj[pos * cs + w * ls]: (limbs, 1) for [N][limb],
     // (1, N) for limb-major
     uint32_t* recv = smem + region_bytes<PL, ND>() / 4;
-    constexpr int STRIDE = region_stride<PL, ND>();
     const int tm = 2 + (int)h;
     const uint2 w0 = __ldg(psi + 1);
     cluster_barrier();  // both blocks have started before any remote store
@@ -170,7 +168,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     uint64_t T[E];  // sums of products with the key (see k_keyswitch)
 #pragma unroll
     for (int e = 0; e < E; e++) T[e] = 0;
-    int buf = 0;
     for (int d0 = 0; d0 < ell; d0 += ND) {
         uint32_t x[ND][E];
 #pragma unroll
@@ -193,7 +190,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
                 x[o][e] = h ? hi[o] : lo[o];
             }
         }
-        buf = ntt_forward<PL, ND>(x, psi, m, tau, smem, STRIDE, buf, CtaSync(), tm);
+        ntt_forward<PL, ND>(x, psi, m, tau, smem, d0 > 0, CtaSync(), tm);
 #pragma unroll
         for (int o = 0; o < ND; o++) {
             const int d = d0 + o;
@@ -213,7 +210,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const uint32_t pinv = Q.pinv;
 #pragma unroll
     for (int e = 0; e < E; e++) acc[0][e] = mac_finish<true>(T[e], pinv, m);
-    ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, STRIDE, buf, CtaSync(), tm);
+    ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, CtaSync(), tm);
     pair_finish(acc, recv, h, tau, p, __ldg(ipsi + 1), resid + ((size_t)job * k + prime) * (2 * kPairHalf));
 }
 

@@ -6,8 +6,8 @@
 // block of G = N/E threads owns one length-N transform: every thread keeps E
 // coefficients in registers, the log2(N) stages are grouped into passes of at
 // most LOGE stages that run entirely in registers, and consecutive passes swap
-// data through a padded shared-memory buffer (one barrier per swap, two
-// alternating buffers). Several operands (NOPS) of the same prime share the
+// data through a shared-memory buffer, in place (one barrier per swap, between
+// the threads that share a sub-transform). Several operands (NOPS) of the same prime share the
 // twiddle loads and interleave for instruction-level parallelism.
 //
 // Transform (merged negacyclic twist): forward Cooley-Tukey on natural-order
@@ -39,7 +39,8 @@ struct NttPlan {
     static constexpr int G = N >> LOGE;  // threads per transform
     static constexpr int NPASS = (LOGN + LOGE - 1) / LOGE;
     static constexpr int R0 = LOGN - (NPASS - 1) * LOGE;  // the first pass takes the remainder
-    static constexpr int SMW = N + (N >> LOGE);            // words per operand buffer (with padding)
+    // words per operand buffer: N, and one more per 2^LOGE with 32 or 64 coefficients (XMap)
+    static constexpr int SMW = LOGE >= 5 ? N + (N >> LOGE) : N;
     __host__ __device__ static constexpr int R(int pass) { return pass == 0 ? R0 : LOGE; }
     __host__ __device__ static constexpr int S0(int pass) { return pass == 0 ? 0 : R0 + (pass - 1) * LOGE; }
     __host__ __device__ static constexpr int LOGD(int pass) { return LOGN - S0(pass) - R(pass); }
@@ -58,33 +59,31 @@ struct GroupSync {
     }
 };
 
-// Shared-memory layout of the exchange between two passes whose butterflies
-// span 2^DA and 2^DB positions (LOGD of the writing and the reading pass), for
-// E = 2^R coefficients per thread. For one register slot a warp touches 32
-// consecutive positions when LOGD >= 5, else 32/2^D runs of 2^D positions that
-// are 2^(D+R) apart. Banks are kept distinct on both sides by
-//   * P padding words after every 32 (an address stays base + constant): P = 1
-//     when the strided side has LOGD = 0, P = 2^(5-R) when it has LOGD = R;
-//   * an XOR of the low 5 bits with bits of the row (pos >> 5) when both sides
-//     are strided (LOGD = R and 0), which permutes words inside each 32-word row.
-// Every layout is a bijection into SMW = N + N/2^R words.
-// With R = 6 (64 coefficients per thread) one word is added after every 64:
-// the side with LOGD = 0 then reads 64 consecutive positions per thread at a
-// stride of 65 words between lanes (all banks distinct), and the side whose
-// lanes hold consecutive positions stays conflict free.
-template <int R, int DA, int DB>
-struct XLayout {
-    static constexpr int DMIN = DA < DB ? DA : DB;
-    static constexpr int DMAX = DA < DB ? DB : DA;
-    static constexpr bool SWZ = DMAX < 5 && (R == 3 || R == 4);
-    static constexpr int PAD = (DMIN >= 5 || DMIN == 0 || DMIN != R || R >= 5) ? 1 : (1 << (5 - R));
-    static constexpr int PSH = R >= 6 ? 6 : 5;  // padding period 2^PSH words
-    // the padded word of a position whose bits below PSH and above are independent
-    __host__ __device__ static constexpr int pad(int pos) { return pos + PAD * (pos >> PSH); }
-    __device__ __forceinline__ static int swz(int pos) {
+// Shared-memory layout of the exchanges of a plan with E = 2^R coefficients per
+// thread. For one register slot of a pass whose butterflies span 2^D positions
+// (D = LOGD) a warp touches 32 consecutive positions when D >= 5, else 32/2^D runs of
+// 2^D positions 2^(D+R) apart; D is 0, R, 2R, .. . One layout for all of them, free of bank
+// conflicts, so that every exchange of a plan is in place:
+//   * R = 3, 4: an XOR of the low 5 bits with bits of the row (pos >> 5), which permutes
+//     words inside each 32-word row. It is linear over XOR, so the address of slot u of a
+//     group is the group's address XOR a constant, and only the low 5 bits of that need
+//     an instruction;
+//   * R >= 5: one padding word after every 2^R (an address stays base + constant): lanes
+//     32 or 64 positions apart fall on distinct banks, runs of 32 stay together.
+// Every pass, slot and warp of every plan was checked for conflicts on the host.
+template <int R>
+struct XMap {
+    static constexpr bool SWZ = R == 3 || R == 4;
+    __host__ __device__ static constexpr int map(int pos) {
         const int x = pos >> 5;
-        if constexpr (R == 3) return pos ^ (x & 7) ^ (((x >> 1) & 3) << 3);
-        else return pos ^ (x & 15) ^ (((x >> 3) & 1) << 4);
+        if (R == 3) return pos ^ (x & 7) ^ (((x >> 1) & 3) << 3);
+        if (R == 4) return pos ^ (x & 15) ^ (((x >> 3) & 1) << 4);
+        return pos + (pos >> (R >= 6 ? 6 : 5));
+    }
+    // address of the position g | k from base = map(g), for k with no bit in common with g
+    __device__ __forceinline__ static int at(int base, int k) {
+        const int c = map(k);
+        return SWZ ? (base ^ (c & 31)) + (c & ~31) : base + c;
     }
 };
 
@@ -219,58 +218,62 @@ __device__ __forceinline__ void inv_pass(uint32_t (&x)[NOPS][PL::E], const uint2
     }
 }
 
-// Registers laid out for pass PA -> registers laid out for pass PB, through
-// shared memory `sm` (NOPS buffers of SMW words). Callers that alternate
-// between two such regions need one barrier (the next write cannot race with a
-// slow reader of this region); a caller with a single region passes
-// `sync_before` to add a barrier ahead of the writes.
+// Registers laid out for pass PA -> registers laid out for pass PB (a neighbour), through
+// shared memory `sm` (NOPS buffers of SMW words). In place: every exchange of a plan uses
+// one layout, so a thread writes exactly the words it read in the exchange before, and one
+// barrier, between the writes and the reads, is enough. Only the first forward exchange
+// into a buffer whose words other threads may still be reading (the transform before)
+// needs one ahead of its writes (`sync_before`). When the passes' sub-transforms (the N >> S0
+// positions that the earlier pass's butterflies stay within) belong to one warp, the
+// barrier is the warp's.
+// Two alternating regions (fewer blocks per SM), or two barriers per exchange, took its place
+// before. With 16 coefficients per thread, 512 products at N = 4096, 127-bit q: 164 -> 150 us, 512
+// keyswitches 171 -> 154 us; 512 x 14 transforms of length 8192: 220 -> 158 us forward, 212 ->
+// 161 us inverse.
 template <class PL, int PA, int PB, int NOPS, class Sync = CtaSync>
 __device__ __forceinline__ void exchange(uint32_t (&x)[NOPS][PL::E], uint32_t* sm, int tau, bool sync_before,
                                          Sync bar = Sync()) {
     constexpr int RA = PL::R(PA), LA = PL::LOGD(PA), NVA = PL::E >> RA;
     constexpr int RB = PL::R(PB), LB = PL::LOGD(PB), NVB = PL::E >> RB;
-    using X = XLayout<PL::LOGE, LA, LB>;
+    constexpr int PLO = PA < PB ? PA : PB;
+    // threads that share a sub-transform of pass PLO (whole warps hold whole groups)
+    constexpr bool WARP = PL::G >= 32 && ((PL::N >> PL::S0(PLO)) >> PL::LOGE) <= 32;
+    using X = XMap<PL::LOGE>;
     if (sync_before) bar.sync();
 #pragma unroll
     for (int v = 0; v < NVA; v++) {
-        const int g = group_base<PL, PA>(tau, v);  // bits of u << LA are zero in g
-        const int base = X::pad(g);
+        const int base = X::map(group_base<PL, PA>(tau, v));  // bits of u << LA are zero in it
 #pragma unroll
         for (int u = 0; u < (1 << RA); u++) {
-            const int a = X::SWZ ? X::swz(g | (u << LA)) : base + X::pad(u << LA);
+            const int a = X::at(base, u << LA);
 #pragma unroll
             for (int o = 0; o < NOPS; o++) sm[o * PL::SMW + a] = x[o][(v << RA) + u];
         }
     }
-    bar.sync();
+    if constexpr (WARP) __syncwarp();
+    else bar.sync();
 #pragma unroll
     for (int v = 0; v < NVB; v++) {
-        const int g = group_base<PL, PB>(tau, v);
-        const int base = X::pad(g);
+        const int base = X::map(group_base<PL, PB>(tau, v));
 #pragma unroll
         for (int u = 0; u < (1 << RB); u++) {
-            const int a = X::SWZ ? X::swz(g | (u << LB)) : base + X::pad(u << LB);
+            const int a = X::at(base, u << LB);
 #pragma unroll
             for (int o = 0; o < NOPS; o++) x[o][(v << RB) + u] = sm[o * PL::SMW + a];
         }
     }
 }
 
-// Forward passes PASS .. NPASS-1. `buf` counts the exchanges made so far by the
-// block; exchange number b uses region (b & 1) of `sm`, regions `stride` words
-// apart (stride >= NOPS * SMW for every NOPS the kernel uses), or the single
-// region `sm` when stride == 0. Returns the updated count.
+// Forward passes PASS .. NPASS-1 (sync_before: as in exchange, for the first one).
 template <class PL, int PASS, int NOPS, class Sync = CtaSync>
 struct FwdFrom {
-    __device__ __forceinline__ static int run(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw,
-                                              const Mod& m, int tau, uint32_t* sm, int stride, int buf,
-                                              Sync bar = Sync(), int tm = 1, const uint2* __restrict__ twr = nullptr) {
-        if constexpr (PASS >= PL::NPASS) {
-            return buf;
-        } else {
-            exchange<PL, PASS - 1, PASS, NOPS, Sync>(x, sm + (buf & 1) * stride, tau, stride == 0, bar);
+    __device__ __forceinline__ static void run(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw,
+                                               const Mod& m, int tau, uint32_t* sm, bool sync_before,
+                                               Sync bar = Sync(), int tm = 1, const uint2* __restrict__ twr = nullptr) {
+        if constexpr (PASS < PL::NPASS) {
+            exchange<PL, PASS - 1, PASS, NOPS, Sync>(x, sm, tau, sync_before, bar);
             fwd_pass<PL, PASS, NOPS>(x, tw, m, tau, tm, twr);
-            return FwdFrom<PL, PASS + 1, NOPS, Sync>::run(x, tw, m, tau, sm, stride, buf + 1, bar, tm, twr);
+            FwdFrom<PL, PASS + 1, NOPS, Sync>::run(x, tw, m, tau, sm, false, bar, tm, twr);
         }
     }
 };
@@ -278,38 +281,38 @@ struct FwdFrom {
 // Inverse passes PASS .. 0 where pass PASS+1 was the previous one.
 template <class PL, int PASS, int NOPS, class Sync = CtaSync>
 struct InvFrom {
-    __device__ __forceinline__ static int run(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw,
-                                              const Mod& m, int tau, uint32_t* sm, int stride, int buf,
-                                              Sync bar = Sync(), int tm = 1, const uint2* __restrict__ twr = nullptr,
-                                              const uint32_t* __restrict__ scale = nullptr) {
-        if constexpr (PASS < 0) {
-            return buf;
-        } else {
-            exchange<PL, PASS + 1, PASS, NOPS, Sync>(x, sm + (buf & 1) * stride, tau, stride == 0, bar);
+    __device__ __forceinline__ static void run(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw,
+                                               const Mod& m, int tau, uint32_t* sm, Sync bar = Sync(), int tm = 1,
+                                               const uint2* __restrict__ twr = nullptr,
+                                               const uint32_t* __restrict__ scale = nullptr) {
+        if constexpr (PASS >= 0) {
+            exchange<PL, PASS + 1, PASS, NOPS, Sync>(x, sm, tau, false, bar);
             inv_pass<PL, PASS, NOPS>(x, tw, m, tau, tm, twr, scale);
-            return InvFrom<PL, PASS - 1, NOPS, Sync>::run(x, tw, m, tau, sm, stride, buf + 1, bar, tm, twr, scale);
+            InvFrom<PL, PASS - 1, NOPS, Sync>::run(x, tw, m, tau, sm, bar, tm, twr, scale);
         }
     }
 };
 
 // Full forward transform: registers in pass-0 layout (natural order) ->
-// registers in last-pass layout (bit-reversed order).
+// registers in last-pass layout (bit-reversed order). sync_before: other threads may still
+// be reading `sm` (a transform before this one in the same block).
 template <class PL, int NOPS, class Sync = CtaSync>
-__device__ __forceinline__ int ntt_forward(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
-                                           int tau, uint32_t* sm, int stride, int buf, Sync bar = Sync(),
-                                           int tm = 1, const uint2* __restrict__ twr = nullptr) {
+__device__ __forceinline__ void ntt_forward(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
+                                            int tau, uint32_t* sm, bool sync_before = false, Sync bar = Sync(),
+                                            int tm = 1, const uint2* __restrict__ twr = nullptr) {
     fwd_pass<PL, 0, NOPS>(x, tw, m, tau, tm, twr);
-    return FwdFrom<PL, 1, NOPS, Sync>::run(x, tw, m, tau, sm, stride, buf, bar, tm, twr);
+    FwdFrom<PL, 1, NOPS, Sync>::run(x, tw, m, tau, sm, sync_before, bar, tm, twr);
 }
 
-// Full inverse transform: registers in last-pass layout -> pass-0 layout.
+// Full inverse transform: registers in last-pass layout -> pass-0 layout. `sm` may hold a
+// forward transform of this block (each thread then writes the words it read last).
 template <class PL, int NOPS, class Sync = CtaSync>
-__device__ __forceinline__ int ntt_inverse(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
-                                           int tau, uint32_t* sm, int stride, int buf, Sync bar = Sync(),
-                                           int tm = 1, const uint2* __restrict__ twr = nullptr,
-                                           const uint32_t* __restrict__ scale = nullptr) {
+__device__ __forceinline__ void ntt_inverse(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
+                                            int tau, uint32_t* sm, Sync bar = Sync(), int tm = 1,
+                                            const uint2* __restrict__ twr = nullptr,
+                                            const uint32_t* __restrict__ scale = nullptr) {
     inv_pass<PL, PL::NPASS - 1, NOPS>(x, tw, m, tau, tm, twr, scale);
-    return InvFrom<PL, PL::NPASS - 2, NOPS, Sync>::run(x, tw, m, tau, sm, stride, buf, bar, tm, twr, scale);
+    InvFrom<PL, PL::NPASS - 2, NOPS, Sync>::run(x, tw, m, tau, sm, bar, tm, twr, scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -407,13 +410,11 @@ __device__ __forceinline__ void ntt64_forward(uint32_t (&x)[NOPS][64], const uin
     }
 }
 
-// Inverse transform, row layout -> column layout; `sync_before`: a barrier
-// before the exchange's writes (the region was read just before); scale as in
-// inv_pass (or null).
+// Inverse transform, row layout -> column layout; scale as in inv_pass (or null).
 template <class PL, int NOPS>
 __device__ __forceinline__ void ntt64_inverse(uint32_t (&x)[NOPS][64], const uint2* __restrict__ tw,
                                               const uint2* __restrict__ twr, const Mod& m, int tau, uint32_t* sm,
-                                              bool sync_before, const uint32_t* __restrict__ scale) {
+                                              const uint32_t* __restrict__ scale) {
     static_assert(PL::LOGN == 12 && PL::LOGE == 6, "two passes of six stages");
 #pragma unroll 1
     for (int it = 0; it < 2; it++) {
@@ -422,7 +423,7 @@ __device__ __forceinline__ void ntt64_inverse(uint32_t (&x)[NOPS][64], const uin
         int tws;
         pass64_twiddles(pass, tw, twr, tau, twp, tws);
         inv_pass64<NOPS>(x, twp, tws, m, pass == 0 ? scale : nullptr);
-        if (pass == 1) exchange<PL, 1, 0, NOPS>(x, sm, tau, sync_before);
+        if (pass == 1) exchange<PL, 1, 0, NOPS>(x, sm, tau, false);
     }
 }
 
