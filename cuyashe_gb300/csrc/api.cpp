@@ -161,7 +161,7 @@ static cy_status check_device(int device) {
     return CY_OK;
 }
 
-int tuned_variant(int logn, int l64, int op);
+int tuned_variant(int logn, int l64, int op, long long blocks);
 cy_status run_mixed(const std::vector<const cy_polymul_job*>& jobs, cudaStream_t st);
 cy_status mixed_status(cudaStream_t st);
 bool mixed_supported(const cy_ring* r);
@@ -263,10 +263,11 @@ static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, l
                              const uint64_t* b, long long b_stride, void* out, long long out_stride, int batch,
                              Workspace& ws, cudaStream_t st, int variant = -1) {
     if (batch == 0) return CY_OK;
+    const int n = B.h.n, k = B.h.k, jobs = std::min(batch, chunk_jobs(n, k));
     const KernelSet& ks = kernel_variant(
-        B.h.logn, variant >= 0 ? variant : tuned_variant(B.h.logn, B.h.l64, centered ? TUNE_MULC : TUNE_MUL));
-    const int n = B.h.n, k = B.h.k;
-    const int chunk = product_chunk_jobs(B, ks, centered, std::min(batch, chunk_jobs(n, k)));
+        B.h.logn, variant >= 0 ? variant
+                               : tuned_variant(B.h.logn, B.h.l64, centered ? TUNE_MULC : TUNE_MUL, (long long)jobs * k));
+    const int chunk = product_chunk_jobs(B, ks, centered, jobs);
     const int nchunks = (batch + chunk - 1) / chunk;
     Lanes L;
     CY_TRY(L.begin(ws, st, (size_t)chunk * k * n, nchunks));
@@ -288,13 +289,13 @@ static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint32_t
                                int batch, Workspace& ws, cudaStream_t st, int variant = -1, int chunk_k = 0,
                                int lm = 0) {
     if (batch == 0) return CY_OK;
-    const KernelSet& ks =
-        kernel_variant(B.h.logn, variant >= 0 ? variant : tuned_variant(B.h.logn, B.h.l64, TUNE_KS));
     const int n = B.h.n, k = B.h.k, l64 = B.h.l64;
+    const int jobs = std::min(batch, chunk_jobs(n, chunk_k > 0 ? std::max(k, chunk_k) : k));
+    const KernelSet& ks = kernel_variant(
+        B.h.logn, variant >= 0 ? variant : tuned_variant(B.h.logn, B.h.l64, TUNE_KS, (long long)jobs * k));
     int sel = 0;
     CY_TRY(keyswitch_digits_per_pass(ks, ell, &sel));
-    const int chunk = wave_chunk(std::min(batch, chunk_jobs(n, chunk_k > 0 ? std::max(k, chunk_k) : k)),
-                                 ks.ks_for(l64, sel), ks.threads, ks.smem_ks[sel], k * ks.blocks_per_prime);
+    const int chunk = wave_chunk(jobs, ks.ks_for(l64, sel), ks.threads, ks.smem_ks[sel], k * ks.blocks_per_prime);
     const int nchunks = (batch + chunk - 1) / chunk;
     Lanes L;
     CY_TRY(L.begin(ws, st, (size_t)chunk * k * n, nchunks));
@@ -316,13 +317,16 @@ cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t*
                         int ks_variant) {
     if (batch == 0) return CY_OK;
     const int n = tensor.h.n, l64 = tensor.h.l64;
-    const KernelSet& kt = kernel_variant(tensor.h.logn, tuned_variant(tensor.h.logn, l64, TUNE_MULC));
-    const KernelSet& kr = kernel_variant(
-        relin.h.logn, ks_variant >= 0 ? ks_variant : tuned_variant(relin.h.logn, l64, TUNE_KS));
     const int kmax = std::max(tensor.h.k, do_relin ? relin.h.k : 0);
+    int chunk = std::min(batch, chunk_jobs(n, kmax));
+    const KernelSet& kt = kernel_variant(
+        tensor.h.logn, tuned_variant(tensor.h.logn, l64, TUNE_MULC, (long long)chunk * tensor.h.k));
+    const KernelSet& kr =
+        kernel_variant(relin.h.logn, ks_variant >= 0 ? ks_variant
+                                                     : tuned_variant(relin.h.logn, l64, TUNE_KS,
+                                                                     (long long)chunk * relin.h.k));
     int sel = 0;
     if (do_relin) CY_TRY(keyswitch_digits_per_pass(kr, ell, &sel));
-    int chunk = std::min(batch, chunk_jobs(n, kmax));
     if (do_relin)  // whole waves of the keyswitch
         chunk = wave_chunk(chunk, kr.ks_for(l64, sel), kr.threads, kr.smem_ks[sel], relin.h.k * kr.blocks_per_prime);
     const int nchunks = (batch + chunk - 1) / chunk;
@@ -357,7 +361,8 @@ static cy_status run_ntt(const Basis& B, uint32_t* res, int batch, bool inverse,
                          int variant = -1) {
     if (batch == 0) return CY_OK;
     const KernelSet& ks =
-        kernel_variant(B.h.logn, variant >= 0 ? variant : tuned_variant(B.h.logn, B.h.l64, TUNE_NTT));
+        kernel_variant(B.h.logn, variant >= 0 ? variant
+                                              : tuned_variant(B.h.logn, B.h.l64, TUNE_NTT, (long long)batch * B.h.k));
     const uint32_t* ninv = B.d_ninv;
     const long long rows = (long long)batch * B.h.k * (B.h.n / 64);
     if (inverse && ks.intt_tma && B.h.logn == 12 && ntt_tma_usable(res, rows)) {  // input tiles by TMA
@@ -432,7 +437,7 @@ int yashe_chunk_jobs(const Basis& tensor, const Basis& relin, int ell, bool do_r
     const int n = tensor.h.n, l64 = tensor.h.l64;
     int chunk = chunk_jobs(n, std::max(tensor.h.k, do_relin ? relin.h.k : 0));
     if (do_relin) {
-        const KernelSet& kr = kernel_variant(relin.h.logn, tuned_variant(relin.h.logn, l64, TUNE_KS));
+        const KernelSet& kr = kernel_variant(relin.h.logn, tuned_variant(relin.h.logn, l64, TUNE_KS, (long long)chunk * relin.h.k));
         int sel = 0;
         if (keyswitch_digits_per_pass(kr, ell, &sel) == CY_OK)
             chunk = wave_chunk(chunk, kr.ks_for(l64, sel), kr.threads, kr.smem_ks[sel], relin.h.k * kr.blocks_per_prime);
@@ -600,8 +605,10 @@ cy_status cy_polymul(cy_ring* r, const uint64_t* d_a, const uint64_t* d_b, uint6
 cy_status cy_polymul_host(cy_ring* r, const uint64_t* h_a, const uint64_t* h_b, uint64_t* h_c, int batch) {
     CY_TRY(validate_poly_args(r, h_a, h_b, h_c, batch));
     if (batch == 0) return CY_OK;
-    const KernelSet& ks = kernel_variant(r->mul.h.logn, tuned_variant(r->mul.h.logn, r->mul.h.l64, TUNE_MUL));
-    const int chunk = product_chunk_jobs(r->mul, ks, false, chunk_jobs(r->n, r->mul.h.k));
+    const int jobs = std::min(batch, chunk_jobs(r->n, r->mul.h.k));
+    const KernelSet& ks = kernel_variant(
+        r->mul.h.logn, tuned_variant(r->mul.h.logn, r->mul.h.l64, TUNE_MUL, (long long)jobs * r->mul.h.k));
+    const int chunk = product_chunk_jobs(r->mul, ks, false, jobs);
     return run_host_pipeline((size_t)r->n * r->l64, batch, chunk, h_a, h_b, h_c,
                              [r](cy_workspace* ws, const uint64_t* a, const uint64_t* b, uint64_t* c, int nj,
                                  cudaStream_t st) { return cy_polymul_ws(r, ws, a, b, c, nj, st); });

@@ -24,9 +24,8 @@ struct KernelSet {
 
 // Kernel sets for transforms of length 2^logn (1 <= logn <= LOGN_MAX). Each
 // length has one or more schedules ("variants": coefficients per thread, hence
-// threads per transform and passes); variant 0 is the default, the autotuner
-// may pick another per ring (tuning.cpp).
-const KernelSet& kernel_set(int logn);
+// threads per transform and passes); the autotuner may pick one per ring, else
+// default_variant does (tuning.cpp).
 int variant_count(int logn);
 const KernelSet& kernel_variant(int logn, int v);
 

@@ -46,7 +46,6 @@ static const VariantTable& variants() {
             fill(ks);
             T.v[logn].push_back(ks);
         };
-        // variant 0 first: the default schedule of each length
         add(10, fill_n10_e3);
         add(10, fill_n10_e4);
         add(11, fill_n11_e3);
@@ -86,7 +85,6 @@ const KernelSet& kernel_variant(int logn, int v) {
     const std::vector<KernelSet>& vs = variants().v[logn];
     return vs[(v >= 0 && v < (int)vs.size()) ? v : 0];
 }
-const KernelSet& kernel_set(int logn) { return kernel_variant(logn, 0); }
 
 #define CY_EPI_ROW(L) {(void*)k_epi<L, EPI_MODQ>, (void*)k_epi<L, EPI_YASHE>, (void*)k_epi<L, EPI_DECRYPT>}
 

@@ -18,6 +18,7 @@
 
 namespace cy {
 
+int default_variant(int logn, int l64, int op, long long blocks);
 int trace_begin(const char* name, int logn, cudaStream_t st);
 void trace_end(int idx, cudaStream_t st);
 
@@ -91,7 +92,8 @@ extern "C" cy_status cy_polymul_noalloc(cy_ring* r, const uint64_t* d_a, const u
     // Nothing in the scratch has to start at zero: the product kernel writes every
     // residue word that the epilogue of the same call reads.
     cudaStream_t st = (cudaStream_t)stream;
-    const KernelSet& ks = kernel_set(B.h.logn);
+    const KernelSet& ks =
+        kernel_variant(B.h.logn, default_variant(B.h.logn, B.h.l64, TUNE_MUL, (long long)batch * k));
     const BasisDev* Bd = B.d;
     long long stride = (long long)n * r->l64;
     void* args[] = {(void*)&B.prod, (void*)&d_a, (void*)&stride, (void*)&d_b, (void*)&stride, (void*)&scratch};

@@ -43,12 +43,66 @@ static const char* kOpNames[TUNE_OPS] = {"mul", "mulc", "ks", "ntt"};
 static std::mutex g_mu;
 static std::map<std::tuple<int, int, int, int>, int> g_choice;  // (device, logn, l64, op) -> variant
 
-int tuned_variant(int logn, int l64, int op) {
+// SMs of the current device (the GB300's 152 if it cannot be queried).
+static int sm_count() {
+    static std::mutex mu;
+    static std::map<int, int> known;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 152;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(dev);
+    if (it != known.end()) return it->second;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 152;
+    return known[dev] = sms;
+}
+
+// The schedule of a call that the autotuner has not chosen one for: `blocks` transforms'
+// blocks per launch (jobs times primes). Two regimes: up to one block per SM the time is one
+// block's latency (more threads per transform, or a pair of blocks); above, throughput. The
+// lines, measured with every schedule at q of 62, 127 (or 190) and 380 bits (us per call,
+// the schedule taken first):
+//   N = 1024   products of six limbs: 16 coefficients per thread from two blocks per SM on
+//              (512: 181 against 242; one: 17.0 against 15.2); all else within 3%
+//   N = 4096   products: 16 per thread, three blocks per SM (2048, 127-bit: 583 against 678 with
+//              8 per thread; one: 12.5 against 14.3). Keyswitch: 16 per thread, two blocks (2048:
+//              591 against 636), up to one block per SM 8 per thread, whole register file
+//              (one: 14.7 against 15.7). Transforms: 16 per thread (2048: 160 against 187)
+//   N = 8192   products: 16 per thread, two blocks (512, 190-bit: 670 against 721), up to one
+//              block per SM 128 registers (380-bit, one: 27.1 against 29.2). Keyswitch: 16 per
+//              thread and 128 registers (512, 190-bit: 712 against 1020, 64 registers spill),
+//              one limb two blocks (512: 149 against 173)
+//   N = 16384  up to one block per SM a pair of blocks per prime (380-bit, one: product 33
+//              against 50, keyswitch 78 against 165), above 32 per thread (64: 465 against 524
+//              and 885 against 1139), one limb 16 per thread (64: product 71 against 78,
+//              keyswitch 52 against 60)
+int default_variant(int logn, int l64, int op, long long blocks) {
+    const int sms = sm_count();
+    const bool small = blocks <= sms;
+    const bool product = op == TUNE_MUL || op == TUNE_MULC;
+    switch (logn) {
+        case 10: return product && l64 == 6 && blocks >= 2 * sms ? 1 : 0;
+        case 12: return op == TUNE_KS ? (small ? 2 : 3) : 8;
+        case 13:
+            if (op == TUNE_KS) return l64 == 1 ? 0 : 2;
+            return product && small ? 2 : 0;
+        case 14:
+            if (op == TUNE_NTT) return 0;
+            if (2 * blocks <= sms) return 3;
+            return l64 == 1 ? 0 : 1;
+        default: return 0;
+    }
+}
+
+// The autotuner's (or an imported) choice, else the default for `blocks`.
+int tuned_variant(int logn, int l64, int op, long long blocks) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    std::lock_guard<std::mutex> lock(g_mu);
-    auto it = g_choice.find(std::make_tuple(dev, logn, l64, op));
-    return it == g_choice.end() ? 0 : it->second;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto it = g_choice.find(std::make_tuple(dev, logn, l64, op));
+        if (it != g_choice.end()) return it->second;
+    }
+    return default_variant(logn, l64, op, blocks);
 }
 
 static void set_choice(int dev, int logn, int l64, int op, int v) {
