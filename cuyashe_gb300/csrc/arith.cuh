@@ -15,6 +15,49 @@
 
 namespace cy {
 
+// Programmatic dependent launch: a kernel launched with that attribute may start while
+// the kernel before it in the stream drains. dep_wait() returns once that one has finished
+// and its writes are visible; nothing that an earlier kernel writes is read, and nothing it
+// reads is written, before it. dep_launch() lets the next kernel start once every block has
+// called it: near a kernel's end, when its blocks leave the SMs together. (Called at the
+// start, the next kernel's blocks pile up on the SMs that drain first: 42 products of six
+// limbs at N = 1024 took 40 us instead of 28.) Both do nothing in ordinary launches.
+//
+// Data that an earlier kernel may have written is read with ld_dep from pointers that went
+// through dep_wait: plain loads (a read-only load may move above the wait), which cannot
+// precede it because their address comes out of it, and which the compiler is otherwise
+// free to order.
+template <class P>
+__device__ __forceinline__ void dep_wait(P*& p) {
+    asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+}
+template <class P>
+__device__ __forceinline__ void dep_wait(P*& p, P*& q) {
+    asm volatile("griddepcontrol.wait;" : "+l"(p), "+l"(q) : : "memory");
+}
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ uint4 ld_dep(const uint4* p) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_dep(const uint2* p) {
+    uint2 v;
+    asm("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint64_t ld_dep(const uint64_t* p) {
+    uint64_t v;
+    asm("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_dep_cg(const uint32_t* p) {
+    uint32_t v;
+    asm("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // x in [0, 2m) -> [0, m)   (x - m wraps above x when x < m)
 __device__ __forceinline__ uint32_t red(uint32_t x, uint32_t m) { return __viaddmin_u32(x, 0u - m, x); }
 

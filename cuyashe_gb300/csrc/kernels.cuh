@@ -99,7 +99,7 @@ __device__ __forceinline__ uint32_t crt_coef(const uint64_t* __restrict__ src, i
     uint64_t T = 0;
     bool gt = false;
     for (int j = 0; j < l64; j++) {
-        const uint64_t limb = __ldg(s + j);
+        const uint64_t limb = ld_dep(s + j);
         const uint32_t lo = (uint32_t)limb, hi = (uint32_t)(limb >> 32);
         T = lazy_high(T, c.m) + (uint64_t)lo * crt[2 * j] + (uint64_t)hi * crt[2 * j + 1];
         if (CENTER) {
@@ -116,7 +116,7 @@ __device__ __forceinline__ void load_words(const uint64_t* __restrict__ p, uint3
     if constexpr (L64 % 2 == 0) {
 #pragma unroll
         for (int i = 0; i < L64 / 2; i++) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
+            const uint4 v = ld_dep(reinterpret_cast<const uint4*>(p) + i);
             w[4 * i] = v.x;
             w[4 * i + 1] = v.y;
             w[4 * i + 2] = v.z;
@@ -125,7 +125,7 @@ __device__ __forceinline__ void load_words(const uint64_t* __restrict__ p, uint3
     } else {
 #pragma unroll
         for (int i = 0; i < L64; i++) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(p) + i);
+            const uint2 v = ld_dep(reinterpret_cast<const uint2*>(p) + i);
             w[2 * i] = v.x;
             w[2 * i + 1] = v.y;
         }
@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
 
     const uint64_t* a = A + (size_t)job * a_stride;
     const uint64_t* b = Bv + (size_t)job * b_stride;
+    dep_wait(a, b);
     uint32_t x[2][E];
     if constexpr (L64 > 0) {
         constexpr int W = 2 * L64;
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
     if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, rows_of(M.ipsi_r, prime), c.m, tau, smem, nullptr);
     else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime));
+    dep_launch();
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = z[0][e];
@@ -351,6 +353,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     // loads of one limb are then contiguous). Kernel parameters, so that they stay
     // in the constant bank.
 
+    dep_wait(cj);
     uint64_t T[E];           // sums of products
     uint32_t acc[1][E];      // reduced sums: the inverse transform's input
 #pragma unroll
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
                 bool both = false;  // two limbs side by side: one 16-byte load
                 if constexpr (ND == 4 && L64 % 2 == 0) {
                     if (ls == 1) {
-                        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+                        const uint4 v = ld_dep(reinterpret_cast<const uint4*>(src));
                         w[0] = v.x;
                         w[1] = v.y;
                         w[ND - 2] = v.z;
@@ -382,7 +385,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
                 if (!both) {
 #pragma unroll
                     for (int o = 0; o < ND; o += 2) {
-                        const uint2 v = __ldg(reinterpret_cast<const uint2*>(src + (o >> 1) * ls));
+                        const uint2 v = ld_dep(reinterpret_cast<const uint2*>(src + (o >> 1) * ls));
                         w[o] = v.x;
                         w[o + 1] = v.y;
                     }
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
                     const int d = d0 + o;
                     uint32_t w = 0;
                     if (d < ell) {
-                        const uint64_t limb = __ldg(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
+                        const uint64_t limb = ld_dep(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
                         w = (uint32_t)(limb >> (32 * (d & 1)));
                     }
                     x[o][e] = red_2p(w, m);  // digit < 2^32 < 6p -> [0, 4p)
@@ -454,6 +457,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     }
     if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, rows_of(M.ipsi_r, prime), m, tau, smem, nullptr);
     else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime));
+    dep_launch();
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = acc[0][e];
@@ -1047,7 +1051,7 @@ __device__ __noinline__ uint64_t yashe_round_exact_g(const BasisDev* __restrict_
     c1.zero();
     for (int i = 0; i < k; i++) {
         const uint32_t p = B->p[i];
-        const uint32_t y = red(shoup(__ldcg(r0 + (size_t)i * stride), B->ycon[i], B->ycon_sh[i], p), p);
+        const uint32_t y = red(shoup(ld_dep_cg(r0 + (size_t)i * stride), B->ycon[i], B->ycon_sh[i], p), p);
         c1.mac(y, B->A1[i]);
         if (i % 3 == 2) c1.norm();
     }
@@ -1130,6 +1134,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
     const long long job = idx >> logn;
     const int coef = (int)(idx & (n - 1));
     const uint32_t* r0 = resid + (size_t)job * k * n + coef;
+    dep_wait(r0);
 
     Cols<L> x;   // sum y_i A0_i
     Cols<2> z;   // YASHE: Z = sum y_i F_i in 32-bit columns
@@ -1149,7 +1154,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
     if constexpr (K > 0) {
         uint32_t r[K];
 #pragma unroll
-        for (int i = 0; i < K; i++) r[i] = __ldcg(r0 + (size_t)i * n);
+        for (int i = 0; i < K; i++) r[i] = ld_dep_cg(r0 + (size_t)i * n);
 #pragma unroll
         for (int i = 0; i < K; i++) {
             absorb(P.pr[i], r[i]);
@@ -1163,7 +1168,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
         uint32_t cur[4], nxt[4];
         auto load = [&](int i, uint32_t(&d)[4]) {  // past the last prime: its residue again, not used
 #pragma unroll
-            for (int j = 0; j < 4; j++) d[j] = __ldcg(r0 + (size_t)min(i + j, k - 1) * n);
+            for (int j = 0; j < 4; j++) d[j] = ld_dep_cg(r0 + (size_t)min(i + j, k - 1) * n);
         };
         load(0, cur);
 #pragma unroll 1
@@ -1203,6 +1208,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
 #pragma unroll
     for (int w = 0; w < L; w++) qn[w] = P.qn[w];
     barrett_c<L>(x, qn, P.mu_lo, P.mu_hi, rm);  // rm = (result mod q) << shift
+    dep_launch();
     if constexpr (MODE == EPI_DECRYPT) {
         Cols<L> c2;
 #pragma unroll

@@ -58,6 +58,7 @@ __device__ __forceinline__ void pair_finish(uint32_t (&x)[1][PairPlan::E], uint3
 #pragma unroll
     for (int e = 0; e < E; e++) store_peer(&recv[slot_pos<PairPlan, 0>(tau, e)], h ^ 1u, x[0][e]);
     cluster_barrier();  // the peer's half has arrived
+    dep_launch();
 #pragma unroll
     for (int e = 0; e < E; e++) {
         const int pos = slot_pos<PairPlan, 0>(tau, e);
@@ -92,6 +93,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     // exchange, which follows the barrier below)
     const uint64_t* a = A + (size_t)job * a_stride + (size_t)h * kPairHalf * l64;
     const uint64_t* b = Bv + (size_t)job * b_stride + (size_t)h * kPairHalf * l64;
+    dep_wait(a, b);
     uint32_t x[2][E];
 #pragma unroll
     for (int e = 0; e < E; e++) {
@@ -164,6 +166,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const int tm = 2 + (int)h;
     const uint2 w0 = __ldg(psi + 1);
     cluster_barrier();  // both blocks have started before any remote store
+    dep_wait(cj);
 
     uint64_t T[E];  // sums of products with the key (see k_keyswitch)
 #pragma unroll
@@ -179,8 +182,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
                 const int d = d0 + o;
                 uint32_t wl = 0, wh = 0;
                 if (L64 > 0 || d < ell) {  // digits past the top word of q are zero
-                    const uint64_t ll = __ldg(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
-                    const uint64_t lh = __ldg(cj + (size_t)(pos + kPairHalf) * cs + (size_t)(d >> 1) * ls);
+                    const uint64_t ll = ld_dep(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
+                    const uint64_t lh = ld_dep(cj + (size_t)(pos + kPairHalf) * cs + (size_t)(d >> 1) * ls);
                     wl = (uint32_t)(ll >> (32 * (d & 1)));
                     wh = (uint32_t)(lh >> (32 * (d & 1)));
                 }
