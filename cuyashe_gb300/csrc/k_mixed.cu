@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(MixedSched<LOGE>::THREADS, MixedSched<LOGE>::M
             uint32_t* __restrict__ done, uint32_t* __restrict__ ctl, unsigned spin_limit,
             unsigned long long frac_limit) {
     constexpr int THREADS = MixedSched<LOGE>::THREADS;
-    extern __shared__ uint32_t smem[];
+    extern __shared__ __align__(16) uint32_t smem[];
     __shared__ EpiShared S;
     __shared__ int s_unit, s_ok;
     for (;;) {

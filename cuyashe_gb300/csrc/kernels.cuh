@@ -219,6 +219,13 @@ constexpr int ks_min_blocks() {
     return target < 1 ? 1 : (target > 16 ? 16 : target);
 }
 
+template <int LOGN, int LOGE>
+constexpr int ntt_min_blocks() {
+    constexpr int G = NttPlan<LOGN, LOGE>::G;
+    constexpr int target = (LOGE <= 4 ? 1024 : 512) / G;
+    return target < 1 ? 1 : (target > 16 ? 16 : target);
+}
+
 // MINB > 0 overrides the blocks per SM the kernel is compiled for (a schedule
 // with a larger register budget per thread).
 template <int LOGN, int LOGE, int L64, bool CENTER, int MINB = 0>
@@ -227,7 +234,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
           const uint64_t* __restrict__ Bv, long long b_stride, uint32_t* __restrict__ resid) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
-    extern __shared__ uint32_t smem[];  // exchange buffer, 2 operands x SMW
+    extern __shared__ __align__(16) uint32_t smem[];  // exchange buffer, 2 operands x SMW
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
@@ -337,7 +344,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     constexpr int LAST = PL::NPASS - 1;
     constexpr bool ONE = ks_one_pass<L64, ND>();
     constexpr bool ACC32 = !ONE && LOGE > 4;
-    extern __shared__ uint32_t smem[];  // exchange buffer, ND operands x SMW
+    extern __shared__ __align__(16) uint32_t smem[];  // exchange buffer, ND operands x SMW
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
     const int job = blockIdx.x;
@@ -471,13 +478,13 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
 // once.
 // --------------------------------------------------------------------------
 template <int LOGN, int LOGE, bool INV>
-__global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G)
+__global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, LOGE>()))
     k_ntt(const __grid_constant__ ProdParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
           int njobs) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
     constexpr int LAST = PL::NPASS - 1;
-    extern __shared__ uint32_t smem[];
+    extern __shared__ __align__(16) uint32_t smem[];
     const int tau = threadIdx.x;
     const int prime = blockIdx.x;
     const int job0 = 2 * blockIdx.y;
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
     constexpr int E = PL::E;
     constexpr int LAST = PL::NPASS - 1;
     static_assert(!COAL || (PL::NPASS == 2 && LOGE == 6 && LOGN == 12), "row-side staging: N = 4096, E = 64");
-    extern __shared__ uint32_t smem_all[];
+    extern __shared__ __align__(16) uint32_t smem_all[];
     const int sub = TPB > 1 ? (int)threadIdx.x / PL::G : 0;
     const int tau = TPB > 1 ? (int)threadIdx.x % PL::G : (int)threadIdx.x;
     uint32_t* smem = smem_all + sub * PL::SMW;

@@ -75,7 +75,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
                const uint64_t* __restrict__ Bv, long long b_stride, uint32_t* __restrict__ resid) {
     using PL = PairPlan;
     constexpr int E = PL::E;
-    extern __shared__ uint32_t smem[];
+    extern __shared__ __align__(16) uint32_t smem[];
     const int tau = threadIdx.x;
     const uint32_t h = cluster_rank();
     const int prime = blockIdx.y;
@@ -148,7 +148,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
                      int ell, uint32_t* __restrict__ resid, int cs, int ls) {
     using PL = PairPlan;
     constexpr int E = PL::E;
-    extern __shared__ uint32_t smem[];
+    extern __shared__ __align__(16) uint32_t smem[];
     const int tau = threadIdx.x;
     const uint32_t h = cluster_rank();
     const int prime = blockIdx.y;

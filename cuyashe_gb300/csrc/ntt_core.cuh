@@ -64,10 +64,11 @@ struct GroupSync {
 // (D = LOGD) a warp touches 32 consecutive positions when D >= 5, else 32/2^D runs of
 // 2^D positions 2^(D+R) apart; D is 0, R, 2R, .. . One layout for all of them, free of bank
 // conflicts, so that every exchange of a plan is in place:
-//   * R = 3, 4: an XOR of the low 5 bits with bits of the row (pos >> 5), which permutes
-//     words inside each 32-word row. It is linear over XOR, so the address of slot u of a
-//     group is the group's address XOR a constant, and only the low 5 bits of that need
-//     an instruction;
+//   * R = 3, 4: an XOR of bits 2 .. 4 with bits of the row (pos >> 5), which permutes the
+//     16-byte pieces of each 32-word row. It is linear over XOR, so the address of slot u of
+//     a group is the group's address XOR a constant, and only the low 5 bits of that need an
+//     instruction. The pass with D = 0 (a thread's positions are consecutive) moves 16 bytes
+//     at a time, 8 lanes on distinct pieces of a row's 8;
 //   * R >= 5: one padding word after every 2^R (an address stays base + constant): lanes
 //     32 or 64 positions apart fall on distinct banks, runs of 32 stay together.
 // Every pass, slot and warp of every plan was checked for conflicts on the host.
@@ -76,8 +77,8 @@ struct XMap {
     static constexpr bool SWZ = R == 3 || R == 4;
     __host__ __device__ static constexpr int map(int pos) {
         const int x = pos >> 5;
-        if (R == 3) return pos ^ (x & 7) ^ (((x >> 1) & 3) << 3);
-        if (R == 4) return pos ^ (x & 15) ^ (((x >> 3) & 1) << 4);
+        if (R == 3) return pos ^ ((x & 7) << 2);
+        if (R == 4) return pos ^ (((x & 3) | (((x >> 3) & 1) << 2)) << 2);
         return pos + (pos >> (R >= 6 ? 6 : 5));
     }
     // address of the position g | k from base = map(g), for k with no bit in common with g
@@ -239,15 +240,28 @@ __device__ __forceinline__ void exchange(uint32_t (&x)[NOPS][PL::E], uint32_t* s
     // threads that share a sub-transform of pass PLO (whole warps hold whole groups)
     constexpr bool WARP = PL::G >= 32 && ((PL::N >> PL::S0(PLO)) >> PL::LOGE) <= 32;
     using X = XMap<PL::LOGE>;
+    // consecutive positions: 16-byte accesses
+    constexpr bool VECA = X::SWZ && LA == 0 && NVA == 1, VECB = X::SWZ && LB == 0 && NVB == 1;
     if (sync_before) bar.sync();
 #pragma unroll
     for (int v = 0; v < NVA; v++) {
         const int base = X::map(group_base<PL, PA>(tau, v));  // bits of u << LA are zero in it
+        if constexpr (VECA) {
 #pragma unroll
-        for (int u = 0; u < (1 << RA); u++) {
-            const int a = X::at(base, u << LA);
+            for (int u = 0; u < PL::E; u += 4) {
+                const int a = X::at(base, u);
 #pragma unroll
-            for (int o = 0; o < NOPS; o++) sm[o * PL::SMW + a] = x[o][(v << RA) + u];
+                for (int o = 0; o < NOPS; o++)
+                    *reinterpret_cast<uint4*>(sm + o * PL::SMW + a) =
+                        make_uint4(x[o][u], x[o][u + 1], x[o][u + 2], x[o][u + 3]);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < (1 << RA); u++) {
+                const int a = X::at(base, u << LA);
+#pragma unroll
+                for (int o = 0; o < NOPS; o++) sm[o * PL::SMW + a] = x[o][(v << RA) + u];
+            }
         }
     }
     if constexpr (WARP) __syncwarp();
@@ -255,11 +269,26 @@ __device__ __forceinline__ void exchange(uint32_t (&x)[NOPS][PL::E], uint32_t* s
 #pragma unroll
     for (int v = 0; v < NVB; v++) {
         const int base = X::map(group_base<PL, PB>(tau, v));
+        if constexpr (VECB) {
 #pragma unroll
-        for (int u = 0; u < (1 << RB); u++) {
-            const int a = X::at(base, u << LB);
+            for (int u = 0; u < PL::E; u += 4) {
+                const int a = X::at(base, u);
 #pragma unroll
-            for (int o = 0; o < NOPS; o++) x[o][(v << RB) + u] = sm[o * PL::SMW + a];
+                for (int o = 0; o < NOPS; o++) {
+                    const uint4 q = *reinterpret_cast<const uint4*>(sm + o * PL::SMW + a);
+                    x[o][u] = q.x;
+                    x[o][u + 1] = q.y;
+                    x[o][u + 2] = q.z;
+                    x[o][u + 3] = q.w;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < (1 << RB); u++) {
+                const int a = X::at(base, u << LB);
+#pragma unroll
+                for (int o = 0; o < NOPS; o++) x[o][(v << RB) + u] = sm[o * PL::SMW + a];
+            }
         }
     }
 }
