@@ -21,10 +21,11 @@ void fill_n14_pair(KernelSet& ks) {
     static_assert(PairPlan::G == NttPlan<14, 4>::G, "one thread count for the whole set");
     for (int l = 0; l < 7; l++)
         for (int j = 0; j < 2; j++) ks.mul[l][j] = ks.ks[l][j] = nullptr;
-    fill_pair_l64<0>(ks);
     fill_pair_l64<1>(ks);
     fill_pair_l64<2>(ks);
     fill_pair_l64<3>(ks);
+    fill_pair_l64<4>(ks);
+    fill_pair_l64<5>(ks);
     fill_pair_l64<6>(ks);
     ks.smem_mul = pair_smem_bytes<2>();
     ks.smem_ks[0] = ks.smem_ks[1] = pair_smem_bytes<2>();

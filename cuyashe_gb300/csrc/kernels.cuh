@@ -213,7 +213,7 @@ constexpr int mul_min_blocks() {
     return target < 1 ? 1 : (target > 16 ? 16 : target);
 }
 template <int LOGN, int LOGE>
-constexpr int ks_min_blocks() {
+__host__ __device__ constexpr int ks_min_blocks() {
     constexpr int G = NttPlan<LOGN, LOGE>::G;
     constexpr int target = 1024 / G;
     return target < 1 ? 1 : (target > 16 ? 16 : target);
@@ -328,8 +328,11 @@ __device__ __forceinline__ uint32_t mac_finish(uint64_t T, uint32_t pinv, const 
 // reduced once per coefficient by a Montgomery step; a Shoup product per digit and
 // coefficient took three multiplies and twice the key bytes.
 // ONE: all digits in one pass (kernels of one or two limbs), no sums kept across
-// transforms. Otherwise the 64-bit sums stay in registers with 8 or 16 coefficients
-// per thread; with more (ACC32) each pass's sums are reduced and added to 32-bit ones.
+// transforms. Otherwise the 64-bit sums stay in registers where there is room; with more
+// than 16 coefficients per thread, or 16 in 64 registers (ACC32), each pass's sums are
+// reduced and added to 32-bit ones (three more cycles of the fma-heavy pipe per digit and
+// coefficient, but fewer spills: 64 keyswitches at N = 16384, 380-bit q, 1059 -> 821 us; 512 at N =
+// 8192, 190-bit q, 948 -> 765 us).
 template <int L64, int ND>
 __host__ __device__ constexpr bool ks_one_pass() {
     return (L64 == 1 && ND >= 2) || (L64 == 2 && ND >= 4);
@@ -343,7 +346,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     constexpr int E = PL::E;
     constexpr int LAST = PL::NPASS - 1;
     constexpr bool ONE = ks_one_pass<L64, ND>();
-    constexpr bool ACC32 = !ONE && LOGE > 4;
+    constexpr int REGS = 65536 / (PL::G * (MINB > 0 ? MINB : ks_min_blocks<LOGN, LOGE>()));
+    constexpr bool ACC32 = !ONE && (LOGE > 4 || (LOGE == 4 && REGS <= 64));
     extern __shared__ __align__(16) uint32_t smem[];  // exchange buffer, ND operands x SMW
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
@@ -1291,8 +1295,9 @@ void fill_l64(KernelSet& ks) {
     ks.ks[L64][1] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_HI, MB_KS>;
 }
 
-// SPECIALISE: also instantiate the kernels for 1, 2, 3 and 6 limbs (q of up to
-// 64, 128, 192 and 384 bits); other limb counts use the generic kernels.
+// SPECIALISE: instantiate the kernels for each limb count of SPEC_MASK (all six by default:
+// 512 products of four limbs at N = 4096 @L4@ us against 531 with the generic
+// kernels); limb counts left out use the generic kernels.
 // MB_MUL / MB_KS > 0: blocks per SM the product / keyswitch kernels are
 // compiled for (0: the defaults above).
 // ND_LO: digits per pass of the keyswitch kernel used when four do not fit (2, or 1
@@ -1301,21 +1306,19 @@ void fill_l64(KernelSet& ks) {
 // SPEC_MASK: the limb counts (bit L64) that get specialised kernels when
 // SPECIALISE is set.
 template <int LOGN, int LOGE, bool SPECIALISE, int MB_MUL = 0, int MB_KS = 0, int ND_LO = 2, int ND_HI = 4,
-          unsigned SPEC_MASK = 0x4Eu>
+          unsigned SPEC_MASK = 0x7Eu>
 void fill_kernel_set(KernelSet& ks) {
     using PL = NttPlan<LOGN, LOGE>;
     ks.logn = LOGN;
     ks.loge = LOGE;
     ks.threads = PL::G;
-    fill_l64<LOGN, LOGE, 0, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
-    if constexpr (SPECIALISE && (SPEC_MASK & 2u))
-        fill_l64<LOGN, LOGE, 1, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
-    if constexpr (SPECIALISE && (SPEC_MASK & 4u))
-        fill_l64<LOGN, LOGE, 2, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
-    if constexpr (SPECIALISE && (SPEC_MASK & 8u))
-        fill_l64<LOGN, LOGE, 3, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
-    if constexpr (SPECIALISE && (SPEC_MASK & 64u))
-        fill_l64<LOGN, LOGE, 6, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (!SPECIALISE || SPEC_MASK != 0x7Eu) fill_l64<LOGN, LOGE, 0, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (SPECIALISE && (SPEC_MASK & 2u)) fill_l64<LOGN, LOGE, 1, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (SPECIALISE && (SPEC_MASK & 4u)) fill_l64<LOGN, LOGE, 2, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (SPECIALISE && (SPEC_MASK & 8u)) fill_l64<LOGN, LOGE, 3, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (SPECIALISE && (SPEC_MASK & 16u)) fill_l64<LOGN, LOGE, 4, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (SPECIALISE && (SPEC_MASK & 32u)) fill_l64<LOGN, LOGE, 5, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
+    if constexpr (SPECIALISE && (SPEC_MASK & 64u)) fill_l64<LOGN, LOGE, 6, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (LOGE >= 6) {  // one transform per block (k_ntt1), coalesced row side at N = 4096
         // N = 4096: coalesced row side, the two passes as a loop over one copy of the
         // pass code, 96 registers (10 blocks per SM), measured best in both directions

@@ -80,15 +80,11 @@ int default_variant(int logn, int l64, int op, long long blocks) {
     const bool small = blocks <= sms;
     const bool product = op == TUNE_MUL || op == TUNE_MULC;
     switch (logn) {
-        case 10: return product && l64 == 6 && blocks >= 2 * sms ? 1 : 0;
+        case 10: return product && l64 >= 3 && blocks >= 2 * sms ? 1 : 0;
+        case 11: return product ? 1 : 0;
         case 12: return op == TUNE_KS ? (small ? 2 : 3) : 8;
-        case 13:
-            if (op == TUNE_KS) return l64 == 1 ? 0 : 2;
-            return product && small ? 2 : 0;
-        case 14:
-            if (op == TUNE_NTT) return 0;
-            if (2 * blocks <= sms) return 3;
-            return l64 == 1 ? 0 : 1;
+        case 13: return op == TUNE_KS && l64 > 1 ? 2 : 0;
+        case 14: return op != TUNE_NTT && 2 * blocks <= sms ? 3 : 0;
         default: return 0;
     }
 }
