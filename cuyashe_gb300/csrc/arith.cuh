@@ -77,11 +77,6 @@ struct Mod {
     uint32_t p, p2, np, np2;  // p, 2p, -p, -2p (mod 2^32)
 };
 
-// The same constants computed from p in registers: the compiler folds them
-// (fewer live registers, two more instructions per butterfly), for kernels that
-// are short of registers.
-__device__ __forceinline__ Mod mod_of(uint32_t p) { return Mod{p, 2 * p, 0u - p, 0u - 2 * p}; }
-
 // x * w mod p in [0, 2p), any 32-bit x (Shoup, with -p from m)
 __device__ __forceinline__ uint32_t shoup_m(uint32_t x, uint32_t w, uint32_t ws, const Mod& m) {
     return __umulhi(x, ws) * m.np + x * w;

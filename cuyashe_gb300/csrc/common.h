@@ -111,6 +111,8 @@ struct MixedJob {
     const uint64_t* b;
     uint64_t* c;
     uint32_t* resid;     // [max(k, k2)][N] residues of this job in the batch scratch
+    const void* epi;     // EpiConst of B and of B2 (constants of the epilogues)
+    const void* epi2;
     const uint32_t* evk; // keyswitch key [ell][k2][N] (NTT domain, times 2^32)
     int logn, k, l32, l64;
     int mode;            // EPI_MODQ (product) or EPI_YASHE (tensor rounding)

@@ -45,5 +45,6 @@ struct EpiConstKernel {
     void (*fill)(const BasisDev& h, void* param);
 };
 const EpiConstKernel* epi_const(int l32, int k, int mode);
+const EpiConstKernel* epi_const_any(int l32, int mode);  // for any prime count
 
 }  // namespace cy

@@ -26,11 +26,15 @@ const EpiConstKernel* epi_any1(int l32, int mode);  // 1 .. 5 words
 const EpiConstKernel* epi_any2(int l32, int mode);  // 6 .. 9
 const EpiConstKernel* epi_any3(int l32, int mode);  // 10 .. 12
 
+const EpiConstKernel* epi_const_any(int l32, int mode) {
+    if (l32 < 1 || l32 > L32MAX || mode < 0 || mode > 2) return nullptr;
+    return l32 <= 5 ? epi_any1(l32, mode) : l32 <= 9 ? epi_any2(l32, mode) : epi_any3(l32, mode);
+}
+
 const EpiConstKernel* epi_const(int l32, int k, int mode) {
     for (const EpiEntry& e : kEpiSpecial)
         if (e.l32 == l32 && e.k == k && e.mode == mode) return &e.s;
-    if (l32 < 1 || l32 > L32MAX || k < 1 || k > KMAX || mode < 0 || mode > 2) return nullptr;
-    return l32 <= 5 ? epi_any1(l32, mode) : l32 <= 9 ? epi_any2(l32, mode) : epi_any3(l32, mode);
+    return k >= 1 && k <= KMAX ? epi_const_any(l32, mode) : nullptr;
 }
 
 }  // namespace cy

@@ -974,17 +974,6 @@ __device__ __forceinline__ void epi_coefs(const EpiShared& S, const BasisDev* __
     }
 }
 
-// One coefficient (the mixed-batch kernel's epilogue units).
-template <int L, int MODE>
-__device__ __forceinline__ void epi_coef(const EpiShared& S, const BasisDev* __restrict__ B,
-                                         const uint32_t* __restrict__ r0, size_t stride, uint64_t* __restrict__ dst,
-                                         uint64_t frac_limit = 0) {
-    const uint32_t* const rr[1] = {r0};
-    uint64_t* const dd[1] = {dst};
-    const bool st[1] = {true};
-    epi_coefs<L, MODE, 1>(S, B, rr, stride, dd, st, frac_limit);
-}
-
 // lm: outputs limb-major ([job][limb][N]) instead of [job][N][limb] (modes
 // MODQ and YASHE; the HE multiply's intermediate before its keyswitch)
 template <int L, int MODE>
@@ -1131,21 +1120,17 @@ __device__ __forceinline__ uint64_t barrett_c(const Cols<L>& x, const uint32_t (
 // x in [0, 2m) -> [0, m) with nm = -m
 __device__ __forceinline__ uint32_t red_neg(uint32_t x, uint32_t nm) { return __viaddmin_u32(x, nm, x); }
 
-template <int L, int MODE, int K>
-__global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<L, (K ? K : KMAX)> P,
-                                               const BasisDev* __restrict__ B, const uint32_t* __restrict__ resid,
-                                               void* __restrict__ out, int njobs, unsigned long long frac_limit,
-                                               int lm) {
+// One coefficient: residues r0[i n] of primes i < k, result to out (word j at out[j
+// lstride], or one word for DECRYPT). P: the basis's constants (a kernel parameter, or a
+// copy in shared memory).
+// DEP: called by k_epi_c (dependent launches).
+template <int L, int MODE, int K, bool DEP, class Const>
+__device__ __forceinline__ void epi_c_one(const Const& P, const BasisDev* __restrict__ B,
+                                          const uint32_t* __restrict__ r0, int n, uint64_t* __restrict__ out,
+                                          size_t lstride, unsigned long long frac_limit) {
     constexpr int L64 = (L + 1) / 2;
-    const int logn = P.logn, shift = P.shift;
-    const int n = 1 << logn;
+    const int shift = P.shift;
     const int k = K ? K : P.k;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)njobs << logn) return;
-    const long long job = idx >> logn;
-    const int coef = (int)(idx & (n - 1));
-    const uint32_t* r0 = resid + (size_t)job * k * n + coef;
-    dep_wait(r0);
 
     Cols<L> x;   // sum y_i A0_i
     Cols<2> z;   // YASHE: Z = sum y_i F_i in 32-bit columns
@@ -1219,7 +1204,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
 #pragma unroll
     for (int w = 0; w < L; w++) qn[w] = P.qn[w];
     barrett_c<L>(x, qn, P.mu_lo, P.mu_hi, rm);  // rm = (result mod q) << shift
-    dep_launch();
+    if (DEP) dep_launch();
     if constexpr (MODE == EPI_DECRYPT) {
         Cols<L> c2;
 #pragma unroll
@@ -1229,7 +1214,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
         uint32_t rd[L];
         uint64_t Q = barrett_c<L>(c2, qn, P.mu_lo, P.mu_hi, rd);  // round(t x / q) in [0, t]
         if (Q >= P.t) Q -= P.t;
-        reinterpret_cast<uint64_t*>(out)[idx] = Q;
+        out[0] = Q;
     } else {
         uint64_t o[L64];
 #pragma unroll
@@ -1237,19 +1222,37 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
             auto word = [&](int w) { return w < L ? __funnelshift_r(rm[w], w + 1 < L ? rm[w + 1] : 0u, shift) : 0u; };
             o[j] = (uint64_t)word(2 * j + 1) << 32 | word(2 * j);
         }
-        uint64_t* dst = reinterpret_cast<uint64_t*>(out) + (size_t)job * n * L64;
-        if (lm) {
+        if constexpr (L64 % 2 == 0) {
+            if (lstride == 1) {
+                ulonglong2* d2 = reinterpret_cast<ulonglong2*>(out);
 #pragma unroll
-            for (int j = 0; j < L64; j++) dst[(size_t)j * n + coef] = o[j];
-        } else if constexpr (L64 % 2 == 0) {
-            ulonglong2* d2 = reinterpret_cast<ulonglong2*>(dst + (size_t)coef * L64);
-#pragma unroll
-            for (int j = 0; j < L64 / 2; j++) d2[j] = make_ulonglong2(o[2 * j], o[2 * j + 1]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < L64; j++) dst[(size_t)coef * L64 + j] = o[j];
+                for (int j = 0; j < L64 / 2; j++) d2[j] = make_ulonglong2(o[2 * j], o[2 * j + 1]);
+                return;
+            }
         }
+#pragma unroll
+        for (int j = 0; j < L64; j++) out[j * lstride] = o[j];
     }
+}
+
+template <int L, int MODE, int K>
+__global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<L, (K ? K : KMAX)> P,
+                                               const BasisDev* __restrict__ B, const uint32_t* __restrict__ resid,
+                                               void* __restrict__ out, int njobs, unsigned long long frac_limit,
+                                               int lm) {
+    constexpr int L64 = (L + 1) / 2;
+    const int logn = P.logn;
+    const int n = 1 << logn;
+    const int k = K ? K : P.k;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)njobs << logn) return;
+    const long long job = idx >> logn;
+    const int coef = (int)(idx & (n - 1));
+    const uint32_t* r0 = resid + (size_t)job * k * n + coef;
+    dep_wait(r0);
+    uint64_t* dst = reinterpret_cast<uint64_t*>(out) +
+                    (MODE == EPI_DECRYPT ? (size_t)idx : (size_t)job * n * L64 + (lm ? (size_t)coef : (size_t)coef * L64));
+    epi_c_one<L, MODE, K, true>(P, B, r0, n, dst, lm ? (size_t)n : 1, frac_limit);
 }
 
 // Constants of a basis for k_epi_c (K = 0 or KS = K primes).

@@ -33,6 +33,7 @@ unsigned long long epi_frac_limit();
 int trace_begin(const char* name, int logn, cudaStream_t st);
 void trace_end(int idx, cudaStream_t st);
 
+// (14 primes at most: kMixedPrimes in k_mixed.cu)
 static bool mixable(const cy_ring* r) { return r->logn >= 10 && r->logn <= 13 && r->l32 <= 6; }
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
@@ -44,6 +45,7 @@ constexpr int kEpiUnitCoefs = 2048;
 static MixedJob product_job(const cy_ring* r, const uint64_t* a, const uint64_t* b, uint64_t* c) {
     MixedJob J{};
     J.B = r->mul.d;
+    J.epi = r->mul.d_epi;
     J.a = a;
     J.b = b;
     J.c = c;
@@ -64,6 +66,8 @@ static MixedJob yashe_job(const cy_yashe* y, const uint64_t* c1, const uint64_t*
     MixedJob J{};
     J.B = y->tensor.d;
     J.B2 = relin ? y->relin.d : nullptr;
+    J.epi = y->tensor.d_epi;
+    J.epi2 = relin ? y->relin.d_epi : nullptr;
     J.a = c1;
     J.b = c2;
     J.c = out;
@@ -116,6 +120,16 @@ static std::vector<MixedUnit> build_units(const std::vector<MixedJob>& jobs) {
     units.reserve(a.size() + b.size() + c.size() + d.size());
     for (auto* v : {&a, &b, &c, &d}) units.insert(units.end(), v->begin(), v->end());
     return units;
+}
+
+// The schedule of a list that the autotuner has not chosen one for. Two blocks per SM
+// (schedule 0) do more per second, one (schedule 1) ends a unit sooner, which is what counts
+// while an SM gets few of them: with twelve multiplies of N = 2048, 4096 and 8192 123 us against 70,
+// with 144 (10 transform units per SM) 245 against 232, with 192 (14) 316 against 344.
+static int default_schedule(const std::vector<MixedUnit>& units, int sms) {
+    long long transforms = 0;
+    for (const MixedUnit& u : units) transforms += u.kind == 0 || u.kind == 2;
+    return transforms >= 12ll * sms ? 0 : 1;
 }
 
 // residue words of job j in the batch scratch
@@ -241,9 +255,11 @@ cy_status run_mixed(const std::vector<const cy_polymul_job*>& jobs, cudaStream_t
     uint32_t* d_done = reinterpret_cast<uint32_t*>(S.d_meta + jobs_b + units_b);
     uint32_t* d_ctl = reinterpret_cast<uint32_t*>(S.d_meta + jobs_b + units_b + done_b);
     S.d_ctl = d_ctl;
-    int grid = 1;
-    CY_TRY(persistent_grid(0, dev, nu, &grid));
-    CY_TRY(launch_mixed(0, grid, d_jobs, d_units, nu, d_done, d_ctl, mixed_spin_default(), st));
+    int grid = 1, sms = 0;
+    CY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int sched = default_schedule(units, sms);
+    CY_TRY(persistent_grid(sched, dev, nu, &grid));
+    CY_TRY(launch_mixed(sched, grid, d_jobs, d_units, nu, d_done, d_ctl, mixed_spin_default(), st));
     CY_CUDA(cudaEventRecord(S.last_done, st));
     S.launched = true;
     return CY_OK;
@@ -340,6 +356,9 @@ cy_status cy_mixed_plan_create(const cy_mixed_job* jobs, int njobs, cy_mixed_pla
     P->done_bytes = sizeof(uint32_t) * (4 * (size_t)njobs + 4);
     CY_CUDA(cudaMalloc(&P->d_done, P->done_bytes));
     for (int s = 0; s < mixed_schedules(); s++) CY_TRY(persistent_grid(s, P->device, P->n_units, &P->grid[s]));
+    int sms = 0;
+    CY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, P->device));
+    P->sched = default_schedule(units, sms);
     P->spin = mixed_spin_default();
     *out = P.release();
     return CY_OK;

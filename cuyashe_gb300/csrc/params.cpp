@@ -262,6 +262,7 @@ cy_status basis_constants(BasisDev& h, int* crt_bits, int n, const BigUInt& q, i
 Basis::~Basis() {
     if (d) cudaFree(d);
     if (d_ninv) cudaFree(d_ninv);
+    if (d_epi) cudaFree(d_epi);
 }
 
 cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, const BigUInt& bound, uint32_t t,
@@ -312,6 +313,11 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
     if (!b.epi) return set_error(CY_ERR_INTERNAL, "missing epilogue");
     b.epi_param.assign(b.epi->param_bytes, 0);
     b.epi->fill(b.h, b.epi_param.data());
+    const EpiConstKernel* any = epi_const_any(b.h.l32, b.h.mode);
+    std::vector<unsigned char> blob(any->param_bytes, 0);
+    any->fill(b.h, blob.data());
+    CY_CUDA(cudaMalloc(&b.d_epi, blob.size()));
+    CY_CUDA(cudaMemcpy(b.d_epi, blob.data(), blob.size(), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMalloc(&b.d, sizeof(BasisDev)));
     CY_CUDA(cudaMemcpy(b.d, &b.h, sizeof(BasisDev), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMalloc(&b.d_ninv, sizeof(uint32_t) * ninv.size()));

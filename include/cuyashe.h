@@ -196,9 +196,9 @@ cy_status cy_mixed_plan_launch(cy_mixed_plan *plan, cy_stream_t stream);
  * launch gave up waiting for earlier units of its job (a bounded wait that does
  * not expire while the device makes progress). */
 cy_status cy_mixed_plan_status(cy_mixed_plan *plan, cy_stream_t stream);
-/* Schedules of the mixed kernel: 0 = 8 coefficients per thread in 1024-thread
- * blocks, 1 = 16 per thread in 512-thread blocks. The autotuner runs each on the
- * plan's own buffers (results must agree bit for bit), times it with CUDA
+/* Schedules of the mixed kernel (512-thread blocks, 16 coefficients per thread):
+ * 0 = two blocks per SM, 1 = one with twice the registers. A plan starts with the
+ * one that suits its size. The autotuner runs each on the plan's own buffers (results must agree bit for bit), times it with CUDA
  * events and keeps the fastest; it synchronises. */
 cy_status cy_mixed_plan_set_schedule(cy_mixed_plan *plan, int schedule);
 cy_status cy_mixed_plan_get_schedule(const cy_mixed_plan *plan, int *schedule);
