@@ -272,11 +272,35 @@ static int product_chunk_jobs(const Basis& B, const KernelSet& ks, bool centered
 }
 
 // products of `batch` jobs with basis B: out_j = epilogue(a_j * b_j); `variant`
-// selects the NTT schedule (-1: the tuned one for this device and size)
+// selects the NTT schedule (-1: the tuned one for this device and size). key: the kept
+// transform of a (a_stride = 0), used from two products on (a block takes two) where there is a
+// kernel for it
 static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, long long a_stride,
                              const uint64_t* b, long long b_stride, void* out, long long out_stride, int batch,
-                             Workspace& ws, cudaStream_t st, int variant = -1) {
+                             Workspace& ws, cudaStream_t st, int variant = -1, const uint32_t* key = nullptr) {
     if (batch == 0) return CY_OK;
+    const KeyKernel* kk = key && batch > 1 ? key_kernel(B.h.logn, B.h.l64) : nullptr;
+    if (kk) {
+        const int n = B.h.n, k = B.h.k;
+        const int chunk = wave_chunk(std::min(batch, chunk_jobs(n, k)), kk->func, kk->threads, kk->smem, (k + 1) / 2);
+        const int nchunks = (batch + chunk - 1) / chunk;
+        Lanes L;
+        CY_TRY(L.begin(ws, st, (size_t)chunk * k * n, nchunks));
+        cy_status status = CY_OK;
+        for (int c = 0; c < nchunks && status == CY_OK; c++) {
+            const int j0 = c * chunk;
+            int nj = std::min(chunk, batch - j0);
+            const uint64_t* bj = b + (size_t)j0 * b_stride;
+            uint32_t* resid = L.scratch(c);
+            void* args[] = {(void*)&B.prod, (void*)&key, (void*)&bj, (void*)&b_stride, (void*)&resid, (void*)&nj};
+            status = launch(kk->func, "mul_key", B.h.logn, dim3((nj + 1) / 2, k), dim3(kk->threads), kk->smem,
+                            L.stream(c), args, true);
+            if (status == CY_OK)
+                status = launch_epi(B, resid, (char*)out + (size_t)j0 * out_stride * sizeof(uint64_t), nj, L.stream(c),
+                                    epi_name(B.h.mode));
+        }
+        return L.end(ws, st, status);
+    }
     const int n = B.h.n, k = B.h.k, jobs = std::min(batch, chunk_jobs(n, k));
     const KernelSet& ks = kernel_variant(
         B.h.logn, variant >= 0 ? variant
@@ -441,8 +465,8 @@ cy_status check_aligned_api(const void* a, const void* b, const void* c) { retur
 
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
-                          cudaStream_t st, int variant) {
-    return run_product(B, centered, a, a_stride, b, b_stride, out, out_stride, batch, ws, st, variant);
+                          cudaStream_t st, int variant, const uint32_t* key) {
+    return run_product(B, centered, a, a_stride, b, b_stride, out, out_stride, batch, ws, st, variant, key);
 }
 
 // Jobs per chunk of an HE multiply of `batch` pairs, as run_yashe_mul cuts it
@@ -462,6 +486,22 @@ int yashe_chunk_jobs(const Basis& tensor, const Basis& relin, int ell, bool do_r
 cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* evk, int ell, uint64_t* out, int batch,
                             Workspace& ws, cudaStream_t st, int variant, int chunk_k, int lm) {
     return run_keyswitch(B, c, evk, ell, out, batch, ws, st, variant, chunk_k, lm);
+}
+
+// The transform of the polynomial at d_poly ([N][l64] limbs) for k_mul_key with basis B:
+// *d_key [k][N], allocated on the first call. N < 1024 has no such kernel: null. On the
+// legacy default stream; the caller synchronises.
+cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key) {
+    if (!key_kernel(B.h.logn, B.h.l64)) return CY_OK;
+    long long total = (long long)B.h.k * B.h.n;
+    if (!*d_key) CY_CUDA(cudaMalloc(d_key, sizeof(uint32_t) * total));
+    uint32_t* res = *d_key;
+    CY_TRY(run_crt(B, d_poly, res, nullptr, 1, 0));
+    CY_TRY(run_ntt(B, res, 1, false, 0));
+    const BasisDev* Bd = B.d;
+    int up = 0;
+    void* args[] = {(void*)&Bd, (void*)&res, (void*)&res, (void*)&total, (void*)&up};
+    return launch(evk_mont_kernel(), "key_mont", B.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0, args);
 }
 
 // Evaluation key in the keyswitch basis, NTT domain, in Montgomery form: d_evk
@@ -486,7 +526,8 @@ cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n,
     if (st == CY_OK) {
         const BasisDev* Bd = relin.d;
         long long total = (long long)words;
-        void* args[] = {(void*)&Bd, (void*)&d_res, (void*)&out, (void*)&total};
+        int up = 1;
+        void* args[] = {(void*)&Bd, (void*)&d_res, (void*)&out, (void*)&total, (void*)&up};
         st = launch(evk_mont_kernel(), "evk_mont", relin.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256),
                     0, 0, args);
         if (st == CY_OK && rows) {

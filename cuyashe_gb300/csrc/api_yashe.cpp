@@ -20,7 +20,8 @@ namespace cy {
 cy_status check_aligned_api(const void* a, const void* b, const void* c);
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
-                          cudaStream_t st, int variant = -1);
+                          cudaStream_t st, int variant = -1, const uint32_t* key = nullptr);
+cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key);
 cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
                         const uint64_t* c2, uint64_t* out, int batch, bool do_relin, Workspace& ws, cudaStream_t st,
                         int ks_variant = -1);
@@ -39,6 +40,9 @@ cy_yashe::~cy_yashe() {
     if (d_f) cudaFree(d_f);
     if (d_f2) cudaFree(d_f2);
     if (d_h) cudaFree(d_h);
+    if (d_h_key) cudaFree(d_h_key);
+    if (d_f_key) cudaFree(d_f_key);
+    if (d_f2_key) cudaFree(d_f2_key);
     if (d_cdt) cudaFree(d_cdt);
     if (d_evk) cudaFree(d_evk);
     if (ring) cy_ring_destroy(ring);
@@ -136,6 +140,9 @@ cy_status cy_yashe_set_keys(cy_yashe* y, const uint64_t* h_f, const uint64_t* h_
     CY_CUDA(cudaMemcpy(y->d_f, h_f, poly * sizeof(uint64_t), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMemcpy(y->d_h, h_h, poly * sizeof(uint64_t), cudaMemcpyHostToDevice));
     CY_TRY(cy_polymul(r, y->d_f, y->d_f, y->d_f2, 1, nullptr));
+    CY_TRY(prepare_key(r->mul, y->d_h, &y->d_h_key));
+    CY_TRY(prepare_key(y->dec, y->d_f, &y->d_f_key));
+    CY_TRY(prepare_key(y->dec, y->d_f2, &y->d_f2_key));
     if (y->d_evk) {
         cudaFree(y->d_evk);
         y->d_evk = nullptr;
@@ -176,7 +183,7 @@ cy_status cy_yashe_decrypt(cy_yashe* y, const uint64_t* d_ct, uint64_t* d_m, int
     std::lock_guard<std::mutex> lock(r->mu);
     const long long stride = (long long)r->n * r->l64;
     return run_product_api(y->dec, false, aftermul ? y->d_f2 : y->d_f, 0, d_ct, stride, d_m, r->n, batch,
-                           r->own_ws.ws, (cudaStream_t)stream);
+                           r->own_ws.ws, (cudaStream_t)stream, -1, aftermul ? y->d_f2_key : y->d_f_key);
 }
 
 cy_status cy_yashe_mul_ws(cy_yashe* y, cy_workspace* ws, const uint64_t* d_c1, const uint64_t* d_c2,

@@ -29,6 +29,14 @@ struct KernelSet {
 int variant_count(int logn);
 const KernelSet& kernel_variant(int logn, int v);
 
+// Products with a kept operand (k_mul_key) for N = 2^logn >= 1024 and l64 limbs.
+struct KeyKernel {
+    void* func;
+    int threads;
+    size_t smem;
+};
+const KeyKernel* key_kernel(int logn, int l64);
+
 // Tuned operations (keys of the autotuner's table).
 enum TuneOp { TUNE_MUL = 0, TUNE_MULC = 1, TUNE_KS = 2, TUNE_NTT = 3, TUNE_OPS = 4 };
 

@@ -164,6 +164,10 @@ struct cy_yashe {
     uint64_t* d_f2 = nullptr;
     uint64_t* d_h = nullptr;    // public key (GPU encryption)
     uint32_t* d_evk = nullptr;  // [ell][k'][N] NTT-domain evaluation key times 2^32
+    // transforms of h, f and f^2 for products with a batch (k_mul_key; null for N < 1024)
+    uint32_t* d_h_key = nullptr;
+    uint32_t* d_f_key = nullptr;
+    uint32_t* d_f2_key = nullptr;
     uint64_t* d_cdt = nullptr;  // discrete Gaussian thresholds (GPU sampling)
     int n_cdt = 0;
     ~cy_yashe();

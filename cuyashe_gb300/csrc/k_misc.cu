@@ -121,14 +121,20 @@ __global__ void k_crt(const BasisDev* __restrict__ B, const uint64_t* __restrict
     }
 }
 
-// Montgomery form of NTT-domain values: out[j] = v 2^32 mod p_i for the residue
-// vectors of a [ell][k][N] array.
+// NTT-domain values times 2^32 (up: keyswitch keys) or 2^-32 (kept operands of products):
+// out[j] = v 2^(+-32) mod p_i for the residue vectors of a [ell][k][N] array.
 __global__ void k_evk_mont(const BasisDev* __restrict__ B, const uint32_t* __restrict__ v, uint32_t* __restrict__ out,
-                           long long total) {
+                           long long total, int up) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int prime = (int)((idx >> B->logn) % B->k);
-    out[idx] = (uint32_t)(((uint64_t)v[idx] << 32) % B->p[prime]);
+    const uint32_t p = B->p[prime];
+    if (up) {
+        out[idx] = (uint32_t)(((uint64_t)v[idx] << 32) % p);
+    } else {  // v 2^-32 = -(m p) / 2^32 with m = v p^-1 mod 2^32
+        const uint32_t h = __umulhi(v[idx] * B->pinv[prime], p);
+        out[idx] = h ? p - h : 0u;
+    }
 }
 
 // The copy of an NTT-domain evaluation key [ell][k][ROWS_N] laid out by lane for
