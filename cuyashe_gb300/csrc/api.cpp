@@ -409,19 +409,19 @@ static cy_status run_ntt(const Basis& B, uint32_t* res, int batch, bool inverse,
         int* err = nullptr;
         CY_TRY(intt_tma_prepare(res, rows, B.h.k, batch, &map, &grid, &err));
         uint32_t spin = ntt_tma_spin_limit(), extra = ntt_tma_extra_tx();
-        void* args[] = {(void*)&B.prod, (void*)&map, (void*)&res, (void*)&ninv, (void*)&batch, (void*)&err, (void*)&spin,
+        void* args[] = {(void*)&B.ntt, (void*)&map, (void*)&res, (void*)&ninv, (void*)&batch, (void*)&err, (void*)&spin,
                         (void*)&extra};
         return launch(intt_tma_kernel(), "ntt_inv", B.h.logn, grid, dim3(64), intt_tma_smem(), st, args);
     }
     if (ks.ntt_jobs_per_block == 1) {  // k_ntt1: grid (jobs, primes)
-        void* args[] = {(void*)&B.prod, (void*)&res, (void*)&ninv, (void*)&batch};
+        void* args[] = {(void*)&B.ntt, (void*)&res, (void*)&ninv, (void*)&batch};
         return launch(ks.ntt[inverse ? 1 : 0], inverse ? "ntt_inv" : "ntt_fwd", B.h.logn, dim3(batch, B.h.k),
                       dim3(ks.threads), ks.smem_ntt, st, args);
     }
     for (int j0 = 0; j0 < batch; j0 += 2 * 65535) {  // two jobs per block
         int nj = std::min(2 * 65535, batch - j0);
         uint32_t* rj = res + (size_t)j0 * B.h.k * B.h.n;
-        void* args[] = {(void*)&B.prod, (void*)&rj, (void*)&ninv, (void*)&nj};
+        void* args[] = {(void*)&B.ntt, (void*)&rj, (void*)&ninv, (void*)&nj};
         CY_TRY(launch(ks.ntt[inverse ? 1 : 0], inverse ? "ntt_inv" : "ntt_fwd", B.h.logn, dim3(B.h.k, (nj + 1) / 2),
                       dim3(ks.threads), ks.smem_ntt, st, args));
     }

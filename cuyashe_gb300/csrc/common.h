@@ -101,6 +101,18 @@ struct ProdParams {
     const uint2* ipsi_r;
 };
 
+// The same for the standalone transforms (700 bytes instead of 3 KB to copy per launch).
+struct NttParams {
+    struct {
+        uint32_t p, p2, np, np2;
+    } pr[KMAX];
+    int k;
+    const uint2* psi;
+    const uint2* ipsi;
+    const uint2* psi_r;
+    const uint2* ipsi_r;
+};
+
 // One job of a mixed batch (different N and q per job) for the persistent
 // kernel k_mixed: a polynomial product (mode MODQ, no keyswitch) or a YASHE
 // multiply (tensor with the rounding epilogue, then optionally the keyswitch).

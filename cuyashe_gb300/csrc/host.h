@@ -59,7 +59,8 @@ const std::vector<uint32_t>& table_primes();  // host-only, no CUDA
 struct Basis {
     BasisDev h{};
     BasisDev* d = nullptr;
-    ProdParams prod{};  // first parameter of the product, keyswitch and transform kernels
+    ProdParams prod{};  // first parameter of the product and keyswitch kernels
+    NttParams ntt{};    // and of the standalone transforms
     uint32_t* d_ninv = nullptr;  // [k][4]: N^-1 mod p_i, N^-1 psi_i^-(NMAX/2), each with its Shoup companion
     int crt_bits = 0;
     const EpiConstKernel* epi = nullptr;   // epilogue of this basis

@@ -130,7 +130,7 @@ __device__ __forceinline__ void write_row(uint8_t* t, int r, const uint32_t (&x)
 // up waiting for a tile (spin_limit polls). `extra_tx` > 0 only in the test of
 // that path (the tile's barrier then waits for bytes that never come).
 __global__ void __launch_bounds__(64, 10)
-    k_intt_tma(const __grid_constant__ ProdParams M, const __grid_constant__ CUtensorMap map, uint32_t* __restrict__ res,
+    k_intt_tma(const __grid_constant__ NttParams M, const __grid_constant__ CUtensorMap map, uint32_t* __restrict__ res,
                const uint32_t* __restrict__ ninv, int njobs, int* __restrict__ err, uint32_t spin_limit,
                uint32_t extra_tx) {
     extern __shared__ uint8_t smem_raw[];

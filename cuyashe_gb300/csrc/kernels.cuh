@@ -44,7 +44,10 @@ __device__ __forceinline__ Mod load_mod(const BasisDev* __restrict__ B, int i) {
 // The tables of prime i (ProdParams).
 __device__ __forceinline__ const uint2* table_of(const uint2* base, int i) { return base + (size_t)i * NMAX; }
 __device__ __forceinline__ const uint2* rows_of(const uint2* base, int i) { return base + (size_t)i * ROWS_WORDS; }
-__device__ __forceinline__ Mod load_mod(const PrimeParam& q) { return Mod{q.p, q.p2, q.np, q.np2}; }
+template <class Param>  // PrimeParam, or a prime of NttParams
+__device__ __forceinline__ Mod load_mod(const Param& q) {
+    return Mod{q.p, q.p2, q.np, q.np2};
+}
 
 // a + b reduced from [0, 4p) to [0, 2p) (a, b in [0, 2p)): one add, one add-then-min
 __device__ __forceinline__ uint32_t mac_red(uint32_t a, uint32_t b, const Mod& m) {
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, MINB)
 // --------------------------------------------------------------------------
 template <int LOGN, int LOGE, bool INV>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, LOGE>()))
-    k_ntt(const __grid_constant__ ProdParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
+    k_ntt(const __grid_constant__ NttParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
           int njobs) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
@@ -553,8 +556,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
     const int job0 = 2 * blockIdx.y;
     const bool two = job0 + 1 < njobs;
     const int k = M.k;
-    const PrimeParam& Q = M.pr[prime];
-    const Mod m = load_mod(Q);
+    const Mod m = load_mod(M.pr[prime]);
     const uint32_t p = m.p;
     uint32_t* v[2] = {res + ((size_t)job0 * k + prime) * PL::N, res + ((size_t)(two ? job0 + 1 : job0) * k + prime) * PL::N};
     uint32_t x[2][E];
@@ -629,7 +631,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
 // code (ntt_core.cuh, ntt64_forward / ntt64_inverse).
 template <int LOGN, int LOGE, bool INV, int MINB = 0, bool COAL = false, int TPB = 1, bool LOOP = false>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB : 1))
-    k_ntt1(const __grid_constant__ ProdParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
+    k_ntt1(const __grid_constant__ NttParams M, uint32_t* __restrict__ res, const uint32_t* __restrict__ ninv,
            int njobs) {
     using PL = NttPlan<LOGN, LOGE>;
     constexpr int E = PL::E;
@@ -644,8 +646,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
     const int job = store ? job_raw : njobs - 1;
     const int prime = blockIdx.y;
     const int k = M.k;
-    const PrimeParam& Q = M.pr[prime];
-    const Mod m = load_mod(Q);
+    const Mod m = load_mod(M.pr[prime]);
     const uint32_t p = m.p;
     uint32_t* v = res + ((size_t)job * k + prime) * PL::N;
     uint32_t x[1][E];

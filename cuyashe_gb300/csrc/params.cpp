@@ -301,6 +301,7 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
         q.pinv = b.h.pinv[i];
         q.cadd = b.h.p2[i] - b.h.qmont[i];
         std::copy(b.h.crt[i], b.h.crt[i] + L32MAX, q.crt);
+        b.ntt.pr[i] = {q.p, q.p2, q.np, q.np2};
     }
     std::copy(b.h.qhalf, b.h.qhalf + L32MAX, b.prod.qhalf);
     b.prod.k = b.h.k;
@@ -309,6 +310,11 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
     b.prod.ipsi = b.h.ipsi[0];
     b.prod.psi_r = b.h.psi_r[0];
     b.prod.ipsi_r = b.h.ipsi_r[0];
+    b.ntt.k = b.h.k;
+    b.ntt.psi = b.prod.psi;
+    b.ntt.ipsi = b.prod.ipsi;
+    b.ntt.psi_r = b.prod.psi_r;
+    b.ntt.ipsi_r = b.prod.ipsi_r;
     b.epi = epi_const(b.h.l32, b.h.k, b.h.mode);
     if (!b.epi) return set_error(CY_ERR_INTERNAL, "missing epilogue");
     b.epi_param.assign(b.epi->param_bytes, 0);

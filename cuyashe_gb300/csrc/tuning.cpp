@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -45,15 +46,14 @@ static std::map<std::tuple<int, int, int, int>, int> g_choice;  // (device, logn
 
 // SMs of the current device (the GB300's 152 if it cannot be queried).
 static int sm_count() {
-    static std::mutex mu;
-    static std::map<int, int> known;
+    static std::atomic<int> known[64];
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 152;
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = known.find(dev);
-    if (it != known.end()) return it->second;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+    sms = known[dev].load(std::memory_order_relaxed);
+    if (sms > 0) return sms;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 152;
-    return known[dev] = sms;
+    known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
 }
 
 // The schedule of a call that the autotuner has not chosen one for: `blocks` transforms'
