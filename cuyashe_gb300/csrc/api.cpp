@@ -495,17 +495,21 @@ cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key) 
     if (!key_kernel(B.h.logn, B.h.l64)) return CY_OK;
     long long total = (long long)B.h.k * B.h.n;
     if (!*d_key) CY_CUDA(cudaMalloc(d_key, sizeof(uint32_t) * total));
-    uint32_t* res = *d_key;
-    CY_TRY(run_crt(B, d_poly, res, nullptr, 1, 0));
-    CY_TRY(run_ntt(B, res, 1, false, 0));
+    uint32_t* res = nullptr;
+    CY_CUDA(cudaMalloc(&res, sizeof(uint32_t) * total));
+    cy_status st = run_crt(B, d_poly, res, nullptr, 1, 0);
+    if (st == CY_OK) st = run_ntt(B, res, 1, false, 0);
     const BasisDev* Bd = B.d;
     int up = 0;
-    void* args[] = {(void*)&Bd, (void*)&res, (void*)&res, (void*)&total, (void*)&up};
-    return launch(evk_mont_kernel(), "key_mont", B.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0, args);
+    void* args[] = {(void*)&Bd, (void*)&res, (void*)d_key, (void*)&total, (void*)&up};
+    if (st == CY_OK)
+        st = launch(evk_mont_kernel(), "key_mont", B.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0, args);
+    cudaFree(res);  // waits for the kernels
+    return st;
 }
 
 // Evaluation key in the keyswitch basis, NTT domain, in Montgomery form: d_evk
-// [ell][k][N] of value 2^32 mod p (the keyswitch sums products with the digits in 64
+// [ell][k][N] (key_index) of value 2^32 mod p (the keyswitch sums products with the digits in 64
 // bits and reduces once); at N = ROWS_N a second copy laid out by lane follows it
 // (the 64-coefficient keyswitch reads that one). Synchronous.
 cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint32_t** d_evk) {

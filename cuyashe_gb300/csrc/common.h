@@ -19,6 +19,17 @@ constexpr int ROWS_N = 1 << ROWS_LOGN;
 constexpr int ROWS_G = ROWS_N >> 6;       // threads per transform
 constexpr int ROWS_WORDS = 63 * ROWS_G;   // sum over the six stages of 2^l * G
 
+// Index of position `pos` in a kept transform of length n (evaluation keys, kept operands):
+// the 16-byte pieces of 16 consecutive positions are n / 4 words apart, so that threads with
+// 16 (or 8) consecutive positions each load consecutive pieces (a 16-byte load of a warp that
+// steps 64 bytes per lane takes four times the L1 cycles).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int key_index(int pos, int n) {
+    return n < 64 ? pos : ((pos >> 2) & 3) * (n >> 2) + (pos >> 4) * 4 + (pos & 3);
+}
+
 // What the epilogue of a product kernel computes from the recombined integer X
 // (|X| < M/4, M the basis product):
 //   MODQ     X mod q                                  -> [N][L] limbs

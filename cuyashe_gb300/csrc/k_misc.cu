@@ -121,20 +121,23 @@ __global__ void k_crt(const BasisDev* __restrict__ B, const uint64_t* __restrict
     }
 }
 
-// NTT-domain values times 2^32 (up: keyswitch keys) or 2^-32 (kept operands of products):
-// out[j] = v 2^(+-32) mod p_i for the residue vectors of a [ell][k][N] array.
+// NTT-domain values times 2^32 (up: keyswitch keys) or 2^-32 (kept operands of products), in
+// the order of key_index: for the residue vectors of a [ell][k][N] array.
 __global__ void k_evk_mont(const BasisDev* __restrict__ B, const uint32_t* __restrict__ v, uint32_t* __restrict__ out,
                            long long total, int up) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
+    const int n = 1 << B->logn, pos = (int)(idx & (n - 1));
     const int prime = (int)((idx >> B->logn) % B->k);
     const uint32_t p = B->p[prime];
+    uint32_t r;
     if (up) {
-        out[idx] = (uint32_t)(((uint64_t)v[idx] << 32) % p);
+        r = (uint32_t)(((uint64_t)v[idx] << 32) % p);
     } else {  // v 2^-32 = -(m p) / 2^32 with m = v p^-1 mod 2^32
         const uint32_t h = __umulhi(v[idx] * B->pinv[prime], p);
-        out[idx] = h ? p - h : 0u;
+        r = h ? p - h : 0u;
     }
+    out[idx - pos + key_index(pos, n)] = r;
 }
 
 // The copy of an NTT-domain evaluation key [ell][k][ROWS_N] laid out by lane for
@@ -146,7 +149,7 @@ __global__ void k_evk_rows(const uint32_t* __restrict__ in, uint32_t* __restrict
     const long long row = idx / ROWS_N;
     const int pos = (int)(idx % ROWS_N);
     const int tau = pos >> 6, u = pos & 63;
-    out[row * ROWS_N + (u >> 2) * 4 * ROWS_G + 4 * tau + (u & 3)] = in[idx];
+    out[row * ROWS_N + (u >> 2) * 4 * ROWS_G + 4 * tau + (u & 3)] = in[row * ROWS_N + key_index(pos, ROWS_N)];
 }
 
 // Elementwise c = a +/- b mod q over [count][l64] limbs (inputs in [0, q)).

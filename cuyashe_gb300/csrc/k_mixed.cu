@@ -143,7 +143,7 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
             const int d = d0 + o;
             if (d < ell) {
                 uint32_t v[E];
-                load_evk<PL>(J.evk + ((size_t)d * k2 + prime) * PL::N, tau, v);
+                load_evk<PL::N, E>(J.evk + ((size_t)d * k2 + prime) * PL::N, last_pos<PL>(tau), v);
 #pragma unroll
                 for (int e = 0; e < E; e++) T[e] += (uint64_t)x[o][e] * v[e];
             }

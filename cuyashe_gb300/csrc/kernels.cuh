@@ -295,18 +295,15 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
 // --------------------------------------------------------------------------
 // k_keyswitch: one block per (job, prime). Digits are the 32-bit words of the
 // coefficients of c in [0, q) (w = 2^32), processed ND at a time.
-// evk: [ell][k][N] values times 2^32 mod p in the forward-NTT output order.
+// evk: [ell][k][N] values times 2^32 mod p in the forward-NTT output order (key_index).
 // --------------------------------------------------------------------------
-// The E key values of thread tau after the last forward pass (contiguous positions).
-template <class PL>
-__device__ __forceinline__ void load_evk(const uint32_t* __restrict__ g, int tau, uint32_t (&v)[PL::E]) {
-    constexpr int LAST = PL::NPASS - 1, E = PL::E;
-    static_assert(PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE, "contiguous last-pass positions");
-    const uint32_t* s = g + group_base<PL, LAST>(tau, 0);
+// The E key values (key_index order in a row of N) of the consecutive positions pos0 ...
+template <int N, int E>
+__device__ __forceinline__ void load_evk(const uint32_t* __restrict__ row, int pos0, uint32_t (&v)[E]) {
     if constexpr (E % 4 == 0) {
 #pragma unroll
         for (int h = 0; h < E / 4; h++) {
-            const uint4 W = __ldg(reinterpret_cast<const uint4*>(s) + h);
+            const uint4 W = __ldg(reinterpret_cast<const uint4*>(row + key_index(pos0 + 4 * h, N)));
             v[4 * h] = W.x;
             v[4 * h + 1] = W.y;
             v[4 * h + 2] = W.z;
@@ -314,8 +311,15 @@ __device__ __forceinline__ void load_evk(const uint32_t* __restrict__ g, int tau
         }
     } else {
 #pragma unroll
-        for (int e = 0; e < E; e++) v[e] = __ldg(s + e);
+        for (int e = 0; e < E; e++) v[e] = __ldg(row + key_index(pos0 + e, N));
     }
+}
+// first of thread tau's consecutive positions after the last forward pass
+template <class PL>
+__device__ __forceinline__ int last_pos(int tau) {
+    constexpr int LAST = PL::NPASS - 1;
+    static_assert(PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE, "contiguous last-pass positions");
+    return group_base<PL, LAST>(tau, 0);
 }
 
 // Sum of up to four products of a digit in [0, 4p) and a key value below p (T < 4p 2^32)
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
                 }
                 if (d < ell) {
                     uint32_t v[E];
-                    load_evk<PL>(evk + ((size_t)d * k + prime) * PL::N, tau, v);
+                    load_evk<PL::N, E>(evk + ((size_t)d * k + prime) * PL::N, last_pos<PL>(tau), v);
 #pragma unroll
                     for (int e = 0; e < E; e++) T[e] += (uint64_t)x[o][e] * v[e];
                 }
@@ -479,8 +483,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
 
 // --------------------------------------------------------------------------
 // k_mul_key: products of a batch with one polynomial whose transform is kept (a scheme's
-// keys: encryption's h, decryption's f and f^2). key: [k][N] transforms times 2^-32, in the
-// forward-NTT output order. One split, one forward and one inverse transform per product and
+// keys: encryption's h, decryption's f and f^2). key: [k][N] transforms times 2^-32
+// (key_index). One split, one forward and one inverse transform per product and
 // prime instead of two, two and one; a block takes two jobs (shared twiddles and key values;
 // with an odd count the last block repeats its job and stores it once).
 // 512 products with a kept operand (256 encryptions and their decryptions) at N = 4096, 127-bit
@@ -520,7 +524,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, MINB)
     }
     ntt_forward<PL, 2>(x, table_of(M.psi, prime), c.m, tau, smem);
     uint32_t v[E];
-    load_evk<PL>(key + (size_t)prime * PL::N, tau, v);
+    load_evk<PL::N, E>(key + (size_t)prime * PL::N, last_pos<PL>(tau), v);
 #pragma unroll
     for (int o = 0; o < 2; o++)
 #pragma unroll
@@ -560,18 +564,29 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
     const uint32_t p = m.p;
     uint32_t* v[2] = {res + ((size_t)job0 * k + prime) * PL::N, res + ((size_t)(two ? job0 + 1 : job0) * k + prime) * PL::N};
     uint32_t x[2][E];
-    // after the last pass a thread's E positions are contiguous (16-byte accesses)
+    // after the last pass a thread's E positions are contiguous (16-byte accesses); with
+    // whole warps and 16-byte pieces in the buffer they change places inside the warp first, so that
+    // a warp's access covers 512 consecutive bytes (2048 x 9 forward transforms of length 4096: 162
+    // -> 140 us; 512 x 14 of length 8192: 161 -> 146 forward, 159 -> 151 us inverse)
     constexpr bool VEC = PL::LOGD(LAST) == 0 && PL::R(LAST) == PL::LOGE && E % 4 == 0;
+    constexpr bool COAL = VEC && lanes_ok<PL>();
     if (!INV) {
 #pragma unroll
         for (int o = 0; o < 2; o++)
 #pragma unroll
             for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, 0>(tau, e)];
         ntt_forward<PL, 2>(x, table_of(M.psi, prime), m, tau, smem);
+        if constexpr (COAL) rows_to_lanes<PL, 2>(x, smem, tau);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
             if (o == 1 && !two) break;
-            if constexpr (VEC) {
+            if constexpr (COAL) {
+#pragma unroll
+                for (int e = 0; e < E; e += 4)
+                    *reinterpret_cast<uint4*>(v[o] + lane_pos<PL>(tau, e)) =
+                        make_uint4(red(red_2p(x[o][e], m), p), red(red_2p(x[o][e + 1], m), p),
+                                   red(red_2p(x[o][e + 2], m), p), red(red_2p(x[o][e + 3], m), p));
+            } else if constexpr (VEC) {
                 uint4* d4 = reinterpret_cast<uint4*>(v[o] + group_base<PL, LAST>(tau, 0));
 #pragma unroll
                 for (int h = 0; h < E / 4; h++)
@@ -586,7 +601,16 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
         const uint32_t w = ninv[4 * prime], ws = ninv[4 * prime + 1];
 #pragma unroll
         for (int o = 0; o < 2; o++) {
-            if constexpr (VEC) {
+            if constexpr (COAL) {
+#pragma unroll
+                for (int e = 0; e < E; e += 4) {
+                    const uint4 q4 = *reinterpret_cast<const uint4*>(v[o] + lane_pos<PL>(tau, e));
+                    x[o][e] = q4.x;
+                    x[o][e + 1] = q4.y;
+                    x[o][e + 2] = q4.z;
+                    x[o][e + 3] = q4.w;
+                }
+            } else if constexpr (VEC) {
                 const uint4* s4 = reinterpret_cast<const uint4*>(v[o] + group_base<PL, LAST>(tau, 0));
 #pragma unroll
                 for (int h = 0; h < E / 4; h++) {
@@ -601,6 +625,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
                 for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, LAST>(tau, e)];
             }
         }
+        if constexpr (COAL) lanes_to_rows<PL, 2>(x, smem, tau);
         ntt_inverse<PL, 2>(x, table_of(M.ipsi, prime), m, tau, smem);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
@@ -1359,7 +1384,7 @@ void fill_l64(KernelSet& ks) {
 }
 
 // SPECIALISE: instantiate the kernels for each limb count of SPEC_MASK (all six by default:
-// 512 products of four limbs at N = 4096 @L4@ us against 531 with the generic
+// 512 products of four limbs at N = 4096 376 us against 531 with the generic
 // kernels); limb counts left out use the generic kernels.
 // MB_MUL / MB_KS > 0: blocks per SM the product / keyswitch kernels are
 // compiled for (0: the defaults above).

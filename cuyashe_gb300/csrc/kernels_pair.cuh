@@ -203,7 +203,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
             }
             if (d < ell) {
                 uint32_t v[E];
-                load_evk<PL>(evk + ((size_t)d * k + prime) * (2 * kPairHalf) + h * kPairHalf, tau, v);
+                load_evk<2 * kPairHalf, E>(evk + ((size_t)d * k + prime) * (2 * kPairHalf),
+                                            (int)h * kPairHalf + last_pos<PL>(tau), v);
 #pragma unroll
                 for (int e = 0; e < E; e++) T[e] += (uint64_t)x[o][e] * v[e];
             }

@@ -293,6 +293,69 @@ __device__ __forceinline__ void exchange(uint32_t (&x)[NOPS][PL::E], uint32_t* s
     }
 }
 
+// The last pass's layout (thread tau has the E positions from E tau on) against one in which
+// four consecutive registers of a warp's lanes are 128 consecutive positions: register e (a
+// multiple of 4) of lane L is position E 32 (tau / 32) + 32 e + 4 L, so that a warp's 16-byte global
+// accesses are consecutive. Inside a warp's own words of `sm`; rows_to_lanes follows a forward
+// transform, lanes_to_rows precedes an inverse one.
+template <class PL>
+__host__ __device__ constexpr bool lanes_ok() {
+    return XMap<PL::LOGE>::SWZ && PL::G >= 32;
+}
+template <class PL>
+__device__ __forceinline__ int lane_pos(int tau, int e) {
+    return ((tau >> 5) << (5 + PL::LOGE)) + 32 * e + 4 * (tau & 31);
+}
+template <class PL, int NOPS>
+__device__ __forceinline__ void rows_to_lanes(uint32_t (&x)[NOPS][PL::E], uint32_t* sm, int tau) {
+    using X = XMap<PL::LOGE>;
+    const int base = X::map(tau << PL::LOGE);
+#pragma unroll
+    for (int u = 0; u < PL::E; u += 4)
+#pragma unroll
+        for (int o = 0; o < NOPS; o++)
+            *reinterpret_cast<uint4*>(sm + o * PL::SMW + X::at(base, u)) =
+                make_uint4(x[o][u], x[o][u + 1], x[o][u + 2], x[o][u + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < PL::E; e += 4) {
+        const int a = X::map(lane_pos<PL>(tau, e));
+#pragma unroll
+        for (int o = 0; o < NOPS; o++) {
+            const uint4 q = *reinterpret_cast<const uint4*>(sm + o * PL::SMW + a);
+            x[o][e] = q.x;
+            x[o][e + 1] = q.y;
+            x[o][e + 2] = q.z;
+            x[o][e + 3] = q.w;
+        }
+    }
+}
+template <class PL, int NOPS>
+__device__ __forceinline__ void lanes_to_rows(uint32_t (&x)[NOPS][PL::E], uint32_t* sm, int tau) {
+    using X = XMap<PL::LOGE>;
+#pragma unroll
+    for (int e = 0; e < PL::E; e += 4) {
+        const int a = X::map(lane_pos<PL>(tau, e));
+#pragma unroll
+        for (int o = 0; o < NOPS; o++)
+            *reinterpret_cast<uint4*>(sm + o * PL::SMW + a) = make_uint4(x[o][e], x[o][e + 1], x[o][e + 2], x[o][e + 3]);
+    }
+    __syncwarp();
+    const int base = X::map(tau << PL::LOGE);
+#pragma unroll
+    for (int u = 0; u < PL::E; u += 4) {
+        const int a = X::at(base, u);
+#pragma unroll
+        for (int o = 0; o < NOPS; o++) {
+            const uint4 q = *reinterpret_cast<const uint4*>(sm + o * PL::SMW + a);
+            x[o][u] = q.x;
+            x[o][u + 1] = q.y;
+            x[o][u + 2] = q.z;
+            x[o][u + 3] = q.w;
+        }
+    }
+}
+
 // Forward passes PASS .. NPASS-1 (sync_before: as in exchange, for the first one).
 template <class PL, int PASS, int NOPS, class Sync = CtaSync>
 struct FwdFrom {
