@@ -152,6 +152,25 @@ __global__ void k_evk_rows(const uint32_t* __restrict__ in, uint32_t* __restrict
     out[row * ROWS_N + (u >> 2) * 4 * ROWS_G + 4 * tau + (u & 3)] = in[row * ROWS_N + key_index(pos, ROWS_N)];
 }
 
+// A lane-ordered twiddle table (rows_index) of length 2^logn and 2^loge coefficients per
+// thread: entry (l, h, tau) = tw[2^(logn - loge + l) + tau 2^l + h].
+__global__ void k_lane_table(const uint2* __restrict__ tw, uint2* __restrict__ out, int logn, int loge, int primes) {
+    const int G = 1 << (logn - loge), words = (1 << logn) - G;
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)primes * words) return;
+    const int prime = (int)(idx / words), src = (int)(idx % words);  // src: stage-major, natural order in a stage
+    const int l = 31 - __clz(src / G + 1);
+    const int j = src - G * ((1 << l) - 1), tau = j >> l, h = j & ((1 << l) - 1);
+    out[(long long)prime * words + rows_index(G, l, h, tau)] = tw[(size_t)prime * NMAX + ((size_t)G << l) + j];
+}
+
+cy_status build_lane_table(const uint2* tw, uint2* out, int logn, int loge, int primes) {
+    const long long total = (long long)primes * ((1 << logn) - (1 << (logn - loge)));
+    k_lane_table<<<(unsigned)((total + 255) / 256), 256>>>(tw, out, logn, loge, primes);
+    CY_CUDA(cudaGetLastError());
+    return CY_OK;
+}
+
 // Elementwise c = a +/- b mod q over [count][l64] limbs (inputs in [0, q)).
 template <int L64, bool SUB>
 __global__ void k_addsub(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b, uint64_t* __restrict__ c,

@@ -79,11 +79,11 @@ __device__ __forceinline__ void mixed_ntt_unit(const MixedJob& J, const MixedUni
     if (J.l64 == 1) mixed_split<PL, 1>(x, J, B, prime, tau, centered, c);
     else if (J.l64 == 2) mixed_split<PL, 2>(x, J, B, prime, tau, centered, c);
     else mixed_split<PL, 3>(x, J, B, prime, tau, centered, c);
-    ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, false, bar);
+    ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, false, bar, 1, lanes_of<PL>(B->tw.psi_lanes, prime));
     uint32_t z[1][E];
 #pragma unroll
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
-    ntt_inverse<PL, 1, GroupSync>(z, B->ipsi[prime], m, tau, sm, bar);
+    ntt_inverse<PL, 1, GroupSync>(z, B->ipsi[prime], m, tau, sm, bar, 1, lanes_of<PL>(B->tw.ipsi_lanes, prime));
     uint32_t* out = J.resid + (size_t)prime * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = z[0][e];
@@ -135,7 +135,8 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
                 x[o][e] = __viaddmin_u32(w, m.np2, w);  // digit < 2^32 < 6p -> [0, 4p)
             }
         }
-        ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, d0 > 0, bar);
+        ntt_forward<PL, 2, GroupSync>(x, B->psi[prime], m, tau, sm, d0 > 0, bar, 1,
+                                      lanes_of<PL>(B->tw.psi_lanes, prime));
 #pragma unroll
         for (int e = 0; e < E; e++) T[e] = ACC32 ? 0 : lazy_high(T[e], m);
 #pragma unroll
@@ -157,7 +158,7 @@ __device__ __forceinline__ void mixed_ks_unit(const MixedJob& J, const MixedUnit
 #pragma unroll
         for (int e = 0; e < E; e++) acc[0][e] = mac_finish<true>(T[e], pinv, m);
     }
-    ntt_inverse<PL, 1, GroupSync>(acc, B->ipsi[prime], m, tau, sm, bar);
+    ntt_inverse<PL, 1, GroupSync>(acc, B->ipsi[prime], m, tau, sm, bar, 1, lanes_of<PL>(B->tw.ipsi_lanes, prime));
     uint32_t* out = J.resid + (size_t)prime * PL::N;
 #pragma unroll
     for (int e = 0; e < E; e++) out[slot_pos<PL, 0>(tau, e)] = acc[0][e];

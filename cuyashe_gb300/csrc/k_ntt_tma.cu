@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(64, 10)
     const int prime = blockIdx.y;
     const int k = M.k;
     const Mod m = load_mod(M.pr[prime]);
-    const uint2* __restrict__ tw = table_of(M.ipsi, prime);
-    const uint2* __restrict__ twr = rows_of(M.ipsi_r, prime);
+    const uint2* __restrict__ tw = table_of(M.tw.ipsi, prime);
+    const uint2* __restrict__ twr = lanes_of<NttPlan<12, 6>>(M.tw.ipsi_lanes, prime);
     const int step = gridDim.x;
     int job = blockIdx.x;
     if (tau == 0) {

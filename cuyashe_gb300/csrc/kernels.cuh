@@ -41,9 +41,13 @@ __device__ __forceinline__ Mod load_mod(const BasisDev* __restrict__ B, int i) {
     return m;
 }
 
-// The tables of prime i (ProdParams).
+// The tables of prime i.
 __device__ __forceinline__ const uint2* table_of(const uint2* base, int i) { return base + (size_t)i * NMAX; }
-__device__ __forceinline__ const uint2* rows_of(const uint2* base, int i) { return base + (size_t)i * ROWS_WORDS; }
+template <class PL>
+__device__ __forceinline__ auto lanes_of(const uint2* const (&tab)[4], int i) {
+    if constexpr (has_lane_table(PL::LOGN, PL::LOGE)) return tab[PL::LOGE - 3] + (size_t)i * (PL::N - PL::G);
+    else return NoLanes();
+}
 template <class Param>  // PrimeParam, or a prime of NttParams
 __device__ __forceinline__ Mod load_mod(const Param& q) {
     return Mod{q.p, q.p2, q.np, q.np2};
@@ -244,8 +248,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
     const int k = M.k;
     const PrimeParam& Q = M.pr[prime];
     const PrimeCtx c = load_prime_ctx(Q);
-    const uint2* __restrict__ psi = table_of(M.psi, prime);
-    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
+    const uint2* __restrict__ psi = table_of(M.tw.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.tw.ipsi, prime);
 
     const uint64_t* a = A + (size_t)job * a_stride;
     const uint64_t* b = Bv + (size_t)job * b_stride;
@@ -279,13 +283,13 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : mul
     // 64 coefficients per thread at N = 4096: both transforms loop over one copy of
     // the pass code (the unrolled three transforms overflow the instruction cache)
     constexpr bool LOOP64 = LOGN == 12 && LOGE == 6;
-    if constexpr (LOOP64) ntt64_forward<PL, 2>(x, psi, rows_of(M.psi_r, prime), c.m, tau, smem);
-    else ntt_forward<PL, 2>(x, psi, c.m, tau, smem, false, CtaSync(), 1, rows_of(M.psi_r, prime));
+    if constexpr (LOOP64) ntt64_forward<PL, 2>(x, psi, lanes_of<PL>(M.tw.psi_lanes, prime), c.m, tau, smem);
+    else ntt_forward<PL, 2>(x, psi, c.m, tau, smem, false, CtaSync(), 1, lanes_of<PL>(M.tw.psi_lanes, prime));
     uint32_t z[1][E];
 #pragma unroll
     for (int e = 0; e < E; e++) z[0][e] = mont(red_2p(x[0][e], c.m), red_2p(x[1][e], c.m), c.pinv, c.m);
-    if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, rows_of(M.ipsi_r, prime), c.m, tau, smem, nullptr);
-    else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime));
+    if constexpr (LOOP64) ntt64_inverse<PL, 1>(z, ipsi, lanes_of<PL>(M.tw.ipsi_lanes, prime), c.m, tau, smem, nullptr);
+    else ntt_inverse<PL, 1>(z, ipsi, c.m, tau, smem, CtaSync(), 1, lanes_of<PL>(M.tw.ipsi_lanes, prime));
     dep_launch();
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
@@ -363,8 +367,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
     const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
     const Mod m = load_mod(Q);
     const uint32_t p = m.p, pinv = Q.pinv;
-    const uint2* __restrict__ psi = table_of(M.psi, prime);
-    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
+    const uint2* __restrict__ psi = table_of(M.tw.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.tw.ipsi, prime);
     const uint64_t* cj = C + (size_t)job * PL::N * l64;
     // limb w of coefficient pos at cj[pos * cs + w * ls]: (cs, ls) = (limbs, 1) for
     // [N][limb], (1, N) for limb-major (the HE multiply's intermediate: a warp's
@@ -424,11 +428,11 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
             }
         }
         if constexpr (LOGN == 12 && LOGE == 6) {  // one copy of the pass code (see k_mul)
-            ntt64_forward<PL, ND>(x, psi, rows_of(M.psi_r, prime), m, tau, smem, d0 > 0);
+            ntt64_forward<PL, ND>(x, psi, lanes_of<PL>(M.tw.psi_lanes, prime), m, tau, smem, d0 > 0);
         } else {
-            ntt_forward<PL, ND>(x, psi, m, tau, smem, d0 > 0, CtaSync(), 1, rows_of(M.psi_r, prime));
+            ntt_forward<PL, ND>(x, psi, m, tau, smem, d0 > 0, CtaSync(), 1, lanes_of<PL>(M.tw.psi_lanes, prime));
         }
-        if constexpr (rows_pass<PL, LAST>()) {
+        if constexpr (E == 64) {
             // the key's copy laid out by lane (after the [ell][k][N] table): values u .. u+3
             // of lane tau are the 16-byte record [u/4][tau]
             static_assert(ND == 1, "one digit per pass with 64 coefficients per thread");
@@ -469,12 +473,12 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
             }
         }
     }
-    if constexpr (!ACC32 && !rows_pass<PL, LAST>()) {
+    if constexpr (!ACC32 && E < 64) {
 #pragma unroll
         for (int e = 0; e < E; e++) acc[0][e] = mac_finish<!(ONE && ND <= 2)>(T[e], pinv, m);
     }
-    if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, rows_of(M.ipsi_r, prime), m, tau, smem, nullptr);
-    else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime));
+    if constexpr (LOGN == 12 && LOGE == 6) ntt64_inverse<PL, 1>(acc, ipsi, lanes_of<PL>(M.tw.ipsi_lanes, prime), m, tau, smem, nullptr);
+    else ntt_inverse<PL, 1>(acc, ipsi, m, tau, smem, CtaSync(), 1, lanes_of<PL>(M.tw.ipsi_lanes, prime));
     dep_launch();
     uint32_t* out = resid + ((size_t)job * k + prime) * PL::N;
 #pragma unroll
@@ -522,14 +526,14 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, MINB)
         load_words<L64>(b1 + (size_t)pos * L64, w);
         x[1][e] = crt_words<W, false>(w, cc, qh, c);
     }
-    ntt_forward<PL, 2>(x, table_of(M.psi, prime), c.m, tau, smem);
+    ntt_forward<PL, 2>(x, table_of(M.tw.psi, prime), c.m, tau, smem, false, CtaSync(), 1, lanes_of<PL>(M.tw.psi_lanes, prime));
     uint32_t v[E];
     load_evk<PL::N, E>(key + (size_t)prime * PL::N, last_pos<PL>(tau), v);
 #pragma unroll
     for (int o = 0; o < 2; o++)
 #pragma unroll
         for (int e = 0; e < E; e++) x[o][e] = mont(x[o][e], v[e], c.pinv, c.m);  // [0, 4p) times [0, p) -> (0, 2p)
-    ntt_inverse<PL, 2>(x, table_of(M.ipsi, prime), c.m, tau, smem);
+    ntt_inverse<PL, 2>(x, table_of(M.tw.ipsi, prime), c.m, tau, smem, CtaSync(), 1, lanes_of<PL>(M.tw.ipsi_lanes, prime));
     dep_launch();
     uint32_t* out = resid + ((size_t)job0 * M.k + prime) * PL::N;
 #pragma unroll
@@ -575,7 +579,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
         for (int o = 0; o < 2; o++)
 #pragma unroll
             for (int e = 0; e < E; e++) x[o][e] = v[o][slot_pos<PL, 0>(tau, e)];
-        ntt_forward<PL, 2>(x, table_of(M.psi, prime), m, tau, smem);
+        ntt_forward<PL, 2>(x, table_of(M.tw.psi, prime), m, tau, smem, false, CtaSync(), 1, lanes_of<PL>(M.tw.psi_lanes, prime));
         if constexpr (COAL) rows_to_lanes<PL, 2>(x, smem, tau);
 #pragma unroll
         for (int o = 0; o < 2; o++) {
@@ -626,7 +630,7 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (ntt_min_blocks<LOGN, 
             }
         }
         if constexpr (COAL) lanes_to_rows<PL, 2>(x, smem, tau);
-        ntt_inverse<PL, 2>(x, table_of(M.ipsi, prime), m, tau, smem);
+        ntt_inverse<PL, 2>(x, table_of(M.tw.ipsi, prime), m, tau, smem, CtaSync(), 1, lanes_of<PL>(M.tw.ipsi_lanes, prime));
 #pragma unroll
         for (int o = 0; o < 2; o++) {
             if (o == 1 && !two) break;
@@ -679,8 +683,8 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
     if (!INV) {
 #pragma unroll
         for (int e = 0; e < E; e++) x[0][e] = COAL ? __ldcs(v + slot_pos<PL, 0>(tau, e)) : v[slot_pos<PL, 0>(tau, e)];
-        if constexpr (LOOP) ntt64_forward<PL, 1>(x, table_of(M.psi, prime), rows_of(M.psi_r, prime), m, tau, smem);
-        else ntt_forward<PL, 1>(x, table_of(M.psi, prime), m, tau, smem, false, CtaSync(), 1, rows_of(M.psi_r, prime));
+        if constexpr (LOOP) ntt64_forward<PL, 1>(x, table_of(M.tw.psi, prime), lanes_of<PL>(M.tw.psi_lanes, prime), m, tau, smem);
+        else ntt_forward<PL, 1>(x, table_of(M.tw.psi, prime), m, tau, smem, false, CtaSync(), 1, lanes_of<PL>(M.tw.psi_lanes, prime));
         if constexpr (COAL) {
             // row tau (positions 64 tau + u) into the padded buffer (word 65 tau + u: the words
             // this thread read last), then column tau (positions tau + 64 m, word 65 m + tau)
@@ -729,9 +733,9 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G * TPB, (MINB > 0 ? MINB
         }
         // N^-1 is applied inside the last stage (outputs in [0, p))
         if constexpr (LOOP)
-            ntt64_inverse<PL, 1>(x, table_of(M.ipsi, prime), rows_of(M.ipsi_r, prime), m, tau, smem, ninv + 4 * prime);
+            ntt64_inverse<PL, 1>(x, table_of(M.tw.ipsi, prime), lanes_of<PL>(M.tw.ipsi_lanes, prime), m, tau, smem, ninv + 4 * prime);
         else
-            ntt_inverse<PL, 1>(x, table_of(M.ipsi, prime), m, tau, smem, CtaSync(), 1, rows_of(M.ipsi_r, prime),
+            ntt_inverse<PL, 1>(x, table_of(M.tw.ipsi, prime), m, tau, smem, CtaSync(), 1, lanes_of<PL>(M.tw.ipsi_lanes, prime),
                                ninv + 4 * prime);
         if (store) {
 #pragma unroll

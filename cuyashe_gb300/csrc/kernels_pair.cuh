@@ -83,8 +83,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
     const PrimeParam& Q = M.pr[prime];
     const PrimeCtx c = load_prime_ctx(Q);
-    const uint2* __restrict__ psi = table_of(M.psi, prime);
-    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
+    const uint2* __restrict__ psi = table_of(M.tw.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.tw.ipsi, prime);
     uint32_t* recv = smem + region_bytes<PL, 2>() / 4;
     cluster_barrier();  // both blocks have started before any remote store
 
@@ -157,8 +157,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
     const Mod m = load_mod(Q);
     const uint32_t p = m.p;
-    const uint2* __restrict__ psi = table_of(M.psi, prime);
-    const uint2* __restrict__ ipsi = table_of(M.ipsi, prime);
+    const uint2* __restrict__ psi = table_of(M.tw.psi, prime);
+    const uint2* __restrict__ ipsi = table_of(M.tw.ipsi, prime);
     const uint64_t* cj = C + (size_t)job * (2 * kPairHalf) * l64;
     // limb w of coefficient pos at cj[pos * cs + w * ls]: (limbs, 1) for [N][limb],
     // (1, N) for limb-major

@@ -23,6 +23,7 @@
 // gamma = tau + v*G (v < E/2^R) with g = gamma / d, r = gamma % d. The
 // twiddle of stage s0+l for element u is tw[2^(s0+l) + g*2^l + (u >> (R-l))].
 #pragma once
+#include <type_traits>
 
 #include <stdint.h>
 
@@ -114,16 +115,28 @@ __device__ __forceinline__ uint2 load_twiddle(const uint2* __restrict__ twl, int
     return (h & 1) ? make_uint2(W2.z, W2.w) : make_uint2(W2.x, W2.y);
 }
 
-// Plans with 64 coefficients per thread end (forward) or start (inverse) with a
-// pass in which thread tau owns the 64 consecutive positions of row tau, and
-// needs twiddles tw[2^(S0+l) + tau 2^l + h] (h < 2^l): 2^l consecutive entries
-// per thread, 512 bytes apart between lanes at l = 6. Those passes read a copy
-// of the table laid out by lane ("rows" table, one per prime and length):
-// stage l starts at entry G (2^l - 1); its twiddle pairs (h, h+1) are 16-byte
-// records [h/2][tau], so that a warp's load covers 512 consecutive bytes.
-template <class PL, int PASS>
+// The last forward (first inverse) pass, in which thread tau owns the E consecutive
+// positions of row tau, needs twiddles tw[2^(S0+l) + tau 2^l + h] (h < 2^l): 2^l consecutive
+// entries per thread. It reads a copy of the table laid out by lane (rows_index), so that a
+// warp's loads are consecutive, where there is one.
+struct NoLanes {};  // in place of that table
+template <class PL, int PASS, class LT>
 __host__ __device__ constexpr bool rows_pass() {
-    return PL::LOGE == 6 && PASS == PL::NPASS - 1 && PL::LOGD(PASS) == 0;
+    return std::is_same<LT, const uint2*>::value && PASS == PL::NPASS - 1 && PL::NPASS > 1;
+}
+template <bool ROWS, class LT>
+__device__ __forceinline__ auto lanes_if(LT twr) {
+    if constexpr (ROWS) return twr;
+    else return NoLanes();
+}
+// first entry of stage l (a pass's group g, or lane tau of a lane-ordered table)
+template <class PL>
+__device__ __forceinline__ const uint2* stage_twiddles(const uint2*, const uint2* __restrict__ twr, int l, int, int tau) {
+    return twr + rows_index(PL::G, l, 0, tau);
+}
+template <class PL>
+__device__ __forceinline__ const uint2* stage_twiddles(const uint2* __restrict__ tws, NoLanes, int l, int g, int) {
+    return tws + (g << l);  // 16-byte aligned for l >= 1
 }
 __device__ __forceinline__ uint2 load_twiddle_rows(const uint2* __restrict__ twl, int h, int l, int G) {
     if (l == 0) return __ldg(twl);
@@ -134,15 +147,15 @@ __device__ __forceinline__ uint2 load_twiddle_rows(const uint2* __restrict__ twl
 // tm: twiddle-offset multiplier. A transform of length N is stages 0.. of one of
 // length 2N restricted to half h of it when its stage-s twiddles start at
 // (2 + h) * 2^s instead of 2^s (tm = 2 + h); tm = 1 for a whole transform.
-// twr: the rows table of this prime and length (plans with 64 coefficients per
-// thread; unused otherwise).
-template <class PL, int PASS, int NOPS>
+// twr: the lane-ordered table of this prime and length, or NoLanes.
+template <class PL, int PASS, int NOPS, class LT = NoLanes>
 __device__ __forceinline__ void fwd_pass(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
-                                         int tau, int tm = 1, const uint2* __restrict__ twr = nullptr) {
+                                         int tau, int tm = 1, LT twr = LT()) {
     constexpr int R = PL::R(PASS), S0 = PL::S0(PASS), LOGD = PL::LOGD(PASS);
     constexpr int GS = 1 << R;
     constexpr int NV = PL::E >> R;
-    constexpr bool ROWS = rows_pass<PL, PASS>();
+    constexpr bool ROWS = rows_pass<PL, PASS, LT>();
+    const auto lanes = lanes_if<ROWS>(twr);
 #pragma unroll
     for (int v = 0; v < NV; v++) {
         const int gam = tau + (v << (PL::LOGN - PL::LOGE));
@@ -150,8 +163,7 @@ __device__ __forceinline__ void fwd_pass(uint32_t (&x)[NOPS][PL::E], const uint2
 #pragma unroll
         for (int l = 0; l < R; l++) {
             const int half = 1 << (R - 1 - l);
-            const uint2* twl = ROWS ? twr + PL::G * ((1 << l) - 1) + (l == 0 ? tau : 2 * tau)
-                                    : tw + (tm << (S0 + l)) + (g << l);  // 16-byte aligned for l >= 1
+            const uint2* twl = stage_twiddles<PL>(tw + (tm << (S0 + l)), lanes, l, g, tau);
             // one flat loop of 2^(R-1) butterflies per stage (a trip count that does
             // not depend on l, so that every loop unrolls fully for R = 6 too):
             // butterfly b is j = b mod half of twiddle group h = b / half
@@ -171,14 +183,15 @@ __device__ __forceinline__ void fwd_pass(uint32_t (&x)[NOPS][PL::E], const uint2
 // scale (inverse, pass 0, optional): {N^-1, Shoup, N^-1 w1, Shoup} with w1 the
 // twiddle of the last stage; that stage then writes (X + Y) N^-1 and
 // (X - Y) w1 N^-1 in [0, p), so no separate scaling pass is needed.
-template <class PL, int PASS, int NOPS>
+template <class PL, int PASS, int NOPS, class LT = NoLanes>
 __device__ __forceinline__ void inv_pass(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
-                                         int tau, int tm = 1, const uint2* __restrict__ twr = nullptr,
+                                         int tau, int tm = 1, LT twr = LT(),
                                          const uint32_t* __restrict__ scale = nullptr) {
     constexpr int R = PL::R(PASS), S0 = PL::S0(PASS), LOGD = PL::LOGD(PASS);
     constexpr int GS = 1 << R;
     constexpr int NV = PL::E >> R;
-    constexpr bool ROWS = rows_pass<PL, PASS>();
+    constexpr bool ROWS = rows_pass<PL, PASS, LT>();
+    const auto lanes = lanes_if<ROWS>(twr);
 #pragma unroll
     for (int v = 0; v < NV; v++) {
         const int gam = tau + (v << (PL::LOGN - PL::LOGE));
@@ -186,8 +199,7 @@ __device__ __forceinline__ void inv_pass(uint32_t (&x)[NOPS][PL::E], const uint2
 #pragma unroll
         for (int l = R - 1; l >= 0; l--) {
             const int half = 1 << (R - 1 - l);
-            const uint2* twl = ROWS ? twr + PL::G * ((1 << l) - 1) + (l == 0 ? tau : 2 * tau)
-                                    : tw + (tm << (S0 + l)) + (g << l);  // 16-byte aligned for l >= 1
+            const uint2* twl = stage_twiddles<PL>(tw + (tm << (S0 + l)), lanes, l, g, tau);
             uint2 W = make_uint2(0u, 0u);
             if (PASS == 0 && l == 0 && scale != nullptr) {  // last stage, N^-1 folded in (S0 = 0, g = 0)
                 const uint32_t n0 = __ldg(scale), n0s = __ldg(scale + 1), n1 = __ldg(scale + 2),
@@ -357,30 +369,30 @@ __device__ __forceinline__ void lanes_to_rows(uint32_t (&x)[NOPS][PL::E], uint32
 }
 
 // Forward passes PASS .. NPASS-1 (sync_before: as in exchange, for the first one).
-template <class PL, int PASS, int NOPS, class Sync = CtaSync>
+template <class PL, int PASS, int NOPS, class Sync = CtaSync, class LT = NoLanes>
 struct FwdFrom {
     __device__ __forceinline__ static void run(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw,
                                                const Mod& m, int tau, uint32_t* sm, bool sync_before,
-                                               Sync bar = Sync(), int tm = 1, const uint2* __restrict__ twr = nullptr) {
+                                               Sync bar = Sync(), int tm = 1, LT twr = LT()) {
         if constexpr (PASS < PL::NPASS) {
             exchange<PL, PASS - 1, PASS, NOPS, Sync>(x, sm, tau, sync_before, bar);
             fwd_pass<PL, PASS, NOPS>(x, tw, m, tau, tm, twr);
-            FwdFrom<PL, PASS + 1, NOPS, Sync>::run(x, tw, m, tau, sm, false, bar, tm, twr);
+            FwdFrom<PL, PASS + 1, NOPS, Sync, LT>::run(x, tw, m, tau, sm, false, bar, tm, twr);
         }
     }
 };
 
 // Inverse passes PASS .. 0 where pass PASS+1 was the previous one.
-template <class PL, int PASS, int NOPS, class Sync = CtaSync>
+template <class PL, int PASS, int NOPS, class Sync = CtaSync, class LT = NoLanes>
 struct InvFrom {
     __device__ __forceinline__ static void run(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw,
                                                const Mod& m, int tau, uint32_t* sm, Sync bar = Sync(), int tm = 1,
-                                               const uint2* __restrict__ twr = nullptr,
+                                               LT twr = LT(),
                                                const uint32_t* __restrict__ scale = nullptr) {
         if constexpr (PASS >= 0) {
             exchange<PL, PASS + 1, PASS, NOPS, Sync>(x, sm, tau, false, bar);
             inv_pass<PL, PASS, NOPS>(x, tw, m, tau, tm, twr, scale);
-            InvFrom<PL, PASS - 1, NOPS, Sync>::run(x, tw, m, tau, sm, bar, tm, twr, scale);
+            InvFrom<PL, PASS - 1, NOPS, Sync, LT>::run(x, tw, m, tau, sm, bar, tm, twr, scale);
         }
     }
 };
@@ -388,23 +400,23 @@ struct InvFrom {
 // Full forward transform: registers in pass-0 layout (natural order) ->
 // registers in last-pass layout (bit-reversed order). sync_before: other threads may still
 // be reading `sm` (a transform before this one in the same block).
-template <class PL, int NOPS, class Sync = CtaSync>
+template <class PL, int NOPS, class Sync = CtaSync, class LT = NoLanes>
 __device__ __forceinline__ void ntt_forward(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
                                             int tau, uint32_t* sm, bool sync_before = false, Sync bar = Sync(),
-                                            int tm = 1, const uint2* __restrict__ twr = nullptr) {
+                                            int tm = 1, LT twr = LT()) {
     fwd_pass<PL, 0, NOPS>(x, tw, m, tau, tm, twr);
-    FwdFrom<PL, 1, NOPS, Sync>::run(x, tw, m, tau, sm, sync_before, bar, tm, twr);
+    FwdFrom<PL, 1, NOPS, Sync, LT>::run(x, tw, m, tau, sm, sync_before, bar, tm, twr);
 }
 
 // Full inverse transform: registers in last-pass layout -> pass-0 layout. `sm` may hold a
 // forward transform of this block (each thread then writes the words it read last).
-template <class PL, int NOPS, class Sync = CtaSync>
+template <class PL, int NOPS, class Sync = CtaSync, class LT = NoLanes>
 __device__ __forceinline__ void ntt_inverse(uint32_t (&x)[NOPS][PL::E], const uint2* __restrict__ tw, const Mod& m,
                                             int tau, uint32_t* sm, Sync bar = Sync(), int tm = 1,
-                                            const uint2* __restrict__ twr = nullptr,
+                                            LT twr = LT(),
                                             const uint32_t* __restrict__ scale = nullptr) {
     inv_pass<PL, PL::NPASS - 1, NOPS>(x, tw, m, tau, tm, twr, scale);
-    InvFrom<PL, PL::NPASS - 2, NOPS, Sync>::run(x, tw, m, tau, sm, bar, tm, twr, scale);
+    InvFrom<PL, PL::NPASS - 2, NOPS, Sync, LT>::run(x, tw, m, tau, sm, bar, tm, twr, scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -481,7 +493,7 @@ __device__ __forceinline__ void pass64_twiddles(int pass, const uint2* __restric
                                                 int tau, const uint2* (&twp)[6], int& tws) {
 #pragma unroll
     for (int l = 0; l < 6; l++)
-        twp[l] = pass == 0 ? tw + (1 << l) : twr + 64 * ((1 << l) - 1) + (l == 0 ? tau : 2 * tau);
+        twp[l] = pass == 0 ? tw + (1 << l) : twr + rows_index(64, l, 0, tau);
     tws = pass == 0 ? 2 : 128;
 }
 

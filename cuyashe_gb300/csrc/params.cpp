@@ -126,41 +126,63 @@ cy_status prime_table(int device, const PrimeTable** out) {
             ipsi[(size_t)i * NMAX + j] = make_uint2(wi, shoup_of(wi, p));
         }
     }
-    // row-pass tables of N = ROWS_N: entry (l, h, tau) = tw[2^(S0+l) + tau 2^l + h]
-    // with S0 = ROWS_LOGN - 6 the first stage of the row pass
-    std::vector<uint2> psi_r((size_t)TABLE_PRIMES * ROWS_WORDS), ipsi_r((size_t)TABLE_PRIMES * ROWS_WORDS);
-    for (int i = 0; i < TABLE_PRIMES; i++)
-        for (int l = 0; l < 6; l++)
-            for (int h = 0; h < (1 << l); h++)
-                for (int tau = 0; tau < ROWS_G; tau++) {
-                    const size_t src = (size_t)i * NMAX + ((size_t)1 << (ROWS_LOGN - 6 + l)) + ((size_t)tau << l) + h;
-                    const size_t dst = (size_t)i * ROWS_WORDS + rows_index(l, h, tau);
-                    psi_r[dst] = psi[src];
-                    ipsi_r[dst] = ipsi[src];
-                }
     PrimeTable* t = new PrimeTable();
     t->device = device;
     t->primes = primes;
     const size_t bytes = sizeof(uint2) * (size_t)TABLE_PRIMES * NMAX;
-    const size_t rbytes = sizeof(uint2) * psi_r.size();
     cudaError_t e = cudaMalloc(&t->d_psi, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&t->d_ipsi, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&t->d_psi_r, rbytes);
-    if (e == cudaSuccess) e = cudaMalloc(&t->d_ipsi_r, rbytes);
     if (e == cudaSuccess) e = cudaMemcpy(t->d_psi, psi.data(), bytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(t->d_ipsi, ipsi.data(), bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(t->d_psi_r, psi_r.data(), rbytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(t->d_ipsi_r, ipsi_r.data(), rbytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(t->d_psi);
         cudaFree(t->d_ipsi);
-        cudaFree(t->d_psi_r);
-        cudaFree(t->d_ipsi_r);
         delete t;
         return cuda_error(e, "prime table upload");
     }
     tables[device] = t;  // kept until process exit
     *out = t;
+    return CY_OK;
+}
+
+cy_status twiddle_tables(const PrimeTable& t, int logn, TwiddleTables* out) {
+    // one set of lane-ordered tables per device and length, kept until process exit
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, TwiddleTables> known;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find({t.device, logn});
+    if (it != known.end()) {
+        *out = it->second;
+        return CY_OK;
+    }
+    TwiddleTables T{};
+    T.psi = t.d_psi;
+    T.ipsi = t.d_ipsi;
+    cy_status st = CY_OK;
+    for (int e = 3; e <= 6 && st == CY_OK; e++) {
+        if (!has_lane_table(logn, e)) continue;
+        const size_t bytes = sizeof(uint2) * (size_t)TABLE_PRIMES * (((size_t)1 << logn) - ((size_t)1 << (logn - e)));
+        for (int inv = 0; inv < 2 && st == CY_OK; inv++) {
+            uint2* d = nullptr;
+            const cudaError_t err = cudaMalloc(&d, bytes);
+            (inv ? T.ipsi_lanes : T.psi_lanes)[e - 3] = d;
+            st = err != cudaSuccess ? cuda_error(err, "twiddle tables")
+                                    : build_lane_table(inv ? t.d_ipsi : t.d_psi, d, logn, e, TABLE_PRIMES);
+        }
+    }
+    if (st == CY_OK) {
+        const cudaError_t err = cudaStreamSynchronize(nullptr);
+        if (err != cudaSuccess) st = cuda_error(err, "twiddle tables");
+    }
+    if (st != CY_OK) {
+        for (int e = 0; e < 4; e++) {
+            cudaFree(const_cast<uint2*>(T.psi_lanes[e]));
+            cudaFree(const_cast<uint2*>(T.ipsi_lanes[e]));
+        }
+        return st;
+    }
+    known[{t.device, logn}] = T;
+    *out = T;
     return CY_OK;
 }
 
@@ -270,13 +292,10 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
     const PrimeTable* tab = nullptr;
     CY_TRY(prime_table(device, &tab));
     CY_TRY(basis_constants(b.h, &b.crt_bits, n, q, mode, bound, t, mont, scale_n, centered));
+    CY_TRY(twiddle_tables(*tab, b.h.logn, &b.h.tw));
     for (int i = 0; i < b.h.k; i++) {
         b.h.psi[i] = tab->d_psi + (size_t)i * NMAX;
         b.h.ipsi[i] = tab->d_ipsi + (size_t)i * NMAX;
-        if (b.h.logn == ROWS_LOGN) {
-            b.h.psi_r[i] = tab->d_psi_r + (size_t)i * ROWS_WORDS;
-            b.h.ipsi_r[i] = tab->d_ipsi_r + (size_t)i * ROWS_WORDS;
-        }
     }
     // per prime: N^-1, and N^-1 times the twiddle of the last inverse stage
     // (psi^-bitrev(1) = psi^-(NMAX/2)), each with its Shoup companion
@@ -306,15 +325,9 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
     std::copy(b.h.qhalf, b.h.qhalf + L32MAX, b.prod.qhalf);
     b.prod.k = b.h.k;
     b.prod.l64 = b.h.l64;
-    b.prod.psi = b.h.psi[0];
-    b.prod.ipsi = b.h.ipsi[0];
-    b.prod.psi_r = b.h.psi_r[0];
-    b.prod.ipsi_r = b.h.ipsi_r[0];
+    b.prod.tw = b.h.tw;
     b.ntt.k = b.h.k;
-    b.ntt.psi = b.prod.psi;
-    b.ntt.ipsi = b.prod.ipsi;
-    b.ntt.psi_r = b.prod.psi_r;
-    b.ntt.ipsi_r = b.prod.ipsi_r;
+    b.ntt.tw = b.h.tw;
     b.epi = epi_const(b.h.l32, b.h.k, b.h.mode);
     if (!b.epi) return set_error(CY_ERR_INTERNAL, "missing epilogue");
     b.epi_param.assign(b.epi->param_bytes, 0);
