@@ -59,32 +59,37 @@ static int sm_count() {
 // The schedule of a call that the autotuner has not chosen one for: `blocks` transforms'
 // blocks per launch (jobs times primes). Two regimes: up to one block per SM the time is one
 // block's latency (more threads per transform, or a pair of blocks); above, throughput. The
-// lines, measured with every schedule at q of 62, 127 (or 190) and 380 bits (us per call,
-// the schedule taken first):
-//   N = 1024   products of six limbs: 16 coefficients per thread from two blocks per SM on
-//              (512: 181 against 242; one: 17.0 against 15.2); all else within 3%
-//   N = 4096   products: 16 per thread, three blocks per SM (2048, 127-bit: 583 against 678 with
-//              8 per thread; one: 12.5 against 14.3). Keyswitch: 16 per thread, two blocks (2048:
-//              591 against 636), up to one block per SM 8 per thread, whole register file
-//              (one: 14.7 against 15.7). Transforms: 16 per thread (2048: 160 against 187)
-//   N = 8192   products: 16 per thread, two blocks (512, 190-bit: 670 against 721), up to one
-//              block per SM 128 registers (380-bit, one: 27.1 against 29.2). Keyswitch: 16 per
-//              thread and 128 registers (512, 190-bit: 712 against 1020, 64 registers spill),
-//              one limb two blocks (512: 149 against 173)
-//   N = 16384  up to one block per SM a pair of blocks per prime (380-bit, one: product 33
-//              against 50, keyswitch 78 against 165), above 32 per thread (64: 465 against 524
-//              and 885 against 1139), one limb 16 per thread (64: product 71 against 78,
-//              keyswitch 52 against 60)
+// lines, measured with every schedule at q of 60 to 380 bits (us per call, the schedule
+// taken first; jobs and bits of q in brackets):
+//   N = 1024   8 coefficients per thread (keyswitch [512, 190] 67 against 95 with 16), but 16 for
+//              products from two blocks per SM on ([2048, 127] 132 against 146, [512, 380] 163
+//              against 205) and transforms from four on ([2048, 127] 33 against 37)
+//   N = 2048   products 16 per thread ([512, 250] 186 against 216; [1, 250] 10.8 against 11.2),
+//              transforms from four blocks per SM on ([2048, 127] 66 against 80; [8, 127] 5.9
+//              against 4.5); keyswitch 8 ([512, 250] 227 against 479)
+//   N = 4096   16 per thread, products and transforms at three blocks per SM ([2048, 127] 567
+//              against 630 and 138 against 172 with 8), keyswitch two blocks of 128 registers
+//              ([2048, 127] 561 against 602), up to one block per SM at the full register file
+//              (one 127-bit: 14.7 against 15.7)
+//   N = 8192   16 per thread at 64 registers ([512, 190] 587 against 708), keyswitches of two
+//              limbs or more 128 registers ([37, 190] 55 against 58; [64, 380] 320 against 383)
+//   N = 16384  a pair of blocks per transform while that is one block per SM at most ([1, 380]
+//              product 27 against 40; [5, 380] keyswitch 73 against 106, but [8, 250] 96 against
+//              73). Above: keyswitch 32 per thread ([64, 62] 46 against 50, [256, 380] 2714
+//              against 2815), products of five limbs or more too ([64, 300] 371 against 386,
+//              [256, 380] 1680 against 1824; [64, 250] 246 against 236), all else 16
 int default_variant(int logn, int l64, int op, long long blocks) {
     const int sms = sm_count();
     const bool small = blocks <= sms;
     const bool product = op == TUNE_MUL || op == TUNE_MULC;
     switch (logn) {
-        case 10: return product && l64 >= 3 && blocks >= 2 * sms ? 1 : 0;
-        case 11: return product ? 1 : 0;
+        case 10: return (product && blocks >= 2 * sms) || (op == TUNE_NTT && blocks >= 4 * sms) ? 1 : 0;
+        case 11: return product || (op == TUNE_NTT && blocks >= 4 * sms) ? 1 : 0;
         case 12: return op == TUNE_KS ? (small ? 2 : 3) : 8;
         case 13: return op == TUNE_KS && l64 > 1 ? 2 : 0;
-        case 14: return op != TUNE_NTT && 2 * blocks <= sms ? 3 : 0;
+        case 14:
+            if (op != TUNE_NTT && 2 * blocks <= sms) return 3;
+            return op == TUNE_KS || (op == TUNE_MUL && l64 >= 5) ? 1 : 0;
         default: return 0;
     }
 }
