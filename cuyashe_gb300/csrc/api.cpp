@@ -180,6 +180,12 @@ cy_status run_mixed(const std::vector<const cy_polymul_job*>& jobs, cudaStream_t
 cy_status mixed_status(cudaStream_t st);
 bool mixed_supported(const cy_ring* r);
 
+// First job of chunk c of `nchunks`: the jobs divided evenly, since after a short last chunk its
+// lane idles while the others finish. HE multiplies at N = 16384, 380-bit q: 32 in chunks of 8
+// instead of 10, 10, 10 and 2 604 -> 533 us, 64 in seven 1085 -> 1029 us; products at N = 8192,
+// 190-bit q, 64 in two 82.5 -> 78.2 us.
+static int chunk_start(int batch, int nchunks, int c) { return (int)((long long)batch * c / nchunks); }
+
 // Lanes for a call of several chunks: lane 0 is the caller's stream with the
 // workspace's scratch, lanes 1.. side streams of the workspace with their own
 // scratch. Chunk c runs on lane c mod lanes (one chunk's kernels fill the tails
@@ -282,14 +288,15 @@ static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, l
     const KeyKernel* kk = key && batch > 1 ? key_kernel(B.h.logn, B.h.l64) : nullptr;
     if (kk) {
         const int n = B.h.n, k = B.h.k;
-        const int chunk = wave_chunk(std::min(batch, chunk_jobs(n, k)), kk->func, kk->threads, kk->smem, (k + 1) / 2);
+        int chunk = wave_chunk(std::min(batch, chunk_jobs(n, k)), kk->func, kk->threads, kk->smem, (k + 1) / 2);
+        if (chunk < batch) chunk += chunk & 1;
         const int nchunks = (batch + chunk - 1) / chunk;
         Lanes L;
         CY_TRY(L.begin(ws, st, (size_t)chunk * k * n, nchunks));
         cy_status status = CY_OK;
         for (int c = 0; c < nchunks && status == CY_OK; c++) {
-            const int j0 = c * chunk;
-            int nj = std::min(chunk, batch - j0);
+            const int j0 = chunk_start((batch + 1) / 2, nchunks, c) * 2;  // a block takes two jobs
+            int nj = std::min(chunk_start((batch + 1) / 2, nchunks, c + 1) * 2, batch) - j0;
             const uint64_t* bj = b + (size_t)j0 * b_stride;
             uint32_t* resid = L.scratch(c);
             void* args[] = {(void*)&B.prod, (void*)&key, (void*)&bj, (void*)&b_stride, (void*)&resid, (void*)&nj};
@@ -311,7 +318,7 @@ static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, l
     CY_TRY(L.begin(ws, st, (size_t)chunk * k * n, nchunks));
     cy_status status = CY_OK;
     for (int c = 0; c < nchunks && status == CY_OK; c++) {
-        const int j0 = c * chunk, nj = std::min(chunk, batch - j0);
+        const int j0 = chunk_start(batch, nchunks, c), nj = chunk_start(batch, nchunks, c + 1) - j0;
         status = product_chunk(B, ks, centered, a + (size_t)j0 * a_stride, a_stride, b + (size_t)j0 * b_stride,
                                b_stride, (char*)out + (size_t)j0 * out_stride * sizeof(uint64_t), nj, L.scratch(c),
                                L.stream(c));
@@ -339,7 +346,7 @@ static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint32_t
     CY_TRY(L.begin(ws, st, (size_t)chunk * k * n, nchunks));
     cy_status status = CY_OK;
     for (int cc = 0; cc < nchunks && status == CY_OK; cc++) {
-        const int j0 = cc * chunk, nj = std::min(chunk, batch - j0);
+        const int j0 = chunk_start(batch, nchunks, cc), nj = chunk_start(batch, nchunks, cc + 1) - j0;
         status = keyswitch_chunk(B, ks, sel, c + (size_t)j0 * n * l64, evk, ell, out + (size_t)j0 * n * l64, nj,
                                  L.scratch(cc), L.stream(cc), lm);
     }
@@ -373,7 +380,11 @@ cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t*
     CY_TRY(L.begin(ws, st, (size_t)chunk * kmax * n, nchunks));
     cy_status status = CY_OK;
     for (int c = 0; c < nchunks && status == CY_OK; c++) {
-        const int j0 = c * chunk, nj = std::min(chunk, batch - j0);
+        // (two chunks stay unequal: even ones run the same phase at the same time, and the tails
+        // of one's launches are not filled by the other's; 64 multiplies at N = 8192, 190-bit q, 40
+        // and 24 172.7 us, 32 and 32 176.0 us)
+        const int j0 = nchunks > 2 ? chunk_start(batch, nchunks, c) : c * chunk;
+        const int nj = (nchunks > 2 ? chunk_start(batch, nchunks, c + 1) : std::min(batch, j0 + chunk)) - j0;
         uint64_t* oj = out + (size_t)j0 * stride;
         // with relinearisation the rounded tensor product goes to `out` limb-major
         // (coalesced digit loads in the keyswitch), and the keyswitch's epilogue
