@@ -354,8 +354,8 @@ static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint32_t
 }
 
 // The HE multiply of `batch` pairs: per chunk, the tensor product with the
-// YASHE rounding into out, then (relin) its keyswitch in place; chunks alternate
-// between two lanes.
+// YASHE rounding into out, then (relin) its keyswitch in place; chunks go round
+// the lanes.
 // ks_variant >= 0 forces the keyswitch schedule (the autotuner's timing runs).
 cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
                         const uint64_t* c2, uint64_t* out, int batch, bool do_relin, Workspace& ws, cudaStream_t st,
