@@ -280,12 +280,15 @@ static int product_chunk_jobs(const Basis& B, const KernelSet& ks, bool centered
 // products of `batch` jobs with basis B: out_j = epilogue(a_j * b_j); `variant`
 // selects the NTT schedule (-1: the tuned one for this device and size). key: the kept
 // transform of a (a_stride = 0), used from two products on (a block takes two) where there is a
-// kernel for it
+// kernel for it; small: b's jobs are small signed words at the start of their rows (L64 = 0 of
+// k_mul_key, any number of products)
 static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, long long a_stride,
                              const uint64_t* b, long long b_stride, void* out, long long out_stride, int batch,
-                             Workspace& ws, cudaStream_t st, int variant = -1, const uint32_t* key = nullptr) {
+                             Workspace& ws, cudaStream_t st, int variant = -1, const uint32_t* key = nullptr,
+                             bool small = false) {
     if (batch == 0) return CY_OK;
-    const KeyKernel* kk = key && batch > 1 ? key_kernel(B.h.logn, B.h.l64) : nullptr;
+    const KeyKernel* kk = key && (batch > 1 || small) ? key_kernel(B.h.logn, small ? 0 : B.h.l64) : nullptr;
+    if (small && !kk) return set_error(CY_ERR_INTERNAL, "missing kernel instantiation");
     if (kk) {
         const int n = B.h.n, k = B.h.k;
         int chunk = wave_chunk(std::min(batch, chunk_jobs(n, k)), kk->func, kk->threads, kk->smem, (k + 1) / 2);
@@ -476,8 +479,8 @@ cy_status check_aligned_api(const void* a, const void* b, const void* c) { retur
 
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
-                          cudaStream_t st, int variant, const uint32_t* key) {
-    return run_product(B, centered, a, a_stride, b, b_stride, out, out_stride, batch, ws, st, variant, key);
+                          cudaStream_t st, int variant, const uint32_t* key, bool small) {
+    return run_product(B, centered, a, a_stride, b, b_stride, out, out_stride, batch, ws, st, variant, key, small);
 }
 
 // Jobs per chunk of an HE multiply of `batch` pairs, as run_yashe_mul cuts it
@@ -501,8 +504,8 @@ cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* e
 
 // The transform of the polynomial at d_poly ([N][l64] limbs) for k_mul_key with basis B:
 // *d_key [k][N], allocated on the first call. N < 1024 has no such kernel: null. On the
-// legacy default stream; the caller synchronises.
-cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key) {
+// legacy default stream; the caller synchronises. up: for products with a small operand.
+cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key, int up) {
     if (!key_kernel(B.h.logn, B.h.l64)) return CY_OK;
     long long total = (long long)B.h.k * B.h.n;
     if (!*d_key) CY_CUDA(cudaMalloc(d_key, sizeof(uint32_t) * total));
@@ -511,7 +514,6 @@ cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key) 
     cy_status st = run_crt(B, d_poly, res, nullptr, 1, 0);
     if (st == CY_OK) st = run_ntt(B, res, 1, false, 0);
     const BasisDev* Bd = B.d;
-    int up = 0;
     void* args[] = {(void*)&Bd, (void*)&res, (void*)d_key, (void*)&total, (void*)&up};
     if (st == CY_OK)
         st = launch(evk_mont_kernel(), "key_mont", B.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0, args);

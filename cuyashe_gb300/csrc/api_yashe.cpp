@@ -20,8 +20,8 @@ namespace cy {
 cy_status check_aligned_api(const void* a, const void* b, const void* c);
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
-                          cudaStream_t st, int variant = -1, const uint32_t* key = nullptr);
-cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key);
+                          cudaStream_t st, int variant = -1, const uint32_t* key = nullptr, bool small = false);
+cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key, int up = 0);
 cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
                         const uint64_t* c2, uint64_t* out, int batch, bool do_relin, Workspace& ws, cudaStream_t st,
                         int ks_variant = -1);
@@ -140,7 +140,8 @@ cy_status cy_yashe_set_keys(cy_yashe* y, const uint64_t* h_f, const uint64_t* h_
     CY_CUDA(cudaMemcpy(y->d_f, h_f, poly * sizeof(uint64_t), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMemcpy(y->d_h, h_h, poly * sizeof(uint64_t), cudaMemcpyHostToDevice));
     CY_TRY(cy_polymul(r, y->d_f, y->d_f, y->d_f2, 1, nullptr));
-    CY_TRY(prepare_key(r->mul, y->d_h, &y->d_h_key));
+    // in the keyswitch basis: |h s| < N 256 q (kCdtMax thresholds) < ell N 2^32 q
+    CY_TRY(prepare_key(y->relin, y->d_h, &y->d_h_key, 1));
     CY_TRY(prepare_key(y->dec, y->d_f, &y->d_f_key));
     CY_TRY(prepare_key(y->dec, y->d_f2, &y->d_f2_key));
     if (y->d_evk) {

@@ -29,7 +29,8 @@ struct KernelSet {
 int variant_count(int logn);
 const KernelSet& kernel_variant(int logn, int v);
 
-// Products with a kept operand (k_mul_key) for N = 2^logn >= 1024 and l64 limbs.
+// Products with a kept operand (k_mul_key) for N = 2^logn >= 1024 and l64 limbs (0: the other
+// operand is small).
 struct KeyKernel {
     void* func;
     int threads;

@@ -14,8 +14,8 @@
 // u is mapped to x = j - B with j the first index of the CDT table with
 // u < T[j] (T: 64-bit cumulative thresholds, see gaussian_cdt).
 //
-// Three steps on the caller's stream: k_enc_sample writes s (as limbs mod q)
-// into the output, the product kernels compute h*s in place (a chunk's product
+// Three steps on the caller's stream: a sampling kernel writes s (as limbs mod q, or
+// as signed words) into the output, the product kernels compute h*s in place (a chunk's product
 // kernel reads its inputs before its epilogue writes), and k_enc_finish adds e
 // and Delta*m and reduces mod q.
 #include <cuda_runtime.h>
@@ -31,7 +31,7 @@ namespace cy {
 
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
-                          cudaStream_t st, int variant = -1, const uint32_t* key = nullptr);
+                          cudaStream_t st, int variant = -1, const uint32_t* key = nullptr, bool small = false);
 int trace_begin(const char* name, int logn, cudaStream_t st);
 void trace_end(int idx, cudaStream_t st);
 
@@ -184,6 +184,18 @@ __global__ void k_enc_sample(const __grid_constant__ EncConsts C, const uint64_t
     const long long b = idx >> C.logn, i = idx & ((1LL << C.logn) - 1);
     const int s = cdt_sample(sT, C.ncdt, C.bound, counter_draw(C.seed, ((uint64_t)(2 * b) << C.logn) + i));
     store_signed<L>(C, s, out + idx * L);
+}
+
+// s -> the first words of each ciphertext's row, one signed word per coefficient
+__global__ void k_enc_sample_small(const __grid_constant__ EncConsts C, const uint64_t* __restrict__ T,
+                                   uint64_t* __restrict__ out, int batch) {
+    __shared__ uint64_t sT[kCdtMax];
+    load_cdt(sT, T, C.ncdt);
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= ((long long)batch << C.logn)) return;
+    const long long b = idx >> C.logn, i = idx & ((1LL << C.logn) - 1);
+    reinterpret_cast<int*>(out + ((b * C.l64) << C.logn))[i] =
+        cdt_sample(sT, C.ncdt, C.bound, counter_draw(C.seed, ((uint64_t)(2 * b) << C.logn) + i));
 }
 
 // ct = [hs + e + Delta*(m mod t)]_q in place (hs in [0, q), e in [-B, B])
@@ -360,9 +372,13 @@ extern "C" cy_status cy_yashe_encrypt(cy_yashe* y, const uint64_t* d_m, uint64_t
     C.ncdt = y->n_cdt;
     const long long total = (long long)batch << r->logn;
     void* sargs[] = {(void*)&C, (void*)&y->d_cdt, (void*)&d_ct, (void*)&batch};
-    CY_TRY(launch_enc(k_enc_sample_for(C.l64), "enc_sample", C, total, st, sargs));
     const long long stride = (long long)r->n * r->l64;
-    CY_TRY(run_product_api(r->mul, false, y->d_h, 0, d_ct, stride, d_ct, stride, batch, r->own_ws.ws, st, -1, y->d_h_key));
+    // The product with s runs in the keyswitch basis, which is wide enough for it and has fewer
+    // primes than the product's (six instead of nine at 127-bit q); N < 1024 takes the ordinary one.
+    const bool small = y->d_h_key != nullptr;
+    CY_TRY(launch_enc(small ? (void*)k_enc_sample_small : k_enc_sample_for(C.l64), "enc_sample", C, total, st, sargs));
+    CY_TRY(run_product_api(small ? y->relin : r->mul, false, y->d_h, 0, d_ct, stride, d_ct, stride, batch, r->own_ws.ws, st,
+                           -1, y->d_h_key, small));
     void* fargs[] = {(void*)&C, (void*)&y->d_cdt, (void*)&d_m, (void*)&d_ct, (void*)&batch};
     return launch_enc(k_enc_finish_for(C.l64), "enc_finish", C, total, st, fargs);
 }

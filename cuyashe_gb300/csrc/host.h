@@ -160,7 +160,8 @@ struct cy_yashe {
     uint64_t* d_f2 = nullptr;
     uint64_t* d_h = nullptr;    // public key (GPU encryption)
     uint32_t* d_evk = nullptr;  // [ell][k'][N] NTT-domain evaluation key times 2^32
-    // transforms of h, f and f^2 for products with a batch (k_mul_key; null for N < 1024)
+    // transforms of h, f and f^2 for products with a batch (k_mul_key; null for N < 1024); h's in
+    // the keyswitch basis, for products with a small s
     uint32_t* d_h_key = nullptr;
     uint32_t* d_f_key = nullptr;
     uint32_t* d_f2_key = nullptr;

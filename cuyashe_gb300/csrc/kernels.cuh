@@ -493,13 +493,17 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, (MINB > 0 ? MINB : ks_
 // with an odd count the last block repeats its job and stores it once).
 // 512 products with a kept operand (256 encryptions and their decryptions) at N = 4096, 127-bit
 // q: 123 us (k_mul: 152).
+// L64 = 0: the other operand is small (encryption's s), a signed 32-bit word per coefficient at
+// the start of its job's row, its residues s or s + p; key: transforms times 2^32. 256
+// encryptions and their decryptions at N = 4096, 127-bit q: 140 us with s as limbs mod q in the
+// product basis (nine primes), 126 with words in the keyswitch basis (six).
 // --------------------------------------------------------------------------
 template <int LOGN, int LOGE, int L64, int MINB>
 __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, MINB)
     k_mul_key(const __grid_constant__ ProdParams M, const uint32_t* __restrict__ key, const uint64_t* __restrict__ Bv,
               long long b_stride, uint32_t* __restrict__ resid, int njobs) {
     using PL = NttPlan<LOGN, LOGE>;
-    constexpr int E = PL::E, W = 2 * L64;
+    constexpr int E = PL::E, W = 2 * (L64 ? L64 : 1);
     extern __shared__ __align__(16) uint32_t smem[];  // exchange buffer, 2 operands x SMW
     const int tau = threadIdx.x;
     const int prime = blockIdx.y;
@@ -520,11 +524,18 @@ __global__ void __launch_bounds__(NttPlan<LOGN, LOGE>::G, MINB)
 #pragma unroll
     for (int e = 0; e < E; e++) {
         const int pos = slot_pos<PL, 0>(tau, e);
-        uint32_t w[W];
-        load_words<L64>(b0 + (size_t)pos * L64, w);
-        x[0][e] = crt_words<W, false>(w, cc, qh, c);
-        load_words<L64>(b1 + (size_t)pos * L64, w);
-        x[1][e] = crt_words<W, false>(w, cc, qh, c);
+        if constexpr (L64 == 0) {
+            const int s0 = (int)ld_dep_cg(reinterpret_cast<const uint32_t*>(b0) + pos);
+            const int s1 = (int)ld_dep_cg(reinterpret_cast<const uint32_t*>(b1) + pos);
+            x[0][e] = s0 < 0 ? s0 + c.m.p : s0;
+            x[1][e] = s1 < 0 ? s1 + c.m.p : s1;
+        } else {
+            uint32_t w[W];
+            load_words<L64>(b0 + (size_t)pos * L64, w);
+            x[0][e] = crt_words<W, false>(w, cc, qh, c);
+            load_words<L64>(b1 + (size_t)pos * L64, w);
+            x[1][e] = crt_words<W, false>(w, cc, qh, c);
+        }
     }
     ntt_forward<PL, 2>(x, table_of(M.tw.psi, prime), c.m, tau, smem, false, CtaSync(), 1, lanes_of<PL>(M.tw.psi_lanes, prime));
     uint32_t v[E];

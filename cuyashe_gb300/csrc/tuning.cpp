@@ -29,7 +29,7 @@ namespace cy {
 
 cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long long a_stride, const uint64_t* b,
                           long long b_stride, void* out, long long out_stride, int batch, Workspace& ws,
-                          cudaStream_t st, int variant, const uint32_t* key = nullptr);
+                          cudaStream_t st, int variant, const uint32_t* key = nullptr, bool small = false);
 cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* evk, int ell, uint64_t* out, int batch,
                             Workspace& ws, cudaStream_t st, int variant, int chunk_k, int lm);
 cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint32_t** d_evk);

@@ -64,3 +64,22 @@ def test_encrypt_with_kept_key_equals_product(n, bits):
     s = y.ring.polysub(se, e)
     hh = y.ring.upload([h] * batch)
     assert torch.equal(ct, y.ring.polyadd(y.ring.polymul(hh, s), e))
+
+
+@pytest.mark.parametrize("n,bits", [(1024, 62), (2048, 310), (4096, 127), (8192, 250), (16384, 190)])
+def test_encrypt_one_equals_first_of_batch(n, bits):
+    """Draws are counted per ciphertext, so a batch begins with the ciphertext of a call of one; h at
+    the edges of [0, q)."""
+    import torch
+
+    import cuyashe_gb300 as cy
+
+    rng = random.Random(n)
+    q = (1 << bits) - 57
+    y = cy.Yashe(n, q, 17)
+    h = [rng.choice([0, 1, q - 1]) for _ in range(n)]
+    y.set_keys([[1] + [0] * (n - 1)], [h], [[0] * n for _ in range(y.ell)])
+    m = torch.randint(17, (5, n), generator=torch.Generator().manual_seed(n)).cuda()
+    whole = y.encrypt(m, seed=11)
+    for batch in (1, 2, 4):
+        assert torch.equal(y.encrypt(m[:batch].contiguous(), seed=11), whole[:batch])
