@@ -45,7 +45,7 @@ constexpr int epi_coefs_per_thread(int l32) { return l32 <= 6 ? 2 : 1; }
 
 // Twiddle tables of the first prime; those of prime i follow i tables on. `lanes`: the last
 // (forward) or first (inverse) pass's twiddles laid out by lane, for plans with 2^e
-// coefficients per thread, e = 3 .. 6 (rows_index; null where no schedule reads them). In the
+// coefficients per thread, e = 4 .. 6 (rows_index; null where no schedule reads them). In the
 // natural order a thread with 16 coefficients reads 64 consecutive bytes of a stage, and a warp's
 // 16-byte loads step 64 bytes per lane: 16 L1 cycles each instead of four. Measured, natural ->
 // lane order: 512 x 14 transforms of length 8192 146 -> 142 us forward, 151 -> 141 inverse; 512
@@ -53,15 +53,16 @@ constexpr int epi_coefs_per_thread(int l32) { return l32 <= 6 ? 2 : 1; }
 struct TwiddleTables {
     const uint2* psi;
     const uint2* ipsi;
-    const uint2* psi_lanes[4];
-    const uint2* ipsi_lanes[4];
+    const uint2* psi_lanes[3];
+    const uint2* ipsi_lanes[3];
 };
-// The plans of at least 1024 with 8 or 16 coefficients per thread, and those with 32 or 64.
+// The plans of at least 1024 with 16 coefficients per thread, and those with 32 or 64. (With 8 a
+// run is 32 bytes: 96 HE multiplies at N = 2048, 62-bit q, 21.15 us with a table, 21.15 without.)
 #ifdef __CUDACC__
 __host__ __device__
 #endif
 constexpr bool has_lane_table(int logn, int loge) {
-    return logn >= 10 && (loge == 3 || loge == 4 || (loge == 5 && logn == LOGN_MAX) || (loge == 6 && logn == ROWS_LOGN));
+    return logn >= 10 && (loge == 4 || (loge == 5 && logn == LOGN_MAX) || (loge == 6 && logn == ROWS_LOGN));
 }
 // Entry of a lane-ordered table (G threads per transform) of stage l, twiddle h (< 2^l) and lane
 // tau: stage l starts at G (2^l - 1); for l >= 1 the pairs (h, h+1) are 16-byte records

@@ -44,8 +44,8 @@ __device__ __forceinline__ Mod load_mod(const BasisDev* __restrict__ B, int i) {
 // The tables of prime i.
 __device__ __forceinline__ const uint2* table_of(const uint2* base, int i) { return base + (size_t)i * NMAX; }
 template <class PL>
-__device__ __forceinline__ auto lanes_of(const uint2* const (&tab)[4], int i) {
-    if constexpr (has_lane_table(PL::LOGN, PL::LOGE)) return tab[PL::LOGE - 3] + (size_t)i * (PL::N - PL::G);
+__device__ __forceinline__ auto lanes_of(const uint2* const (&tab)[3], int i) {
+    if constexpr (has_lane_table(PL::LOGN, PL::LOGE)) return tab[PL::LOGE - 4] + (size_t)i * (PL::N - PL::G);
     else return NoLanes();
 }
 template <class Param>  // PrimeParam, or a prime of NttParams

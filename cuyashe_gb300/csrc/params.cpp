@@ -159,13 +159,13 @@ cy_status twiddle_tables(const PrimeTable& t, int logn, TwiddleTables* out) {
     T.psi = t.d_psi;
     T.ipsi = t.d_ipsi;
     cy_status st = CY_OK;
-    for (int e = 3; e <= 6 && st == CY_OK; e++) {
+    for (int e = 4; e <= 6 && st == CY_OK; e++) {
         if (!has_lane_table(logn, e)) continue;
         const size_t bytes = sizeof(uint2) * (size_t)TABLE_PRIMES * (((size_t)1 << logn) - ((size_t)1 << (logn - e)));
         for (int inv = 0; inv < 2 && st == CY_OK; inv++) {
             uint2* d = nullptr;
             const cudaError_t err = cudaMalloc(&d, bytes);
-            (inv ? T.ipsi_lanes : T.psi_lanes)[e - 3] = d;
+            (inv ? T.ipsi_lanes : T.psi_lanes)[e - 4] = d;
             st = err != cudaSuccess ? cuda_error(err, "twiddle tables")
                                     : build_lane_table(inv ? t.d_ipsi : t.d_psi, d, logn, e, TABLE_PRIMES);
         }
@@ -175,7 +175,7 @@ cy_status twiddle_tables(const PrimeTable& t, int logn, TwiddleTables* out) {
         if (err != cudaSuccess) st = cuda_error(err, "twiddle tables");
     }
     if (st != CY_OK) {
-        for (int e = 0; e < 4; e++) {
+        for (int e = 0; e < 3; e++) {
             cudaFree(const_cast<uint2*>(T.psi_lanes[e]));
             cudaFree(const_cast<uint2*>(T.ipsi_lanes[e]));
         }
