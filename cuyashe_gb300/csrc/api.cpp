@@ -150,17 +150,19 @@ static std::atomic<int> g_epi_generic{0};
 // ICRT epilogue of basis B over `nj` jobs of residues [job][k][N] into `out`.
 // lm: outputs limb-major ([job][limb][N]), for the keyswitch that follows in an
 // HE multiply (its digit loads then cover consecutive words).
-// any_x: residues of any X (cy_icrt), not only of |X| < M/4: k_epi's 64-bit estimate
-// of v decides up to the ends of (-M/2, M/2)
+// any_x: residues of any X (cy_icrt), not only of |X| < M/4: the 64-bit estimate
+// of v decides up to the ends of (-M/2, M/2). (EPI_MODQ only)
 static cy_status launch_epi(const Basis& B, const uint32_t* resid, void* out, int nj, cudaStream_t st,
                             const char* name, int lm = 0, bool any_x = false) {
     const BasisDev* Bd = B.d;
     unsigned long long fl = epi_frac_limit();
     const long long coefs = (long long)nj * B.h.n;
-    if (!any_x && !g_epi_generic.load()) {
-        void* args[] = {(void*)B.epi_param.data(), (void*)&Bd, (void*)&resid, (void*)&out, (void*)&nj, (void*)&fl,
-                        (void*)&lm};
-        return launch(B.epi->func, name, B.h.logn, dim3((unsigned)((coefs + kEpiThreads - 1) / kEpiThreads)),
+    if (!g_epi_generic.load()) {
+        const bool any_k = any_x && !B.epi->any_x;
+        void* func = any_k ? epi_const_any(B.h.l32, B.h.mode)->any_x : any_x ? B.epi->any_x : B.epi->func;
+        void* args[] = {(void*)(any_k ? B.any_param : B.epi_param).data(), (void*)&Bd, (void*)&resid, (void*)&out,
+                        (void*)&nj, (void*)&fl, (void*)&lm};
+        return launch(func, name, B.h.logn, dim3((unsigned)((coefs + kEpiThreads - 1) / kEpiThreads)),
                       dim3(kEpiThreads), 0, st, args, true);
     }
     void* args[] = {(void*)&Bd, (void*)&resid, (void*)&out, (void*)&nj, (void*)&fl, (void*)&lm};

@@ -42,7 +42,7 @@ const KeyKernel* key_kernel(int logn, int l64);
 enum TuneOp { TUNE_MUL = 0, TUNE_MULC = 1, TUNE_KS = 2, TUNE_NTT = 3, TUNE_OPS = 4 };
 
 // ICRT epilogue for `l32` words of q and epilogue mode (EpiMode) with its constants
-// in shared memory (residues of any X: cy_icrt; comparison).
+// in shared memory (for comparison: cy_set_epilogue_generic).
 void* epi_kernel(int l32, int mode);
 
 // Epilogue with the constants of its basis as the first parameter, by value
@@ -52,6 +52,7 @@ struct EpiConstKernel {
     void* func;
     size_t param_bytes;
     void (*fill)(const BasisDev& h, void* param);
+    void* any_x;  // the kernel for residues of any X (cy_icrt; null where the one for any prime count serves)
 };
 const EpiConstKernel* epi_const(int l32, int k, int mode);
 const EpiConstKernel* epi_const_any(int l32, int mode);  // for any prime count

@@ -60,7 +60,8 @@ struct Basis {
     int crt_bits = 0;
     const EpiConstKernel* epi = nullptr;   // epilogue of this basis
     std::vector<unsigned char> epi_param;  // its parameter block (constants by value)
-    void* d_epi = nullptr;  // the parameter block for any prime count, for the mixed batches
+    std::vector<unsigned char> any_param;  // the parameter block of the epilogues for any prime count
+    void* d_epi = nullptr;  // its copy in device memory, for the mixed batches
     Basis() = default;
     Basis(const Basis&) = delete;
     Basis& operator=(const Basis&) = delete;

@@ -3,7 +3,9 @@
 
 namespace cy {
 
-#define CY_EPI_ANY(L, MODE) {(void*)k_epi_c<L, MODE, 0>, sizeof(EpiConst<L, KMAX>), fill_epi_const<L, KMAX>}
+#define CY_EPI_ANY(L, MODE)                                                               \
+    {(void*)k_epi_c<L, MODE, 0>, sizeof(EpiConst<L, KMAX>), fill_epi_const<L, KMAX>, \
+     MODE == EPI_MODQ ? (void*)k_epi_c<L, EPI_MODQ, 0, true> : nullptr}
 #define CY_EPI_ROW(L) {CY_EPI_ANY(L, EPI_MODQ), CY_EPI_ANY(L, EPI_YASHE), CY_EPI_ANY(L, EPI_DECRYPT)}
 
 const EpiConstKernel* epi_any3(int l32, int mode) {

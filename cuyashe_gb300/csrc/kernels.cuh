@@ -1120,15 +1120,14 @@ __global__ void __launch_bounds__(256) k_epi(const BasisDev* __restrict__ B, con
 // cycles, a low one two), so what a prime costs there was cut: v = round(sum y_i / p_i)
 // is summed in 26-bit fixed point from 13-bit factors (one shift and one low product
 // instead of a wide and a high one): each term is low by at most 2^-13 + 2^-13, the sum
-// of 40 by less than 0.01, and |X| < M/4 leaves 0.25. (cy_icrt takes residues of any X
-// and keeps k_epi's 64-bit sum.) Barrett's quotient is formed from 32-bit pieces
+// of 40 by less than 0.01, and |X| < M/4 leaves 0.25. ANYX (cy_icrt: residues of any X in
+// (-M/2, M/2)): k_epi's 64-bit sum. Barrett's quotient is formed from 32-bit pieces
 // of 45-bit operands and is at most one low, so one conditional subtraction ends it.
-// Measured with those of k_epi_k, the kernel this replaces, at N = 4096, 127-bit q.
 // --------------------------------------------------------------------------
 template <int L>
 struct __align__(16) EpiPrimeC {
-    uint32_t p, np, ycon, ycon_sh;
-    uint32_t g, F0, F1, pad;  // floor(2^43 / p); R_i / q in units of 2^-64 (YASHE)
+    uint32_t fhi, np, ycon, ycon_sh;  // floor(2^64 / p) in words fhi, flo (ANYX)
+    uint32_t g, F0, F1, flo;          // floor(2^43 / p); R_i / q in units of 2^-64 (YASHE)
     uint32_t A0[L];
 };
 template <int L, int KS>
@@ -1224,7 +1223,7 @@ __device__ __forceinline__ uint32_t red_neg(uint32_t x, uint32_t nm) { return __
 // lstride], or one word for DECRYPT). P: the basis's constants (a kernel parameter, or a
 // copy in shared memory).
 // DEP: called by k_epi_c (dependent launches).
-template <int L, int MODE, int K, bool DEP, class Const>
+template <int L, int MODE, int K, bool DEP, bool ANYX = false, class Const>
 __device__ __forceinline__ void epi_c_one(const Const& P, const BasisDev* __restrict__ B,
                                           const uint32_t* __restrict__ r0, int n, uint64_t* __restrict__ out,
                                           size_t lstride, unsigned long long frac_limit) {
@@ -1234,12 +1233,13 @@ __device__ __forceinline__ void epi_c_one(const Const& P, const BasisDev* __rest
 
     Cols<L> x;   // sum y_i A0_i
     Cols<2> z;   // YASHE: Z = sum y_i F_i in 32-bit columns
-    uint32_t vs = 0x2000000u;  // sum y_i / p_i + 1/2 in units of 2^-26
+    std::conditional_t<ANYX, uint64_t, uint32_t> vs = ANYX ? 0x80000000u : 0x2000000u;  // sum y_i / p_i + 1/2 in units of 2^-32 or 2^-26
     x.zero();
     z.zero();
     auto absorb = [&](const EpiPrimeC<L>& E, uint32_t res) {
         const uint32_t y = red_neg(__umulhi(res, E.ycon_sh) * E.np + res * E.ycon, E.np);
-        vs += (y >> 17) * E.g;
+        if constexpr (ANYX) vs += (uint64_t)y * E.fhi + __umulhi(y, E.flo);
+        else vs += (y >> 17) * E.g;
 #pragma unroll
         for (int w = 0; w < L; w++) x.c[w] += (uint64_t)y * E.A0[w];
         if (MODE == EPI_YASHE) {
@@ -1282,7 +1282,7 @@ __device__ __forceinline__ void epi_c_one(const Const& P, const BasisDev* __rest
             if (j < rest) absorb(P.pr[whole + j], cur[j]);
     }
     // every table prime is at least 2^18 below 2^30: four products leave 2^50 for what follows
-    const uint32_t v = vs >> 26;  // X = sum y_i Mhat_i - v M
+    const uint32_t v = (uint32_t)(vs >> (ANYX ? 32 : 26));  // X = sum y_i Mhat_i - v M
 #pragma unroll
     for (int w = 0; w < L; w++) x.c[w] += (uint64_t)v * P.B0[w];
     if (MODE == EPI_YASHE) {
@@ -1335,7 +1335,7 @@ __device__ __forceinline__ void epi_c_one(const Const& P, const BasisDev* __rest
     }
 }
 
-template <int L, int MODE, int K>
+template <int L, int MODE, int K, bool ANYX = false>
 __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<L, (K ? K : KMAX)> P,
                                                const BasisDev* __restrict__ B, const uint32_t* __restrict__ resid,
                                                void* __restrict__ out, int njobs, unsigned long long frac_limit,
@@ -1352,7 +1352,7 @@ __global__ void __launch_bounds__(256) k_epi_c(const __grid_constant__ EpiConst<
     dep_wait(r0);
     uint64_t* dst = reinterpret_cast<uint64_t*>(out) +
                     (MODE == EPI_DECRYPT ? (size_t)idx : (size_t)job * n * L64 + (lm ? (size_t)coef : (size_t)coef * L64));
-    epi_c_one<L, MODE, K, true>(P, B, r0, n, dst, lm ? (size_t)n : 1, frac_limit);
+    epi_c_one<L, MODE, K, true, ANYX>(P, B, r0, n, dst, lm ? (size_t)n : 1, frac_limit);
 }
 
 // Constants of a basis for k_epi_c (K = 0 or KS = K primes).
@@ -1362,7 +1362,8 @@ void fill_epi_const(const BasisDev& h, void* param) {
     EpiConst<L, KS>& c = *static_cast<EpiConst<L, KS>*>(param);
     for (int i = 0; i < h.k; i++) {
         EpiPrimeC<L>& e = c.pr[i];
-        e.p = h.p[i];
+        e.fhi = h.fhi[i];
+        e.flo = h.flo[i];
         e.np = 0u - h.p[i];
         e.ycon = h.ycon[i];
         e.ycon_sh = h.ycon_sh[i];

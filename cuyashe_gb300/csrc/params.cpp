@@ -333,10 +333,10 @@ cy_status build_basis(Basis& b, int device, int n, const BigUInt& q, int mode, c
     b.epi_param.assign(b.epi->param_bytes, 0);
     b.epi->fill(b.h, b.epi_param.data());
     const EpiConstKernel* any = epi_const_any(b.h.l32, b.h.mode);
-    std::vector<unsigned char> blob(any->param_bytes, 0);
-    any->fill(b.h, blob.data());
-    CY_CUDA(cudaMalloc(&b.d_epi, blob.size()));
-    CY_CUDA(cudaMemcpy(b.d_epi, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    b.any_param.assign(any->param_bytes, 0);
+    any->fill(b.h, b.any_param.data());
+    CY_CUDA(cudaMalloc(&b.d_epi, b.any_param.size()));
+    CY_CUDA(cudaMemcpy(b.d_epi, b.any_param.data(), b.any_param.size(), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMalloc(&b.d, sizeof(BasisDev)));
     CY_CUDA(cudaMemcpy(b.d, &b.h, sizeof(BasisDev), cudaMemcpyHostToDevice));
     CY_CUDA(cudaMalloc(&b.d_ninv, sizeof(uint32_t) * ninv.size()));
