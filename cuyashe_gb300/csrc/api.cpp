@@ -570,6 +570,16 @@ cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n,
     return CY_OK;
 }
 
+// Host memory that CUDA does not know, so that copies from and to it are synchronous.
+static bool is_pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
 }  // namespace cy
 
 using namespace cy;
@@ -679,10 +689,14 @@ cy_status cy_polymul(cy_ring* r, const uint64_t* d_a, const uint64_t* d_b, uint6
 cy_status cy_polymul_host(cy_ring* r, const uint64_t* h_a, const uint64_t* h_b, uint64_t* h_c, int batch) {
     CY_TRY(validate_poly_args(r, h_a, h_b, h_c, batch));
     if (batch == 0) return CY_OK;
-    const int jobs = std::min(batch, chunk_jobs(r->n, r->mul.h.k));
+    const int full = chunk_jobs(r->n, r->mul.h.k), jobs = std::min(batch, full);
     const KernelSet& ks = kernel_variant(
         r->mul.h.logn, tuned_variant(r->mul.h.logn, r->mul.h.l64, TUNE_MUL, (long long)jobs * r->mul.h.k));
-    const int chunk = product_chunk_jobs(r->mul, ks, false, jobs);
+    // A batch of less than a chunk is cut to whole waves too where the copies run beside the kernels
+    // (37 products at N = 4096, 250-bit q, as 25 and 12: 103 us, in one 125), but the call waits for each
+    // copy of pageable memory (the same: 196 us, in one 155).
+    const bool pageable = is_pageable(h_a) || is_pageable(h_b) || is_pageable(h_c);
+    const int chunk = product_chunk_jobs(r->mul, ks, false, pageable ? full : jobs);
     return run_host_pipeline((size_t)r->n * r->l64, batch, chunk, h_a, h_b, h_c,
                              [r](cy_workspace* ws, const uint64_t* a, const uint64_t* b, uint64_t* c, int nj,
                                  cudaStream_t st) { return cy_polymul_ws(r, ws, a, b, c, nj, st); });
