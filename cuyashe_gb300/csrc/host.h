@@ -53,7 +53,7 @@ const std::vector<uint32_t>& table_primes();  // host-only, no CUDA
 // ---- a CRT basis for one ring and one epilogue ------------------------------
 struct Basis {
     BasisDev h{};
-    BasisDev* d = nullptr;
+    BasisDev* d = nullptr;  // one allocation with d_epi and d_ninv
     ProdParams prod{};  // first parameter of the product and keyswitch kernels
     NttParams ntt{};    // and of the standalone transforms
     uint32_t* d_ninv = nullptr;  // [k][4]: N^-1 mod p_i, N^-1 psi_i^-(NMAX/2), each with its Shoup companion
