@@ -504,70 +504,50 @@ cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* e
     return run_keyswitch(B, c, evk, ell, out, batch, ws, st, variant, chunk_k, lm);
 }
 
-// The transform of the polynomial at d_poly ([N][l64] limbs) for k_mul_key with basis B:
-// *d_key [k][N], allocated on the first call. N < 1024 has no such kernel: null. On the
-// legacy default stream; the caller synchronises. up: for products with a small operand.
-cy_status prepare_key(const Basis& B, const uint64_t* d_poly, uint32_t** d_key, int up) {
-    if (!key_kernel(B.h.logn, B.h.l64)) return CY_OK;
-    long long total = (long long)B.h.k * B.h.n;
-    if (!*d_key) CY_CUDA(cudaMalloc(d_key, sizeof(uint32_t) * total));
-    uint32_t* res = nullptr;
-    CY_CUDA(cudaMalloc(&res, sizeof(uint32_t) * total));
-    cy_status st = run_crt(B, d_poly, res, nullptr, 1, 0);
-    if (st == CY_OK) st = run_ntt(B, res, 1, false, 0);
+// The transforms of `count` residue polynomials [count][k][N] in d_res (overwritten), in the order of
+// key_index: times 2^32 (up: keyswitch keys, kept operands of products with a small one) or 2^-32.
+// On the legacy default stream.
+static cy_status key_transforms(const Basis& B, uint32_t* d_res, int count, uint32_t* d_out, int up) {
+    CY_TRY(run_ntt(B, d_res, count, false, 0));
     const BasisDev* Bd = B.d;
-    void* args[] = {(void*)&Bd, (void*)&res, (void*)d_key, (void*)&total, (void*)&up};
-    if (st == CY_OK)
-        st = launch(evk_mont_kernel(), "key_mont", B.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0, args);
-    cudaFree(res);  // waits for the kernels
-    return st;
+    long long total = (long long)count * B.h.k * B.h.n;
+    void* args[] = {(void*)&Bd, (void*)&d_res, (void*)&d_out, (void*)&total, (void*)&up};
+    return launch(evk_mont_kernel(), "key_mont", B.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0, args);
 }
 
-// Evaluation key in the keyswitch basis, NTT domain, in Montgomery form: d_evk
-// [ell][k][N] (key_index) of value 2^32 mod p (the keyswitch sums products with the digits in 64
+bool has_key_kernel(const Basis& B) { return key_kernel(B.h.logn, B.h.l64) != nullptr; }
+
+// Evaluation key in the keyswitch basis, NTT domain, in Montgomery form: [ell][k][N]
+// (key_index) of value 2^32 mod p (the keyswitch sums products with the digits in 64
 // bits and reduces once); at N = ROWS_N a second copy laid out by lane follows it
-// (the 64-coefficient keyswitch reads that one). Synchronous.
-cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint32_t** d_evk) {
-    const int k = relin.h.k;
-    const size_t words = (size_t)ell * k * n;
-    const bool rows = relin.h.logn == ROWS_LOGN;
-    uint64_t* d_limbs = nullptr;
-    uint32_t* d_res = nullptr;
-    uint32_t* out = nullptr;
-    cudaError_t e = cudaMalloc(&d_limbs, sizeof(uint64_t) * (size_t)ell * n * l64);
-    if (e == cudaSuccess) e = cudaMalloc(&d_res, sizeof(uint32_t) * words);
-    if (e == cudaSuccess) e = cudaMalloc(&out, sizeof(uint32_t) * words * (rows ? 2 : 1));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(d_limbs, h_evk, sizeof(uint64_t) * (size_t)ell * n * l64, cudaMemcpyHostToDevice);
-    cy_status st = (e == cudaSuccess) ? CY_OK : cuda_error(e, "evaluation key upload");
-    if (st == CY_OK) st = run_crt(relin, d_limbs, d_res, nullptr, ell, 0);
-    if (st == CY_OK) st = run_ntt(relin, d_res, ell, false, 0);
-    if (st == CY_OK) {
-        const BasisDev* Bd = relin.d;
-        long long total = (long long)words;
-        int up = 1;
-        void* args[] = {(void*)&Bd, (void*)&d_res, (void*)&out, (void*)&total, (void*)&up};
-        st = launch(evk_mont_kernel(), "evk_mont", relin.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256),
-                    0, 0, args);
-        if (st == CY_OK && rows) {
-            uint32_t* out_rows = out + words;
-            void* rargs[] = {(void*)&out, (void*)&out_rows, (void*)&total};
-            st = launch(evk_rows_kernel(), "evk_rows", relin.h.logn, dim3((unsigned)((total + 255) / 256)),
-                        dim3(256), 0, 0, rargs);
-        }
-    }
-    if (st == CY_OK) {
-        e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) st = cuda_error(e, "evaluation key transform");
-    }
-    cudaFree(d_limbs);
-    cudaFree(d_res);
-    if (st != CY_OK) {
-        cudaFree(out);
-        return st;
-    }
-    *d_evk = out;
-    return CY_OK;
+// (the 64-coefficient keyswitch reads that one).
+size_t evk_words(const Basis& relin, int ell) {
+    return (size_t)ell * relin.h.k * relin.h.n * (relin.h.logn == ROWS_LOGN ? 2 : 1);
+}
+
+// Keys installed by one pass of transforms: the evaluation key at d_limbs ([ell][N][l64]) into d_evk;
+// with h (null: none), the kept transform of the public key into the words before d_evk, so that it is
+// transformed with the evaluation key. d_res: (ell + 1) k N words of scratch. On the legacy default stream.
+cy_status prepare_evk(const Basis& relin, const uint64_t* d_h, const uint64_t* d_limbs, int ell, uint32_t* d_res,
+                      uint32_t* d_evk) {
+    const size_t poly = (size_t)relin.h.k * relin.h.n;
+    if (d_h) CY_TRY(run_crt(relin, d_h, d_res, nullptr, 1, 0));
+    CY_TRY(run_crt(relin, d_limbs, d_res + (d_h ? poly : 0), nullptr, ell, 0));
+    CY_TRY(key_transforms(relin, d_res, ell + (d_h ? 1 : 0), d_evk - (d_h ? poly : 0), 1));
+    if (relin.h.logn != ROWS_LOGN) return CY_OK;
+    long long total = (long long)(ell * poly);
+    const uint32_t* in = d_evk;
+    uint32_t* rows = d_evk + total;
+    void* args[] = {(void*)&in, (void*)&rows, (void*)&total};
+    return launch(evk_rows_kernel(), "evk_rows", relin.h.logn, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, 0,
+                  args);
+}
+
+// The kept transforms of `count` polynomials at d_polys ([count][N][l64]) for products with basis B
+// (k_mul_key): d_keys [count][k][N]; d_res: as many words of scratch. On the legacy default stream.
+cy_status prepare_keys(const Basis& B, const uint64_t* d_polys, int count, uint32_t* d_res, uint32_t* d_keys) {
+    CY_TRY(run_crt(B, d_polys, d_res, nullptr, count, 0));
+    return key_transforms(B, d_res, count, d_keys, 0);
 }
 
 // Host memory that CUDA does not know, so that copies from and to it are synchronous.

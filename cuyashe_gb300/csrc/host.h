@@ -157,15 +157,17 @@ struct cy_yashe {
     cy::Basis dec;     // key * ciphertext, decryption epilogue
     bool has_keys = false;
     std::vector<uint64_t> h_f, h_h, h_evk;
+    // The installed keys, in one allocation made with the first keys and rewritten by later ones: limbs of
+    // f, f^2 and h, the kept transforms of f and f^2 (decryption basis) and of h (keyswitch basis, for
+    // products with a small s; k_mul_key, null for N < 1024), the evaluation key.
+    void* d_keys = nullptr;
     uint64_t* d_f = nullptr;
     uint64_t* d_f2 = nullptr;
     uint64_t* d_h = nullptr;    // public key (GPU encryption)
-    uint32_t* d_evk = nullptr;  // [ell][k'][N] NTT-domain evaluation key times 2^32
-    // transforms of h, f and f^2 for products with a batch (k_mul_key; null for N < 1024); h's in
-    // the keyswitch basis, for products with a small s
-    uint32_t* d_h_key = nullptr;
     uint32_t* d_f_key = nullptr;
     uint32_t* d_f2_key = nullptr;
+    uint32_t* d_h_key = nullptr;
+    uint32_t* d_evk = nullptr;  // [ell][k'][N] NTT-domain evaluation key times 2^32
     uint64_t* d_cdt = nullptr;  // discrete Gaussian thresholds (GPU sampling)
     int n_cdt = 0;
     ~cy_yashe();

@@ -331,7 +331,7 @@ cy_status cy_mixed_plan_create(const cy_mixed_job* jobs, int njobs, cy_mixed_pla
         if (!mixable(r))
             return set_error(CY_ERR_UNSUPPORTED, "mixed plans take N = 1024..8192 and q of up to 192 bits (job " +
                                                      std::to_string(i) + ")");
-        if (q.yashe && q.relin && !q.yashe->d_evk) return set_error(CY_ERR_NO_KEYS, "YASHE job without keys");
+        if (q.yashe && q.relin && !q.yashe->has_keys) return set_error(CY_ERR_NO_KEYS, "YASHE job without keys");
         MixedJob J = q.ring ? product_job(q.ring, q.d_a, q.d_b, q.d_c)
                             : yashe_job(q.yashe, q.d_a, q.d_b, q.d_c, q.relin != 0);
         P->jobs.push_back(J);

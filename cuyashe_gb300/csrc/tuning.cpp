@@ -32,7 +32,9 @@ cy_status run_product_api(const Basis& B, bool centered, const uint64_t* a, long
                           cudaStream_t st, int variant, const uint32_t* key = nullptr, bool small = false);
 cy_status run_keyswitch_api(const Basis& B, const uint64_t* c, const uint32_t* evk, int ell, uint64_t* out, int batch,
                             Workspace& ws, cudaStream_t st, int variant, int chunk_k, int lm);
-cy_status prepare_evk(const Basis& relin, const uint64_t* h_evk, int ell, int n, int l64, uint32_t** d_evk);
+size_t evk_words(const Basis& relin, int ell);
+cy_status prepare_evk(const Basis& relin, const uint64_t* d_h, const uint64_t* d_limbs, int ell, uint32_t* d_res,
+                      uint32_t* d_evk);
 
 cy_status run_ntt_api(const Basis& B, uint32_t* res, int batch, bool inverse, cudaStream_t st, int variant);
 cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
@@ -298,15 +300,18 @@ cy_status cy_yashe_autotune(cy_yashe* y, int batch, cy_stream_t stream) {
     CY_TRY(tune_product(r->mul, false, batch, st));
     CY_TRY(tune_product(y->tensor, true, batch, st));
     const uint32_t* evk = y->d_evk;
-    uint32_t* tmp = nullptr;
-    if (!evk) {  // no keys yet: an evaluation key of random values has the same cost
+    DevBuf tmp, limbs, res;
+    if (!y->has_keys) {  // an evaluation key of random values has the same cost
         std::vector<uint64_t> h = random_polys(y->ell, r->n, r->l64, r->qbits, 4);
-        CY_TRY(prepare_evk(y->relin, h.data(), y->ell, r->n, r->l64, &tmp));
-        evk = tmp;
+        CY_CUDA(cudaMalloc(&limbs.p, h.size() * sizeof(uint64_t)));
+        CY_CUDA(cudaMalloc(&res.p, (size_t)y->ell * y->relin.h.k * r->n * sizeof(uint32_t)));
+        CY_CUDA(cudaMalloc(&tmp.p, evk_words(y->relin, y->ell) * sizeof(uint32_t)));
+        CY_CUDA(cudaMemcpy(limbs.p, h.data(), h.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+        CY_TRY(prepare_evk(y->relin, nullptr, (const uint64_t*)limbs.p, y->ell, (uint32_t*)res.p, (uint32_t*)tmp.p));
+        CY_CUDA(cudaDeviceSynchronize());
+        evk = static_cast<const uint32_t*>(tmp.p);
     }
-    cy_status s = tune_keyswitch(y, evk, batch, st);
-    if (tmp) cudaFree(tmp);
-    return s;
+    return tune_keyswitch(y, evk, batch, st);
 }
 
 cy_status cy_tuning_export(char* buf, size_t len, size_t* needed) {
