@@ -516,18 +516,19 @@ def time_steps(fn, steps: int, stream):
     return start.elapsed_time(end)
 
 
-def kernel_counts(tuning: str) -> dict:
+def kernel_counts() -> dict:
     """Warp instructions and DRAM bytes per job of the kernels of the headline
-    step, for the schedules in `tuning` (cy_tuning_export), from the committed ncu
+    step, for the schedules that its launches run (cy_tuning_schedule), from the committed ncu
     summary profiles/kernel_counts_n4096.json; {} when it has no such entry."""
+    import cuyashe_gb300 as cy
+
     path = os.path.join(ROOT, "profiles", "kernel_counts_n4096.json")
     if not os.path.exists(path):
         return {}
     per = json.load(open(path))["per_unit"]
-    tuned = dict(item.split("=") for item in tuning.split(";") if item.startswith("n4096.l2."))
     out = {}
     for name, op in (("mul_centered", "mulc"), ("keyswitch", "ks"), ("mul", "mul")):
-        key = "%s=%s" % (op, tuned.get("n4096.l2." + op, "0"))
+        key = "%s=%d" % (op, cy.tuning_schedule(N, L, op, 1 << 20))  # launches of many waves
         if key in per:
             out[name] = dict(per[key], source=key)
     for name in ("epi_yashe", "epi_modq"):
@@ -662,7 +663,7 @@ def run_ours(args):
     top_bytes = kernel_bytes(top, kernels[top]["launches"], B, info.tensor_primes, info.relin_primes, info.ell)
     top_gbs = top_bytes / (kernels[top]["ms"] / 1000.0) / 1e9
     # measured counts per job of the schedule each kernel ran with (ncu, committed summary)
-    counts = kernel_counts(tuning)
+    counts = kernel_counts()
     traffic = None
     top_counts = counts.get(top.split("_n")[0])
     if top_counts:

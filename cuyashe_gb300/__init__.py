@@ -183,6 +183,7 @@ SIGNATURES = {
     "cy_yashe_autotune": ([_vp, _i, _vp], _i),
     "cy_tuning_export": ([ctypes.c_char_p, ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)], _i),
     "cy_tuning_import": ([ctypes.c_char_p], _i),
+    "cy_tuning_schedule": ([_i, _i, ctypes.c_char_p, ctypes.c_longlong, ctypes.POINTER(_i)], _i),
     "cy_set_epilogue_exact": ([_i], _i),
     "cy_set_epilogue_generic": ([_i], _i),
     "cy_set_chunk_overlap": ([_i], _i),
@@ -251,6 +252,13 @@ def tuning_export() -> str:
 
 def tuning_import(spec: str) -> None:
     check(lib().cy_tuning_import(spec.encode()), "cy_tuning_import")
+
+
+def tuning_schedule(n: int, limbs: int, op: str, blocks: int) -> int:
+    """Number of the schedule that a call of `blocks` transforms runs."""
+    out = ctypes.c_int(0)
+    check(lib().cy_tuning_schedule(n, limbs, op.encode(), blocks, ctypes.byref(out)), "cy_tuning_schedule")
+    return out.value
 
 
 def launch_count() -> int:

@@ -177,7 +177,7 @@ static cy_status check_device(int device) {
     return CY_OK;
 }
 
-int tuned_variant(int logn, int l64, int op, long long blocks);
+int tuned_variant(int logn, int l64, int op, long long blocks, int number = -1);
 cy_status run_mixed(const std::vector<const cy_polymul_job*>& jobs, cudaStream_t st);
 cy_status mixed_status(cudaStream_t st);
 bool mixed_supported(const cy_ring* r);
@@ -280,7 +280,7 @@ static int product_chunk_jobs(const Basis& B, const KernelSet& ks, bool centered
 }
 
 // products of `batch` jobs with basis B: out_j = epilogue(a_j * b_j); `variant`
-// selects the NTT schedule (-1: the tuned one for this device and size). key: the kept
+// is the number of the NTT schedule (-1: the tuned one for this device and size). key: the kept
 // transform of a (a_stride = 0), used from two products on (a block takes two) where there is a
 // kernel for it; small: b's jobs are small signed words at the start of their rows (L64 = 0 of
 // k_mul_key, any number of products)
@@ -315,8 +315,7 @@ static cy_status run_product(const Basis& B, bool centered, const uint64_t* a, l
     }
     const int n = B.h.n, k = B.h.k, jobs = std::min(batch, chunk_jobs(n, k));
     const KernelSet& ks = kernel_variant(
-        B.h.logn, variant >= 0 ? variant
-                               : tuned_variant(B.h.logn, B.h.l64, centered ? TUNE_MULC : TUNE_MUL, (long long)jobs * k));
+        B.h.logn, tuned_variant(B.h.logn, B.h.l64, centered ? TUNE_MULC : TUNE_MUL, (long long)jobs * k, variant));
     const int chunk = product_chunk_jobs(B, ks, centered, jobs);
     const int nchunks = (batch + chunk - 1) / chunk;
     Lanes L;
@@ -341,8 +340,8 @@ static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint32_t
     if (batch == 0) return CY_OK;
     const int n = B.h.n, k = B.h.k, l64 = B.h.l64;
     const int jobs = std::min(batch, chunk_jobs(n, chunk_k > 0 ? std::max(k, chunk_k) : k));
-    const KernelSet& ks = kernel_variant(
-        B.h.logn, variant >= 0 ? variant : tuned_variant(B.h.logn, B.h.l64, TUNE_KS, (long long)jobs * k));
+    const KernelSet& ks =
+        kernel_variant(B.h.logn, tuned_variant(B.h.logn, B.h.l64, TUNE_KS, (long long)jobs * k, variant));
     int sel = 0;
     CY_TRY(keyswitch_digits_per_pass(ks, ell, &sel));
     const int chunk = wave_chunk(jobs, ks.ks_for(l64, sel), ks.threads, ks.smem_ks[sel], k * ks.blocks_per_prime);
@@ -361,7 +360,7 @@ static cy_status run_keyswitch(const Basis& B, const uint64_t* c, const uint32_t
 // The HE multiply of `batch` pairs: per chunk, the tensor product with the
 // YASHE rounding into out, then (relin) its keyswitch in place; chunks go round
 // the lanes.
-// ks_variant >= 0 forces the keyswitch schedule (the autotuner's timing runs).
+// ks_variant >= 0: the keyswitch schedule of that number (the autotuner's timing runs).
 cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t* evk, int ell, const uint64_t* c1,
                         const uint64_t* c2, uint64_t* out, int batch, bool do_relin, Workspace& ws, cudaStream_t st,
                         int ks_variant) {
@@ -371,10 +370,8 @@ cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t*
     int chunk = std::min(batch, chunk_jobs(n, kmax));
     const KernelSet& kt = kernel_variant(
         tensor.h.logn, tuned_variant(tensor.h.logn, l64, TUNE_MULC, (long long)chunk * tensor.h.k));
-    const KernelSet& kr =
-        kernel_variant(relin.h.logn, ks_variant >= 0 ? ks_variant
-                                                     : tuned_variant(relin.h.logn, l64, TUNE_KS,
-                                                                     (long long)chunk * relin.h.k));
+    const KernelSet& kr = kernel_variant(
+        relin.h.logn, tuned_variant(relin.h.logn, l64, TUNE_KS, (long long)chunk * relin.h.k, ks_variant));
     int sel = 0;
     if (do_relin) CY_TRY(keyswitch_digits_per_pass(kr, ell, &sel));
     if (do_relin)  // whole waves of the keyswitch
@@ -414,9 +411,8 @@ static cy_status run_crt(const Basis& B, const uint64_t* x, uint32_t* res, const
 static cy_status run_ntt(const Basis& B, uint32_t* res, int batch, bool inverse, cudaStream_t st,
                          int variant = -1) {
     if (batch == 0) return CY_OK;
-    const KernelSet& ks =
-        kernel_variant(B.h.logn, variant >= 0 ? variant
-                                              : tuned_variant(B.h.logn, B.h.l64, TUNE_NTT, (long long)batch * B.h.k));
+    const KernelSet& ks = kernel_variant(
+        B.h.logn, tuned_variant(B.h.logn, B.h.l64, TUNE_NTT, (long long)batch * B.h.k, variant));
     const uint32_t* ninv = B.d_ninv;
     const long long rows = (long long)batch * B.h.k * (B.h.n / 64);
     if (inverse && ks.intt_tma && B.h.logn == 12 && ntt_tma_usable(res, rows)) {  // input tiles by TMA

@@ -24,8 +24,8 @@ struct KernelSet {
 
 // Kernel sets for transforms of length 2^logn (1 <= logn <= LOGN_MAX). Each
 // length has one or more schedules ("variants": coefficients per thread, hence
-// threads per transform and passes); the autotuner may pick one per ring, else
-// default_variant does (tuning.cpp).
+// threads per transform and passes). Set v is schedule number v for v > 0, and number 0 is the
+// default rule (tuning.cpp), so set 0 has a second number.
 int variant_count(int logn);
 const KernelSet& kernel_variant(int logn, int v);
 

@@ -61,7 +61,8 @@ static const VariantTable& variants() {
         add(13, fill_n13_e4r);
         add(14, fill_n14_e5);
         // numbers 4 .. 6 at N = 4096 and 3 at N = 8192 differed from earlier ones only by their
-        // exchange regions; saved choices keep their numbers
+        // exchange regions; saved choices keep their numbers. (A choice of number 0 is the default
+        // rule; 5 and 3, and the last ones below, choose the first set itself.)
         add(12, fill_n12_e4r);
         add(12, fill_n12_e3);
         add(12, fill_n12_e4);
@@ -76,6 +77,9 @@ static const VariantTable& variants() {
             fill_n14_pair(ks);
             T.v[14].push_back(ks);
         }
+        add(10, fill_n10_e3);
+        add(11, fill_n11_e3);
+        add(14, fill_n14_e4);
     });
     return T;
 }

@@ -6,7 +6,7 @@
 // operation on a synthetic batch of the caller's ring, checks that its output is
 // bit-identical to the default schedule's, times it with CUDA events and keeps
 // the fastest. Choices live in a process-wide table and can be exported and
-// imported as text ("n4096.l2.mul=1;n4096.l2.ks=0;...") so that a serving
+// imported as text ("n4096.l2.mul=1;n4096.l2.ks=0;...", 0 for the default) so that a serving
 // process tunes once. The reference has a single fixed launch shape per kernel
 // (e.g. src/cuda_functions.cu:447-458) and commented-out block-size notes
 // (src/cuda_bn.cu:983-988, 1014-1019).
@@ -96,16 +96,31 @@ int default_variant(int logn, int l64, int op, long long blocks) {
     }
 }
 
-// The autotuner's (or an imported) choice, else the default for `blocks`.
-int tuned_variant(int logn, int l64, int op, long long blocks) {
+// The kernel set of schedule `number`: 0 is the default rule for a call of `blocks`, and a negative
+// number the autotuner's (or an imported) choice, the default where there is none.
+int tuned_variant(int logn, int l64, int op, long long blocks, int number) {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    {
+    if (number < 0) {
+        number = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return 0;
         std::lock_guard<std::mutex> lock(g_mu);
         auto it = g_choice.find(std::make_tuple(dev, logn, l64, op));
-        if (it != g_choice.end()) return it->second;
+        if (it != g_choice.end()) number = it->second;
     }
-    return default_variant(logn, l64, op, blocks);
+    return number > 0 ? number : default_variant(logn, l64, op, blocks);
+}
+
+// A schedule number that always runs kernel set v.
+static int number_of(int logn, int v) {
+    if (v > 0) return v;
+    switch (logn) {  // set 0's second number (k_misc.cu)
+        case 10: return 2;
+        case 11: return 2;
+        case 12: return 5;
+        case 13: return 3;
+        case 14: return 4;
+        default: return 0;
+    }
 }
 
 static void set_choice(int dev, int logn, int l64, int op, int v) {
@@ -333,6 +348,21 @@ cy_status cy_tuning_export(char* buf, size_t len, size_t* needed) {
         buf[len - 1] = 0;
         if (len < s.size() + 1) return set_error(CY_ERR_INVALID_ARGUMENT, "buffer too small");
     }
+    return CY_OK;
+}
+
+cy_status cy_tuning_schedule(int n, int q_limbs, const char* op, long long blocks, int* schedule) {
+    if (!op || !schedule || blocks < 0) return set_error(CY_ERR_INVALID_ARGUMENT, "bad argument");
+    int logn = 0;
+    while (logn < LOGN_MAX && (1 << logn) < n) logn++;
+    int o = -1;
+    for (int i = 0; i < TUNE_OPS; i++)
+        if (std::strcmp(op, kOpNames[i]) == 0) o = i;
+    if ((1 << logn) != n || logn < 1 || o < 0 || q_limbs < 1 || q_limbs > 6)
+        return set_error(CY_ERR_INVALID_ARGUMENT, "no such operation");
+    int dev = 0;
+    CY_CUDA(cudaGetDevice(&dev));
+    *schedule = number_of(logn, tuned_variant(logn, q_limbs, o, blocks, -1));
     return CY_OK;
 }
 

@@ -503,11 +503,13 @@ cy_status cy_graph_destroy(cy_graph *graph);
 /* Schedule autotuning                                                        */
 /* ------------------------------------------------------------------------ */
 
-/* Each transform length is compiled with one or more NTT schedules (8 or 16
- * coefficients per thread: 512 or 256 threads per transform and 4 or 3
- * register passes at N = 4096). cy_ring_autotune runs every schedule of the
+/* Each transform length is compiled with one or more NTT schedules (8 to 64
+ * coefficients per thread: 512 to 64 threads per transform and 4 to 2
+ * register passes at N = 4096). Unless one is chosen, a call runs the one that
+ * measured fastest for its N, limb count and number of blocks (number 0, the
+ * default). cy_ring_autotune runs every schedule of the
  * ring's product on `batch` synthetic jobs, requires each output to equal the
- * default schedule's bit for bit, and keeps the fastest for this device, N and
+ * default's bit for bit, and keeps the fastest for this device, N and
  * limb count; cy_yashe_autotune does the same for the plain product, the YASHE
  * tensor and the keyswitch. Synchronous; allocates its test buffers. The
  * reference has one fixed launch shape per kernel (src/cuda_functions.cu:447-458)
@@ -516,9 +518,15 @@ cy_status cy_ring_autotune(cy_ring *ring, int batch, cy_stream_t stream);
 cy_status cy_yashe_autotune(cy_yashe *y, int batch, cy_stream_t stream);
 
 /* The current device's choices as text, e.g. "n4096.l2.mul=1;n4096.l2.ks=0;"
- * (*needed gets the size including the terminator), and back. */
+ * (*needed gets the size including the terminator), and back. 0 gives an
+ * operation back to the default. */
 cy_status cy_tuning_export(char *buf, size_t len, size_t *needed);
 cy_status cy_tuning_import(const char *spec);
+/* The schedule that a call of operation `op` ("mul", "mulc", "ks" or "ntt") on
+ * the current device runs whose launch has `blocks` transforms (jobs times
+ * primes; at most those of one chunk of the scratch), as a number that
+ * cy_tuning_import takes. */
+cy_status cy_tuning_schedule(int n, int q_limbs, const char *op, long long blocks, int *schedule);
 
 /* ------------------------------------------------------------------------ */
 /* Observability                                                              */
