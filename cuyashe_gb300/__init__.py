@@ -242,7 +242,7 @@ def limbs_of(x: int, n: int):
 
 
 def tuning_export() -> str:
-    """The autotuner's choices for the current device ("n4096.l2.mul=1;...")."""
+    """The autotuner's choices for the current device ("n4096.l2.mul=1@8;...")."""
     need = ctypes.c_size_t(0)
     check(lib().cy_tuning_export(None, 0, ctypes.byref(need)), "cy_tuning_export")
     buf = ctypes.create_string_buffer(need.value + 1)

@@ -5,9 +5,10 @@
 // 4 or 3 register passes at N = 4096). The autotuner runs each schedule of an
 // operation on a synthetic batch of the caller's ring, checks that its output is
 // bit-identical to the default schedule's, times it with CUDA events and keeps
-// the fastest. Choices live in a process-wide table and can be exported and
-// imported as text ("n4096.l2.mul=1;n4096.l2.ks=0;...", 0 for the default) so that a serving
-// process tunes once. The reference has a single fixed launch shape per kernel
+// the fastest, for calls of the same regime (the default rule depends on the call's size). Choices live
+// in a process-wide table and can be exported and
+// imported as text ("n4096.l2.mul=1@8;n4096.l2.ks=0;...": 0 for the default, @8 for calls whose default is
+// schedule 8) so that a serving process tunes once. The reference has a single fixed launch shape per kernel
 // (e.g. src/cuda_functions.cu:447-458) and commented-out block-size notes
 // (src/cuda_bn.cu:983-988, 1014-1019).
 #include <cuda_runtime.h>
@@ -44,7 +45,11 @@ cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t*
 static const char* kOpNames[TUNE_OPS] = {"mul", "mulc", "ks", "ntt"};
 
 static std::mutex g_mu;
-static std::map<std::tuple<int, int, int, int>, int> g_choice;  // (device, logn, l64, op) -> variant
+// (device, logn, l64, op, rule) -> schedule number. A choice that was measured holds where the default
+// rule takes the same kernel set `rule` as at the measured size: another regime (a single call after a batch
+// was tuned) keeps its default. With 16384 x 380 bits tuned on a batch, a single product takes 27 us, 40 with
+// the batch's schedule. rule = -1: for all sizes (an import that names no rule).
+static std::map<std::tuple<int, int, int, int, int>, int> g_choice;
 
 // SMs of the current device (the GB300's 152 if it cannot be queried).
 static int sm_count() {
@@ -99,15 +104,15 @@ int default_variant(int logn, int l64, int op, long long blocks) {
 // The kernel set of schedule `number`: 0 is the default rule for a call of `blocks`, and a negative
 // number the autotuner's (or an imported) choice, the default where there is none.
 int tuned_variant(int logn, int l64, int op, long long blocks, int number) {
+    const int rule = default_variant(logn, l64, op, blocks);
     int dev = 0;
-    if (number < 0) {
-        number = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (number < 0 && cudaGetDevice(&dev) == cudaSuccess) {
         std::lock_guard<std::mutex> lock(g_mu);
-        auto it = g_choice.find(std::make_tuple(dev, logn, l64, op));
+        auto it = g_choice.find(std::make_tuple(dev, logn, l64, op, rule));
+        if (it == g_choice.end()) it = g_choice.find(std::make_tuple(dev, logn, l64, op, -1));
         if (it != g_choice.end()) number = it->second;
     }
-    return number > 0 ? number : default_variant(logn, l64, op, blocks);
+    return number > 0 ? number : rule;
 }
 
 // A schedule number that always runs kernel set v.
@@ -123,9 +128,13 @@ static int number_of(int logn, int v) {
     }
 }
 
-static void set_choice(int dev, int logn, int l64, int op, int v) {
+static void set_choice(int dev, int logn, int l64, int op, int rule, int number) {
     std::lock_guard<std::mutex> lock(g_mu);
-    g_choice[std::make_tuple(dev, logn, l64, op)] = v;
+    if (rule < 0) {  // for all sizes: nothing else stands
+        auto it = g_choice.lower_bound(std::make_tuple(dev, logn, l64, op, -1));
+        while (it != g_choice.end() && it->first < std::make_tuple(dev, logn, l64, op + 1, -1)) it = g_choice.erase(it);
+    }
+    g_choice[std::make_tuple(dev, logn, l64, op, rule)] = number;
 }
 
 // values < q: random words below the top bit of q
@@ -155,15 +164,15 @@ struct DevBuf {
     }
 };
 
-// Time each schedule of one operation; `run(v, out)` launches it on `st`.
+// Time each schedule of one operation at `blocks` transforms per launch; `run(v, out)` launches it on `st`.
 template <class Run>
-static cy_status tune_op(int logn, int l64, int op, size_t out_bytes, cudaStream_t st, Run run, int* chosen) {
+static cy_status tune_op(int logn, int l64, int op, long long blocks, size_t out_bytes, cudaStream_t st, Run run) {
     const int nv = variant_count(logn);
     int dev = 0;
     CY_CUDA(cudaGetDevice(&dev));
-    *chosen = 0;
+    const int rule = default_variant(logn, l64, op, blocks);
     if (nv <= 1) {
-        set_choice(dev, logn, l64, op, 0);
+        set_choice(dev, logn, l64, op, rule, 0);
         return CY_OK;
     }
     DevBuf ref, cur, flag;
@@ -214,8 +223,7 @@ static cy_status tune_op(int logn, int l64, int op, size_t out_bytes, cudaStream
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (st_all != CY_OK) return st_all;
-    set_choice(dev, logn, l64, op, best_v);
-    *chosen = best_v;
+    set_choice(dev, logn, l64, op, rule, best_v);
     return CY_OK;
 }
 
@@ -233,13 +241,12 @@ static cy_status tune_product(const Basis& B, bool centered, int batch, cudaStre
     const long long stride = (long long)n * l64;
     const long long ostride = B.h.mode == EPI_DECRYPT ? n : stride;
     const size_t obytes = sizeof(uint64_t) * (size_t)batch * ostride;
-    int chosen = 0;
-    return tune_op(B.h.logn, l64, centered ? TUNE_MULC : TUNE_MUL, obytes, st,
+    const long long blocks = (long long)std::min(batch, chunk_jobs(n, B.h.k)) * B.h.k;
+    return tune_op(B.h.logn, l64, centered ? TUNE_MULC : TUNE_MUL, blocks, obytes, st,
                    [&](int v, void* out) {
                        return run_product_api(B, centered, (const uint64_t*)a.p, stride, (const uint64_t*)b.p, stride,
                                               out, ostride, batch, ws, st, v);
-                   },
-                   &chosen);
+                   });
 }
 
 // The keyswitch schedule is chosen inside the HE multiply it serves: each schedule
@@ -259,13 +266,13 @@ static cy_status tune_keyswitch(const cy_yashe* y, const uint32_t* evk, int batc
     CY_CUDA(cudaMemcpy(c2.p, h2.data(), bytes, cudaMemcpyHostToDevice));
     Workspace ws;
     CY_CUDA(cudaGetDevice(&ws.device));
-    int chosen = 0;
-    return tune_op(y->relin.h.logn, l64, TUNE_KS, bytes, st,
+    const long long blocks =
+        (long long)std::min(batch, chunk_jobs(n, std::max(y->tensor.h.k, y->relin.h.k))) * y->relin.h.k;
+    return tune_op(y->relin.h.logn, l64, TUNE_KS, blocks, bytes, st,
                    [&](int v, void* out) {
                        return run_yashe_mul(y->tensor, y->relin, evk, y->ell, (const uint64_t*)c1.p,
                                             (const uint64_t*)c2.p, (uint64_t*)out, batch, true, ws, st, v);
-                   },
-                   &chosen);
+                   });
 }
 
 // The standalone transforms (cy_ntt) of `batch` residue vectors, inverse then
@@ -282,16 +289,14 @@ static cy_status tune_ntt(const Basis& B, int batch, cudaStream_t st) {
     DevBuf src;
     CY_CUDA(cudaMalloc(&src.p, words * sizeof(uint32_t)));
     CY_CUDA(cudaMemcpy(src.p, h.data(), words * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    int chosen = 0;
-    return tune_op(B.h.logn, B.h.l64, TUNE_NTT, words * sizeof(uint32_t), st,
+    return tune_op(B.h.logn, B.h.l64, TUNE_NTT, (long long)batch * B.h.k, words * sizeof(uint32_t), st,
                    [&](int v, void* out) {
                        cudaError_t e = cudaMemcpyAsync(out, src.p, words * sizeof(uint32_t),
                                                        cudaMemcpyDeviceToDevice, st);
                        if (e != cudaSuccess) return cuda_error(e, "autotune copy");
                        CY_TRY(run_ntt_api(B, (uint32_t*)out, batch, true, st, v));
                        return run_ntt_api(B, (uint32_t*)out, batch, false, st, v);
-                   },
-                   &chosen);
+                   });
 }
 
 }  // namespace cy
@@ -338,7 +343,9 @@ cy_status cy_tuning_export(char* buf, size_t len, size_t* needed) {
         for (const auto& kv : g_choice) {
             if (std::get<0>(kv.first) != dev) continue;
             os << "n" << (1 << std::get<1>(kv.first)) << ".l" << std::get<2>(kv.first) << "."
-               << kOpNames[std::get<3>(kv.first)] << "=" << kv.second << ";";
+               << kOpNames[std::get<3>(kv.first)] << "=" << kv.second;
+            if (std::get<4>(kv.first) >= 0) os << "@" << number_of(std::get<1>(kv.first), std::get<4>(kv.first));
+            os << ";";
         }
     }
     const std::string s = os.str();
@@ -378,9 +385,10 @@ cy_status cy_tuning_import(const char* spec) {
         const std::string item = s.substr(pos, end - pos);
         pos = end + 1;
         if (item.empty()) continue;
-        int n = 0, l64 = 0, v = 0;
+        int n = 0, l64 = 0, v = 0, where = 0;
         char op[8] = {0};
-        if (std::sscanf(item.c_str(), "n%d.l%d.%7[a-z]=%d", &n, &l64, op, &v) != 4)
+        const int fields = std::sscanf(item.c_str(), "n%d.l%d.%7[a-z]=%d@%d", &n, &l64, op, &v, &where);
+        if (fields < 4)
             return set_error(CY_ERR_INVALID_ARGUMENT, "bad tuning item: " + item);
         int logn = 0;
         while ((1 << logn) < n) logn++;
@@ -388,9 +396,10 @@ cy_status cy_tuning_import(const char* spec) {
         for (int i = 0; i < TUNE_OPS; i++)
             if (std::strcmp(op, kOpNames[i]) == 0) o = i;
         if ((1 << logn) != n || logn < 1 || logn > LOGN_MAX || o < 0 || v < 0 || v >= variant_count(logn) ||
-            l64 < 1 || l64 > 6)
+            l64 < 1 || l64 > 6 || where < 0 || where >= variant_count(logn))
             return set_error(CY_ERR_INVALID_ARGUMENT, "bad tuning item: " + item);
-        set_choice(dev, logn, l64, o, v);
+        const int rule = fields < 5 ? -1 : where == number_of(logn, 0) ? 0 : where;
+        set_choice(dev, logn, l64, o, rule, v);
     }
     return CY_OK;
 }

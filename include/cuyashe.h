@@ -510,16 +510,17 @@ cy_status cy_graph_destroy(cy_graph *graph);
  * default). cy_ring_autotune runs every schedule of the
  * ring's product on `batch` synthetic jobs, requires each output to equal the
  * default's bit for bit, and keeps the fastest for this device, N and
- * limb count; cy_yashe_autotune does the same for the plain product, the YASHE
+ * limb count, for calls whose default is the same as this batch's; cy_yashe_autotune does the same for the plain product, the YASHE
  * tensor and the keyswitch. Synchronous; allocates its test buffers. The
  * reference has one fixed launch shape per kernel (src/cuda_functions.cu:447-458)
  * and hand-timed block sizes in comments (src/cuda_bn.cu:983-988). */
 cy_status cy_ring_autotune(cy_ring *ring, int batch, cy_stream_t stream);
 cy_status cy_yashe_autotune(cy_yashe *y, int batch, cy_stream_t stream);
 
-/* The current device's choices as text, e.g. "n4096.l2.mul=1;n4096.l2.ks=0;"
- * (*needed gets the size including the terminator), and back. 0 gives an
- * operation back to the default. */
+/* The current device's choices as text, e.g. "n4096.l2.mul=1@8;n4096.l2.ks=0;"
+ * (*needed gets the size including the terminator), and back. "=1@8": schedule 1
+ * for calls whose default is schedule 8; "=1": for calls of any size; "=0": the
+ * default again. */
 cy_status cy_tuning_export(char *buf, size_t len, size_t *needed);
 cy_status cy_tuning_import(const char *spec);
 /* The schedule that a call of operation `op` ("mul", "mulc", "ks" or "ntt") on
