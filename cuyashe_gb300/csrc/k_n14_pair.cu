@@ -27,6 +27,7 @@ void fill_n14_pair(KernelSet& ks) {
     fill_pair_l64<4>(ks);
     fill_pair_l64<5>(ks);
     fill_pair_l64<6>(ks);
+    ks.mul_id = ks.ks_id = -1;
     ks.smem_mul = pair_smem_bytes<2>();
     ks.smem_ks[0] = ks.smem_ks[1] = pair_smem_bytes<2>();
     ks.blocks_per_prime = 2;

@@ -1416,6 +1416,9 @@ void fill_kernel_set(KernelSet& ks) {
     ks.logn = LOGN;
     ks.loge = LOGE;
     ks.threads = PL::G;
+    ks.mul_id = LOGE * 100 + (MB_MUL > 0 ? MB_MUL : mul_min_blocks<LOGN, LOGE>());
+    ks.ks_id = (LOGE * 100 + (MB_KS > 0 ? MB_KS : ks_min_blocks<LOGN, LOGE>())) * 100 + ND_LO * 10 + ND_HI;
+    ks.ntt_id = LOGE;
     if constexpr (!SPECIALISE || SPEC_MASK != 0x7Eu) fill_l64<LOGN, LOGE, 0, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (SPECIALISE && (SPEC_MASK & 2u)) fill_l64<LOGN, LOGE, 1, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);
     if constexpr (SPECIALISE && (SPEC_MASK & 4u)) fill_l64<LOGN, LOGE, 2, MB_MUL, MB_KS, ND_LO, ND_HI>(ks);

@@ -164,6 +164,21 @@ struct DevBuf {
     }
 };
 
+// Whether two kernel sets run an operation alike.
+static bool same_kernels(const KernelSet& a, const KernelSet& b, int op) {
+    if (op == TUNE_NTT) return a.ntt_id == b.ntt_id && a.intt_tma == b.intt_tma;
+    return op == TUNE_KS ? a.ks_id == b.ks_id : a.mul_id == b.mul_id;
+}
+
+// Whether schedule number v runs kernels of its own: not those of the default or of an earlier number.
+static bool distinct(int logn, int op, int rule, int v) {
+    const KernelSet& ks = kernel_variant(logn, v);
+    if (v > 0 && same_kernels(ks, kernel_variant(logn, rule), op)) return false;
+    for (int u = 1; u < v; u++)
+        if (same_kernels(ks, kernel_variant(logn, u), op)) return false;
+    return true;
+}
+
 // Time each schedule of one operation at `blocks` transforms per launch; `run(v, out)` launches it on `st`.
 template <class Run>
 static cy_status tune_op(int logn, int l64, int op, long long blocks, size_t out_bytes, cudaStream_t st, Run run) {
@@ -186,6 +201,7 @@ static cy_status tune_op(int logn, int l64, int op, long long blocks, size_t out
     int best_v = 0;
     cy_status st_all = CY_OK;
     for (int v = 0; v < nv && st_all == CY_OK; v++) {
+        if (!distinct(logn, op, rule, v)) continue;
         void* out = v == 0 ? ref.p : cur.p;
         st_all = run(v, out);  // warm-up and the output to check
         if (st_all != CY_OK && v > 0) {

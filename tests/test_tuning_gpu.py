@@ -80,6 +80,15 @@ def test_tuning_a_batch_leaves_single_calls_alone(cy):
         assert ("n16384.l1.%s=" % op) in cy.tuning_export()
 
 
+def test_the_autotuner_times_each_kernel_once(cy):
+    """N = 8192 has three product kernels and two transforms under numbers 0 .. 3: a check and three timed
+    runs of each, two launches per run."""
+    r = cy.Ring(8192, ring.largest_prime_below(2**62, 2**16))
+    before = cy.launch_count()
+    r.autotune(batch=1)
+    assert cy.launch_count() - before == 4 * 2 * (3 + 2)
+
+
 def test_refused(cy):
     for n, l, op, b in ((1000, 1, "mul", 1), (1024, 0, "mul", 1), (1024, 7, "mul", 1), (1024, 1, "add", 1),
                         (1024, 1, "mul", -1), (32768, 1, "mul", 1)):
