@@ -225,8 +225,11 @@ def check(status: int, where: str) -> None:
 def _stream_handle(stream) -> Optional[int]:
     if stream is None:
         import torch
-        if torch.cuda.is_initialized():  # the raw handle: no stream object per call (2.9 us less)
-            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        if torch.cuda.is_initialized():
+            try:  # the raw handle: no stream object per call (2.9 us less)
+                return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+            except AttributeError:  # private names, which a release of torch may lack
+                pass
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
