@@ -147,7 +147,8 @@ cy_status prime_table(int device, const PrimeTable** out) {
 }
 
 cy_status twiddle_tables(const PrimeTable& t, int logn, TwiddleTables* out) {
-    // one set of lane-ordered tables per device and length, kept until process exit
+    // one set of lane-ordered tables per device and length, kept until process exit as the natural ones are
+    // (32 MB for all five lengths), for the primes that a basis can have
     static std::mutex mu;
     static std::map<std::pair<int, int>, TwiddleTables> known;
     std::lock_guard<std::mutex> lock(mu);
@@ -159,28 +160,30 @@ cy_status twiddle_tables(const PrimeTable& t, int logn, TwiddleTables* out) {
     TwiddleTables T{};
     T.psi = t.d_psi;
     T.ipsi = t.d_ipsi;
-    cy_status st = CY_OK;
-    for (int e = 4; e <= 6 && st == CY_OK; e++) {
-        if (!has_lane_table(logn, e)) continue;
-        const size_t bytes = sizeof(uint2) * (size_t)TABLE_PRIMES * (((size_t)1 << logn) - ((size_t)1 << (logn - e)));
-        for (int inv = 0; inv < 2 && st == CY_OK; inv++) {
-            uint2* d = nullptr;
-            const cudaError_t err = cudaMalloc(&d, bytes);
-            (inv ? T.ipsi_lanes : T.psi_lanes)[e - 4] = d;
-            st = err != cudaSuccess ? cuda_error(err, "twiddle tables")
-                                    : build_lane_table(inv ? t.d_ipsi : t.d_psi, d, logn, e, TABLE_PRIMES);
+    const auto words = [logn](int e) { return (size_t)KMAX * (((size_t)1 << logn) - ((size_t)1 << (logn - e))); };
+    size_t total = 0;
+    for (int e = 4; e <= 6; e++)
+        if (has_lane_table(logn, e)) total += 2 * words(e);
+    if (total > 0) {  // one allocation for a length
+        uint2* mem = nullptr;
+        CY_CUDA(cudaMalloc(&mem, total * sizeof(uint2)));
+        cy_status st = CY_OK;
+        uint2* d = mem;
+        for (int e = 4; e <= 6; e++) {
+            if (!has_lane_table(logn, e)) continue;
+            for (int inv = 0; inv < 2 && st == CY_OK; inv++, d += words(e)) {
+                (inv ? T.ipsi_lanes : T.psi_lanes)[e - 4] = d;
+                st = build_lane_table(inv ? t.d_ipsi : t.d_psi, d, logn, e, KMAX);
+            }
         }
-    }
-    if (st == CY_OK) {
-        const cudaError_t err = cudaStreamSynchronize(nullptr);
-        if (err != cudaSuccess) st = cuda_error(err, "twiddle tables");
-    }
-    if (st != CY_OK) {
-        for (int e = 0; e < 3; e++) {
-            cudaFree(const_cast<uint2*>(T.psi_lanes[e]));
-            cudaFree(const_cast<uint2*>(T.ipsi_lanes[e]));
+        if (st == CY_OK) {
+            const cudaError_t err = cudaStreamSynchronize(nullptr);
+            if (err != cudaSuccess) st = cuda_error(err, "twiddle tables");
         }
-        return st;
+        if (st != CY_OK) {
+            cudaFree(mem);
+            return st;
+        }
     }
     known[{t.device, logn}] = T;
     *out = T;
