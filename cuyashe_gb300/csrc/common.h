@@ -87,7 +87,6 @@ struct BasisDev {
     uint64_t mu;       // floor(2^(32*l32+37) / q')
     uint64_t mu45;     // floor(2^(32*l32+44) / q')
     uint32_t qn[L32MAX];       // q'
-    uint32_t q[L32MAX];        // q
     uint32_t qhalf[L32MAX];    // (q-1)/2
     uint32_t qhalf_n[L32MAX];  // ((q-1)/2) << s
     uint32_t B0[L32MAX];       // MODQ: ((-M) mod q) << s        YASHE: ((-I_M) mod q) << s
@@ -99,7 +98,6 @@ struct BasisDev {
     uint32_t ycon_sh[KMAX];    // Shoup companion of ycon
     uint32_t flo[KMAX], fhi[KMAX];  // floor(2^64/p_i) split in words (estimate of X'/M)
     uint32_t qmont[KMAX];      // q 2^-32 mod p_i (centering)
-    uint32_t r32[KMAX], r32_sh[KMAX];  // 2^32 mod p_i with Shoup companion
     uint32_t crt[KMAX][L32MAX + 1];    // 2^(32 j) mod p_i
     uint32_t A0[KMAX][L32MAX];  // MODQ: (Mhat_i mod q) << s     YASHE: (I_i mod q) << s, t*Mhat_i = I_i q + R_i
     uint32_t A1[KMAX][L32MAX];  //                                YASHE: R_i << s

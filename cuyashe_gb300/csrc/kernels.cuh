@@ -1391,12 +1391,27 @@ void fill_epi_const(const BasisDev& h, void* param) {
 
 namespace cy {
 
+// The kernels of k_mul_key for N = 2^LOGN by limb count (0: the small operand), 16 coefficients per
+// thread, compiled for MINB blocks per SM.
+template <int LOGN, int MINB, int L64>
+KeyKernel key_entry() {
+    return {(void*)k_mul_key<LOGN, 4, L64, MINB>, NttPlan<LOGN, 4>::G, region_bytes<NttPlan<LOGN, 4>, 2>()};
+}
+template <int LOGN, int MINB>
+const KeyKernel* key_row(int l64) {
+    static const KeyKernel row[7] = {key_entry<LOGN, MINB, 0>(), key_entry<LOGN, MINB, 1>(), key_entry<LOGN, MINB, 2>(),
+                                     key_entry<LOGN, MINB, 3>(), key_entry<LOGN, MINB, 4>(), key_entry<LOGN, MINB, 5>(),
+                                     key_entry<LOGN, MINB, 6>()};
+    return &row[l64];
+}
+
 template <int LOGN, int LOGE, int L64, int MB_MUL, int MB_KS, int ND_LO, int ND_HI>
 void fill_l64(KernelSet& ks) {
     ks.mul[L64][0] = (void*)k_mul<LOGN, LOGE, L64, false, MB_MUL>;
     ks.mul[L64][1] = (void*)k_mul<LOGN, LOGE, L64, true, MB_MUL>;
     ks.ks[L64][0] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_LO, MB_KS>;
-    ks.ks[L64][1] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_HI, MB_KS>;
+    // odd limb counts have 1 or 2 digits more than a multiple of four, so none takes ND_HI at a time
+    if constexpr (L64 % 2 == 0) ks.ks[L64][1] = (void*)k_keyswitch<LOGN, LOGE, L64, ND_HI, MB_KS>;
 }
 
 // SPECIALISE: instantiate the kernels for each limb count of SPEC_MASK (all six by default:

@@ -80,7 +80,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const uint32_t h = cluster_rank();
     const int prime = blockIdx.y;
     const int job = blockIdx.x >> 1;
-    const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
+    const int k = M.k;
     const PrimeParam& Q = M.pr[prime];
     const PrimeCtx c = load_prime_ctx(Q);
     const uint2* __restrict__ psi = table_of(M.tw.psi, prime);
@@ -91,30 +91,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     // CRT split of this block's half of a and b only; the peer's half arrives in
     // the first words of this block's exchange region (unused until the first
     // exchange, which follows the barrier below)
-    const uint64_t* a = A + (size_t)job * a_stride + (size_t)h * kPairHalf * l64;
-    const uint64_t* b = Bv + (size_t)job * b_stride + (size_t)h * kPairHalf * l64;
+    const uint64_t* a = A + (size_t)job * a_stride + (size_t)h * kPairHalf * L64;
+    const uint64_t* b = Bv + (size_t)job * b_stride + (size_t)h * kPairHalf * L64;
     dep_wait(a, b);
     uint32_t x[2][E];
 #pragma unroll
     for (int e = 0; e < E; e++) {
         const int pos = slot_pos<PL, 0>(tau, e);
-        if constexpr (L64 > 0) {
-            constexpr int W = 2 * L64;
-            uint32_t cc[W], qh[W];
+        constexpr int W = 2 * L64;
+        uint32_t cc[W], qh[W];
 #pragma unroll
-            for (int j = 0; j < W; j++) {
-                cc[j] = Q.crt[j];
-                qh[j] = M.qhalf[j];
-            }
-            uint32_t w[W];
-            load_words<L64>(a + (size_t)pos * L64, w);
-            x[0][e] = crt_words<W, CENTER>(w, cc, qh, c);
-            load_words<L64>(b + (size_t)pos * L64, w);
-            x[1][e] = crt_words<W, CENTER>(w, cc, qh, c);
-        } else {
-            x[0][e] = crt_coef<CENTER>(a, pos, l64, Q.crt, M.qhalf, c);
-            x[1][e] = crt_coef<CENTER>(b, pos, l64, Q.crt, M.qhalf, c);
+        for (int j = 0; j < W; j++) {
+            cc[j] = Q.crt[j];
+            qh[j] = M.qhalf[j];
         }
+        uint32_t w[W];
+        load_words<L64>(a + (size_t)pos * L64, w);
+        x[0][e] = crt_words<W, CENTER>(w, cc, qh, c);
+        load_words<L64>(b + (size_t)pos * L64, w);
+        x[1][e] = crt_words<W, CENTER>(w, cc, qh, c);
 #pragma unroll
         for (int o = 0; o < 2; o++) store_peer(&smem[o * kPairHalf + pos], h ^ 1u, x[o][e]);
     }
@@ -154,12 +149,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
     const int prime = blockIdx.y;
     const int job = blockIdx.x >> 1;
     const PrimeParam& Q = M.pr[prime];
-    const int k = M.k, l64 = L64 > 0 ? L64 : M.l64;
+    const int k = M.k;
     const Mod m = load_mod(Q);
     const uint32_t p = m.p;
     const uint2* __restrict__ psi = table_of(M.tw.psi, prime);
     const uint2* __restrict__ ipsi = table_of(M.tw.ipsi, prime);
-    const uint64_t* cj = C + (size_t)job * (2 * kPairHalf) * l64;
+    const uint64_t* cj = C + (size_t)job * (2 * kPairHalf) * L64;
     // limb w of coefficient pos at cj[pos * cs + w * ls]: (limbs, 1) for [N][limb],
     // (1, N) for limb-major
     uint32_t* recv = smem + region_bytes<PL, ND>() / 4;
@@ -180,15 +175,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPlan::G, 1)
 #pragma unroll
             for (int o = 0; o < ND; o++) {
                 const int d = d0 + o;
-                uint32_t wl = 0, wh = 0;
-                if (L64 > 0 || d < ell) {  // digits past the top word of q are zero
-                    const uint64_t ll = ld_dep(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
-                    const uint64_t lh = ld_dep(cj + (size_t)(pos + kPairHalf) * cs + (size_t)(d >> 1) * ls);
-                    wl = (uint32_t)(ll >> (32 * (d & 1)));
-                    wh = (uint32_t)(lh >> (32 * (d & 1)));
-                }
-                lo[o] = red_2p(wl, m);  // digit < 2^32 < 6p -> [0, 4p)
-                hi[o] = red_2p(wh, m);
+                // digits past the top word of q are zero
+                const uint64_t ll = ld_dep(cj + (size_t)pos * cs + (size_t)(d >> 1) * ls);
+                const uint64_t lh = ld_dep(cj + (size_t)(pos + kPairHalf) * cs + (size_t)(d >> 1) * ls);
+                lo[o] = red_2p((uint32_t)(ll >> (32 * (d & 1))), m);  // digit < 2^32 < 6p -> [0, 4p)
+                hi[o] = red_2p((uint32_t)(lh >> (32 * (d & 1))), m);
                 ct_bfly(lo[o], hi[o], w0.x, w0.y, m);  // first stage of the whole transform
                 x[o][e] = h ? hi[o] : lo[o];
             }

@@ -223,7 +223,6 @@ cy_status basis_constants(BasisDev& h, int* crt_bits, int n, const BigUInt& q, i
     h.mu = mu.low64();
     h.mu45 = (BigUInt::pow2(32 * h.l32 + 44) / qn).low64();
     qn.to_words32(h.qn, L32MAX);
-    q.to_words32(h.q, L32MAX);
     const BigUInt qhalf = (q - BigUInt(1)).shr(1);
     qhalf.to_words32(h.qhalf, L32MAX);
     qhalf.shl(h.shift).to_words32(h.qhalf_n, L32MAX);
@@ -267,8 +266,6 @@ cy_status basis_constants(BasisDev& h, int* crt_bits, int n, const BigUInt& q, i
         // q 2^-32 = -(m p) / 2^32 with m = q p^-1 mod 2^32 (q: its residue)
         const uint32_t hi = (uint32_t)(((uint64_t)(q.mod_u32(p) * inv) * p) >> 32);
         h.qmont[i] = hi ? p - hi : 0u;
-        h.r32[i] = r32;
-        h.r32_sh[i] = shoup_of(r32, p);
         uint32_t c = 1;
         for (int j = 0; j <= L32MAX; j++) {
             h.crt[i][j] = c;
