@@ -383,8 +383,10 @@ cy_status run_yashe_mul(const Basis& tensor, const Basis& relin, const uint32_t*
     cy_status status = CY_OK;
     for (int c = 0; c < nchunks && status == CY_OK; c++) {
         // (two chunks stay unequal: even ones run the same phase at the same time, and the tails
-        // of one's launches are not filled by the other's; 64 multiplies at N = 8192, 190-bit q, 40
-        // and 24 172.7 us, 32 and 32 176.0 us)
+        // of one's launches are not filled by the other's. Over 21 two-chunk sizes neither cut wins: unequal
+        // : even us for 64 multiplies at N = 8192, 190-bit q, 172.8 : 176.1, 78 213.5 : 221.8, 60 at N =
+        // 16384, 127-bit q, 198.0 : 209.7; but 220 at N = 4096, 127-bit q, 137.7 : 133.6 and 14 at N = 16384,
+        // 380-bit q, 269.1 : 259.9)
         const int j0 = nchunks > 2 ? chunk_start(batch, nchunks, c) : c * chunk;
         const int nj = (nchunks > 2 ? chunk_start(batch, nchunks, c + 1) : std::min(batch, j0 + chunk)) - j0;
         uint64_t* oj = out + (size_t)j0 * stride;

@@ -140,7 +140,7 @@ struct cy_ring {
     cy::BigUInt q;
     std::vector<uint64_t> q_limbs;
     uint64_t* d_q = nullptr;   // q as l64 limbs (elementwise kernels)
-    cy::Basis mul;             // product basis, mod-q epilogue (N^-1 and 2^32 folded)
+    cy::Basis mul;             // product basis, mod-q epilogue (N^-1 and 2^96 folded)
     cy::Basis plain;           // same primes, plain residues (ICRT, scalar multiply, NTT)
     cy_workspace own_ws;
     std::mutex mu;

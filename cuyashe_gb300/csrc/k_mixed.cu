@@ -20,8 +20,8 @@
 // two blocks per SM at 64 registers, where one's barriers, waits and epilogues overlap the
 // other's transforms, or one at 128, where a unit ends sooner. Before, with 8 coefficients per
 // thread in one 1024-thread block, a staged epilogue and a copy of the transforms per limb
-// count and centring: 192 relinearised multiplies of N = 2048, 4096 and 8192 365 us, then 316, now 300; 12 of
-// them 98 us, now 70.
+// count and centring: 192 relinearised multiplies of N = 2048, 4096 and 8192 365 us, now 299; 12 of
+// them 98 us, now 68.
 #include "kernels.cuh"
 
 namespace cy {

@@ -1141,7 +1141,7 @@ struct EpiConst {
 };
 
 // The exact YASHE rounding of yashe_round_exact with the constants read from
-// the basis in global memory (the rare path of k_epi_k).
+// the basis in global memory (the rare path of k_epi_c).
 template <int L>
 __device__ __noinline__ uint64_t yashe_round_exact_g(const BasisDev* __restrict__ B, const uint32_t* __restrict__ r0,
                                                      size_t stride, uint32_t v) {

@@ -124,8 +124,11 @@ static std::vector<MixedUnit> build_units(const std::vector<MixedJob>& jobs) {
 
 // The schedule of a list that the autotuner has not chosen one for. Two blocks per SM
 // (schedule 0) do more per second, one (schedule 1) ends a unit sooner, which is what counts
-// while an SM gets few of them: with twelve multiplies of N = 2048, 4096 and 8192 123 us against 70,
-// with 144 (10 transform units per SM) 245 against 232, with 192 (14) 316 against 344.
+// while an SM gets few of them. us with schedule 0 : 1 of lists of equal parts N = 2048 (62-bit q), 4096 (127)
+// and 8192 (190), relinearised multiplies: twelve 115 : 68, 48 124 : 90, 96 (7 transform units per SM) 172 :
+// 150, 144 (10) 229 : 246, 192 (14) 299 : 331, 576 836 : 977. Lists without keyswitches cross earlier (96
+// tensor products, 4.4 units per SM, 83 : 84; 144, 6.6, 117 : 142), so that the line is late for them and
+// for multiplies between 9 and 12 units; a plan's autotuner picks the faster.
 static int default_schedule(const std::vector<MixedUnit>& units, int sms) {
     long long transforms = 0;
     for (const MixedUnit& u : units) transforms += u.kind == 0 || u.kind == 2;

@@ -78,7 +78,7 @@ extern "C" cy_status cy_polymul_noalloc(cy_ring* r, const uint64_t* d_a, const u
     const int n = B.h.n, k = B.h.k;
     const size_t per_product = (size_t)k * n * sizeof(uint32_t);
     size_t max_batch = CY_NOALLOC_SCRATCH_BYTES / per_product;
-    if (max_batch > 65535) max_batch = 65535;  // one launch: the grid's y dimension holds the products
+    if (max_batch > 65535) max_batch = 65535;  // the call's stated limit
     if ((size_t)batch > max_batch) {
         char msg[200];
         std::snprintf(msg, sizeof(msg),

@@ -1,8 +1,8 @@
 // tuning.cpp -- choice of NTT schedule per (device, N, limb count, operation).
 //
 // Every transform length has one or more compiled schedules (kernel variants:
-// 8 or 16 coefficients per thread, hence 512/256/... threads per transform and
-// 4 or 3 register passes at N = 4096). The autotuner runs each schedule of an
+// 8 to 64 coefficients per thread, hence 512 to 64 threads per transform and
+// 4 to 2 register passes at N = 4096). The autotuner runs each schedule of an
 // operation on a synthetic batch of the caller's ring, checks that its output is
 // bit-identical to the default schedule's, times it with CUDA events and keeps
 // the fastest, for calls of the same regime (the default rule depends on the call's size). Choices live
@@ -66,25 +66,28 @@ static int sm_count() {
 // The schedule of a call that the autotuner has not chosen one for: `blocks` transforms'
 // blocks per launch (jobs times primes). Two regimes: up to one block per SM the time is one
 // block's latency (more threads per transform, or a pair of blocks); above, throughput. The
-// lines, measured with every schedule at q of 60 to 380 bits (us per call, the schedule
-// taken first; jobs and bits of q in brackets):
-//   N = 1024   8 coefficients per thread (keyswitch [512, 190] 67 against 95 with 16), but 16 for
-//              products from two blocks per SM on ([2048, 127] 132 against 146, [512, 380] 163
-//              against 205) and transforms from four on ([2048, 127] 33 against 37)
-//   N = 2048   products 16 per thread ([512, 250] 186 against 216; [1, 250] 10.8 against 11.2),
-//              transforms from four blocks per SM on ([2048, 127] 66 against 80; [8, 127] 5.9
-//              against 4.5); keyswitch 8 ([512, 250] 227 against 479)
-//   N = 4096   16 per thread, products and transforms at three blocks per SM ([2048, 127] 567
-//              against 630 and 138 against 172 with 8), keyswitch two blocks of 128 registers
-//              ([2048, 127] 561 against 602), up to one block per SM at the full register file
-//              (one 127-bit: 14.7 against 15.7)
-//   N = 8192   16 per thread at 64 registers ([512, 190] 587 against 708), keyswitches of two
-//              limbs or more 128 registers ([37, 190] 55 against 58; [64, 380] 320 against 383)
-//   N = 16384  a pair of blocks per transform while that is one block per SM at most ([1, 380]
-//              product 27 against 40; [5, 380] keyswitch 73 against 106, but [8, 250] 96 against
-//              73). Above: keyswitch 32 per thread ([64, 62] 46 against 50, [256, 380] 2714
-//              against 2815), products of five limbs or more too ([64, 300] 371 against 386,
-//              [256, 380] 1680 against 1824; [64, 250] 246 against 236), all else 16
+// lines, measured with every schedule at q of 60 to 380 bits: [jobs, bits of q] us per call with the
+// schedule taken : with the other one.
+//   N = 1024   8 coefficients per thread (keyswitch [512, 380] 213 : 505 with 16, [512, 62] 17.1 : 17.8), but
+//              16 for products from two blocks per SM on ([2048, 127] 132 : 146, [512, 380] 157 : 203, [64,
+//              127] 8.3 : 8.8; at the line [34, 127] 7.5 : 7.0) and transforms from four on ([2048, 127] 33 :
+//              38; below it [64, 127] 4.4 : 4.7)
+//   N = 2048   products 16 per thread ([512, 250] 179 : 214; [1, 250] 9.0 : 8.8), transforms 8 below four
+//              blocks per SM ([8, 127] 4.9 : 5.9), 16 from there on ([2048, 127] 66 : 83); keyswitch 8
+//              ([512, 250] 225 : 445)
+//   N = 4096   16 per thread, products and transforms at three blocks per SM ([2048, 127] 566 : 622 and 138 :
+//              171 with 8; between two and four blocks per SM four fit better, [64, 127] 24.8 : 22.6).
+//              Keyswitch: two blocks of 128 registers ([2048, 127] 560 : 605 with 8); up to one block per SM
+//              8 per thread with the full register file (three limbs [1, 190] 12.9 : 14.7, five [1, 320] 20.5
+//              : 24.4; even digit counts are within 3% either way, [1, 127] 10.5 : 10.2)
+//   N = 8192   16 per thread at 64 registers ([512, 190] 585 : 711 with 8), keyswitches of two
+//              limbs or more 128 registers ([37, 190] 54.7 : 58.0; [64, 380] 300 : 353)
+//   N = 16384  a pair of blocks per transform while that is one block per SM at most ([1, 380] product 26 :
+//              37, [15, 62] 19.5 : 23.8; above it [16, 62] 24.0 : 35.7; keyswitch [5, 380] 73 : 106, above it
+//              [8, 250] 73 : 96). Above: keyswitch 32 per thread ([64, 62] 46 : 50, [256, 380] 2690 : 2800);
+//              products of five limbs or more too ([64, 300] 369 : 380, [256, 380] 1686 : 1822), those of
+//              fewer 16 ([64, 250] 236 : 246), and centred ones always ([64, 300] 359 : 374, [64, 380] 420 :
+//              463; inside the multiply of 256 pairs 4052 : 4177); all else 16
 int default_variant(int logn, int l64, int op, long long blocks) {
     const int sms = sm_count();
     const bool small = blocks <= sms;
